@@ -511,6 +511,18 @@ int qcl_static_contraction(int precision, const qcl_mechanism* op, int NE, int N
   if ((s = dG.upload(G, nb))) return s;
   if ((s = dS.upload(beta != 0.0 ? S : nullptr, nb))) return s;
   if ((s = work.alloc(contraction_work_elems(k, NE, Nk, Nb) * cbytes(sp)))) return s;
+  DevBuf i8;
+  if (sp == QCL_C128) {  // the integer tensor path, where it pays and fits
+    const size_t n = contraction_i8_bytes(k, NE, Nk, Nb);
+    if (n > 0 && cudaMalloc(&i8.p, n) == cudaSuccess) {
+      k.i8_work = i8.p;
+      k.i8_bytes = n;
+      k.status = (int*)st.p;
+    } else {
+      cudaGetLastError();
+      i8.p = nullptr;
+    }
+  }
   if ((s = launch_contraction(sp, k, NE, Nk, Nb, (const double*)dwk.p, dG.p, dS.p, alpha * op->q, beta, work.p, 0)))
     return s;
   QCL_CUDA_CHECK(cudaDeviceSynchronize());

@@ -466,6 +466,12 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
     const int Nc = Nk * N2;
     if (sizeof(R) == 4 && op.tc_bop)  // complex64 fields: tensor cores (scaled FP16 hi/lo)
       return launch_tc_dense_contraction(NE, Nc, op.tc_bop, Gv, Sv, alpha_q, beta, (float*)work, op.status, st);
+    if (sizeof(R) == 8 && op.i8_work && i8_worthwhile(NE, 1, Nc, Nc)) {
+      const void* A[1] = {Gv};
+      void* C[1] = {Sv};
+      return launch_i8_gemm(NE, 1, Nc, Nc, A, NEl, wk, Nk, op.matrix, Nc, C, NEl, alpha_q, beta, op.i8_work, op.i8_bytes,
+                            op.status, st);
+    }
     if (sizeof(R) == 8) {  // complex128: FP64 tensor path (DMMA)
       DmArgs d{NE, Nc, Nc, (const Cx<double>*)Gv, NEl, wk, Nk, (const Cx<double>*)op.matrix, Nc, (Cx<double>*)Sv, NEl,
                alpha_q, beta};
@@ -582,7 +588,13 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
       }
       const double bc = c == 0 ? beta : 1.0;
       const Cx<R>* blk = (const Cx<R>*)op.block + (size_t)N2 * N2 * i0;
-      if (sizeof(R) == 8) {
+      if (sizeof(R) == 8 && op.i8_work && i8_worthwhile((int)Mr, 1, N2, jc * N2)) {
+        const void* A[1] = {Z};
+        void* C[1] = {Sv};
+        if ((s = launch_i8_gemm((int)Mr, 1, N2, jc * N2, A, Mr, nullptr, 1, blk, N2, C, Mr, alpha_q, bc, op.i8_work,
+                                op.i8_bytes, op.status, st)))
+          return s;
+      } else if (sizeof(R) == 8) {
         DmArgs d{(int)Mr, N2, jc * N2, (const Cx<double>*)Z, Mr, nullptr, 1, (const Cx<double>*)blk, N2,
                  (Cx<double>*)Sv, Mr, alpha_q, bc};
         if ((s = launch_dmma_dense(d, st))) return s;
@@ -665,6 +677,33 @@ size_t contraction_work_elems(const KernelOpDev& op, int NE, int Nk, int N) {
     return zf;
   }
   return 0;
+}
+
+// The area for the whole operands, or, for a stage-2 product of a separable
+// sum with many more rows than columns, for a panel of rows.
+size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N) {
+  const int N2 = N * N;
+  if (op.kind == QCL_KERNEL_DENSE) {
+    const int Nc = Nk * N2;
+    return i8_worthwhile(NE, 2, Nc, Nc) ? i8_work_bytes(NE, 2, Nc, Nc) : 0;
+  }
+  if (op.kind == QCL_KERNEL_SEPARABLE_SUM) {
+    const long long Mr = (long long)NE * Nk;
+    const int K = (op.J < kSepChunk ? op.J : kSepChunk) * N2;
+    return i8_worthwhile((int)Mr, 1, N2, K) ? i8_work_bytes((int)(Mr < 4736 ? Mr : 4736), 1, N2, K) : 0;
+  }
+  return 0;
+}
+
+int launch_contraction_pair(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk,
+                            const void* const* G, void* const* S, double alpha_q, void* work, cudaStream_t st) {
+  const int Nc = Nk * N * N;
+  if (precision == QCL_C128 && op.kind == QCL_KERNEL_DENSE && op.i8_work && i8_worthwhile(NE, 2, Nc, Nc))
+    return launch_i8_gemm(NE, 2, Nc, Nc, G, NE, wk, Nk, op.matrix, Nc, S, NE, alpha_q, 0.0, op.i8_work, op.i8_bytes,
+                          op.status, st);
+  for (int f = 0; f < 2; ++f)
+    if (int s = launch_contraction(precision, op, NE, Nk, N, wk, G[f], S[f], alpha_q, 0.0, work, st)) return s;
+  return QCL_OK;
 }
 
 int launch_contraction(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk, const void* G,

@@ -126,6 +126,10 @@ struct KernelOpDev {
   const void* const* tc_chunks = nullptr;
   const void* const* tc_stage1 = nullptr;  // separable sum: stage-1 operand per chunk (radial factors)
   int* status = nullptr;  // device status word for bounded-wait timeouts
+  // complex128 dense and separable operators: work area of the integer tensor
+  // path (i8_gemm.cu); without one, or for small products, the FP64 tensor path runs
+  void* i8_work = nullptr;
+  size_t i8_bytes = 0;
 };
 // Terms of a separable-sum operator contracted per stage-2 GEMM: the
 // intermediate of a chunk holds kSepChunk fields.
@@ -148,6 +152,19 @@ int launch_tc_presplit(int M, int Nout, int Kc, const void* Bop, const float* aw
                        long long oQ, long long oR, double alpha, double beta, int* status, cudaStream_t st);
 int launch_tc_dense_contraction(int NE, int Nc, const void* Bop, const void* G, void* S, double alpha, double beta,
                                 float* awork, int* status, cudaStream_t st);
+// complex128 products on the integer tensor path (i8_gemm.cu): up to two
+// fields of M rows against one operator
+size_t i8_work_bytes(int M, int fields, int N, int K);
+bool i8_worthwhile(int M, int fields, int N, int K);
+int launch_i8_gemm(int M, int fields, int N, int K, const void* const* A, long long lda, const double* w, int wmod,
+                   const void* B, long long ldb, void* const* C, long long ldc, double alpha, double beta, void* work,
+                   size_t work_bytes, int* status, cudaStream_t st);
+int i8_set_wait_limit(long long rounds);
+// Work area of the integer path a complex128 contraction would use (0: none).
+size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N);
+// Two fields through one operator: S[f] = alpha_q K[wk G[f]].
+int launch_contraction_pair(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk,
+                            const void* const* G, void* const* S, double alpha_q, void* work, cudaStream_t st);
 int launch_contraction(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk, const void* G,
                        void* S, double alpha_q, double beta, void* work, cudaStream_t st);
 

@@ -50,8 +50,12 @@ struct Mech {
   std::vector<void*> tc_chunks;  // separable sum: tensor-core operand per term chunk (complex64 fields)
   std::vector<void*> tc_stage1;  // separable sum: stage-1 operand per term chunk
   int* status = nullptr;
+  void* i8_work = nullptr;  // the context's work area of the integer tensor path
+  size_t i8_bytes = 0;
   KernelOpDev view() const {
     KernelOpDev k;
+    k.i8_work = i8_work;
+    k.i8_bytes = i8_bytes;
     k.tc_bop = tc_bop;
     k.tc_chunks = tc_chunks.empty() ? nullptr : tc_chunks.data();
     k.tc_stage1 = tc_stage1.size() == tc_chunks.size() && !tc_stage1.empty() ? tc_stage1.data() : nullptr;
@@ -121,6 +125,9 @@ struct ScbaCtx {
   void* tmp = nullptr;
   void* cwork = nullptr;
   size_t cwork_bytes = 0;
+  void* i8_work = nullptr;  // complex128: work area of the integer tensor path, where the budget has room
+  size_t budget = 0;        // the explicit memory budget (0: the device's free memory)
+  size_t base_peak = 0;     // what the plan without that area needs
   // reductions
   Cx<double>*trL = nullptr, *trG = nullptr;
   double* rpartial = nullptr;
@@ -281,6 +288,7 @@ void scba_destroy(ScbaCtx* c) {
   cudaFree(c->candSL);
   cudaFree(c->tmp);
   cudaFree(c->cwork);
+  cudaFree(c->i8_work);
   cudaFree(c->trL);
   cudaFree(c->trG);
   cudaFree(c->rpartial);
@@ -397,6 +405,33 @@ int scba_estimate_memory(const qcl_scba_problem* p, const qcl_mechanism* mechs, 
   return QCL_OK;
 }
 
+// The work area of the integer tensor path, from what the budget leaves over:
+// the contractions run without one (on the FP64 tensor path), so a budget
+// that holds the plan stays sufficient.  Smaller areas split the operands in
+// panels.  Without an explicit budget other contexts will want the device's
+// free memory too: at most a quarter of it.
+static void i8_area(ScbaCtx* c) {
+  if (c->precision != QCL_C128 || c->i8_work) return;
+  size_t want = 0, room = 0, tot = 0;
+  if (c->budget) room = c->budget > c->base_peak ? c->budget - c->base_peak : 0;
+  else if (cudaMemGetInfo(&room, &tot) == cudaSuccess) room /= 4;
+  else room = 0;
+  for (auto& m : c->mech) want = std::max(want, contraction_i8_bytes(m.view(), c->NE, c->Nk, c->N));
+  for (int cut = 1; want > 0 && cut <= 8; cut *= 2) {
+    const size_t n = want / cut;
+    if (n > room) continue;
+    if (cudaMalloc(&c->i8_work, n) == cudaSuccess) {
+      for (auto& m : c->mech) {
+        m.i8_work = c->i8_work;
+        m.i8_bytes = n;
+      }
+      return;
+    }
+    cudaGetLastError();  // no room after all
+    c->i8_work = nullptr;
+  }
+}
+
 int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx** out) {
   *out = nullptr;
   if (!p || p->NE < 2 || p->Nk < 1 || p->Nb < 1) {
@@ -423,13 +458,14 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
     set_last_error("refinement applies to a reduced-precision context (QCL_C64 or QCL_MIXED)");
     return QCL_ARG;
   }
+  size_t budget = p->memory_budget_bytes, base_peak = 0;
   {
     // preflight: refuse before the first allocation (build_production_cache,
     // production_cache.jl:764-770)
     MemPlan mp;
     int s0 = plan_memory(p, mechs, &mp);
     if (s0) return s0;
-    size_t budget = p->memory_budget_bytes;
+    base_peak = mp.peak();
     if (budget == 0) {
       size_t fr = 0, tot = 0;
       cudaError_t e = cudaMemGetInfo(&fr, &tot);
@@ -617,6 +653,9 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
   }
   TRY(prepare_hilbert_tables(c->hil, c->NE, de, c->precision));
   TRY(ensure_partial(c->hil, (long long)c->Nk * N2));
+  c->budget = p->memory_budget_bytes;
+  c->base_peak = base_peak;
+  i8_area(c);
 #undef TRY
   QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));
   c->pops.assign(c->N, 0.0);
@@ -639,24 +678,26 @@ static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, con
     const KernelOpDev op = m.view();
     void* SL = field_of(dst, i, 1);
     void* SG = field_of(dst, i, 2);
+    const void* X[2] = {GL, GG};
+    void* const Y[2] = {SL, SG};
     if (m.is_LO) {
       // _production_lo_contraction, thermal branch (production_operators.jl:1045-1163):
       //   Sigma< = (N+1) K[G<(E+hw)] + N K[G<(E-hw)],  Sigma> = (N+1) K[G>(E-hw)] + N K[G>(E+hw)].
       // K is linear, so each is one contraction of the combined shifted field,
       // K[(N+1) G(E+-hw) + N G(E-+hw)]: two dense maps instead of four.
+      // The candidate total's field is free until the candidates exist: it
+      // holds the second combined field.
       const double n = c->N_LO;
       if ((s = launch_shift_pair(cp, c->NE, ncols, c->shift[2].view(), c->shift[3].view(), n + 1, n, GL, c->tmp,
                                  c->st)))
         return s;
-      if ((s = launch_contraction(cp, op, c->NE, c->Nk, c->N, c->wk, c->tmp, SL, m.q, 0.0, c->cwork, c->st))) return s;
-      if ((s = launch_shift_pair(cp, c->NE, ncols, c->shift[3].view(), c->shift[2].view(), n + 1, n, GG, c->tmp,
+      if ((s = launch_shift_pair(cp, c->NE, ncols, c->shift[3].view(), c->shift[2].view(), n + 1, n, GG, c->candSL,
                                  c->st)))
         return s;
-      if ((s = launch_contraction(cp, op, c->NE, c->Nk, c->N, c->wk, c->tmp, SG, m.q, 0.0, c->cwork, c->st))) return s;
-    } else {
-      if ((s = launch_contraction(cp, op, c->NE, c->Nk, c->N, c->wk, GL, SL, m.q, 0.0, c->cwork, c->st))) return s;
-      if ((s = launch_contraction(cp, op, c->NE, c->Nk, c->N, c->wk, GG, SG, m.q, 0.0, c->cwork, c->st))) return s;
+      X[0] = c->tmp;
+      X[1] = c->candSL;
     }
+    if ((s = launch_contraction_pair(cp, op, c->NE, c->Nk, c->N, c->wk, X, Y, m.q, c->cwork, c->st))) return s;
     void* SR = field_of(dst, i, 0);
     if (c->drop_real) {
       // Sigma^R = -i Gamma / 2 (production_operators.jl:1174-1177); no roundoff estimate
@@ -1357,6 +1398,7 @@ int scba_promote(ScbaCtx* c) {
     m.tc_stage1.clear();
   }
   c->precision = QCL_C128;
+  i8_area(c);
   c->guard_roundoff = 1.1920928955078125e-07;  // the promoted state's FP32 rounding
   c->fbytes = c->nfield * 16;
   if ((s = prepare_hilbert_tables(c->hil, c->NE, c->de, QCL_C128))) return s;
@@ -1485,7 +1527,10 @@ int sweep_run(Sweep* sw, int max_iter, double tol, qcl_scba_row* last, int* iter
     bool changed = false;
     while (next < n && used + peak[next] <= budget) {
       qcl_scba_problem p = sw->points[next].problem;
-      p.memory_budget_bytes = budget - used;
+      // what the points that fit beside this one leave over may hold its integer-path area
+      size_t rest = budget - used - peak[next];
+      for (int j = next + 1; j < n && peak[j] <= rest; ++j) rest -= peak[j];
+      p.memory_budget_bytes = peak[next] + rest;
       ScbaCtx* c = nullptr;
       int s = scba_create(&p, sw->points[next].mechs.data(), &c);
       if (s) return fail(s);
@@ -1494,8 +1539,9 @@ int sweep_run(Sweep* sw, int max_iter, double tol, qcl_scba_row* last, int* iter
         scba_destroy(c);
         return fail(s);
       }
-      active.push_back({next, c, peak[next]});
-      used += peak[next];
+      const size_t bytes = peak[next] + (c->mech.empty() ? 0 : c->mech[0].i8_bytes);
+      active.push_back({next, c, bytes});
+      used += bytes;
       ++next;
       changed = true;
     }

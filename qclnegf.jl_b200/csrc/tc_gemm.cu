@@ -45,6 +45,7 @@
 #include <mutex>
 
 #include "kernels.cuh"
+#include "tc_prims.cuh"
 
 namespace qcl {
 
@@ -64,7 +65,6 @@ template <int BN> struct TcShape {
   static constexpr int CH = BN / 2;                   // accumulator columns per drain warp
   static constexpr int LDW = CH % 32 == 0 ? 32 : 16;  // tensor-memory load width
 };
-constexpr long long TC_WAIT_LIMIT = 1ll << 22;  // try_wait rounds (~1 s) before a wait gives up
 // Rounds of the main-loop waits (producer, MMA issuer, accumulator drain).  The
 // waits after a failure (in-flight copies and MMAs) always use TC_WAIT_LIMIT.
 // qcl_debug_set_wait_limit lowers it so that a test can take the timeout path.
@@ -81,31 +81,6 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw64(uint32_t saddr) {
 // Instruction descriptor (kind::f16): D f32, A/B f16, both K-major, N = BN, M = 128.
 template <int BN> __device__ __forceinline__ constexpr uint32_t tc_idesc() {
   return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Bounded parity wait; returns false if it gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long limit = TC_WAIT_LIMIT) {
-  for (long long i = 0; i < limit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
 }
 
 // 2D tiled TMA load (no multicast) of the box at (x = K offset, y = row).
@@ -125,10 +100,6 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 // Reads 16 consecutive accumulator columns of this thread's lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
@@ -750,7 +721,7 @@ int launch_tc_presplit(int M, int Nout, int Kc, const void* Bop, const float* aw
 int tc_set_wait_limit(long long rounds) {
   const long long v = rounds >= 0 ? rounds : TC_WAIT_LIMIT;
   QCL_CUDA_CHECK(cudaMemcpyToSymbol(g_tc_main_wait_limit, &v, sizeof(v)));
-  return QCL_OK;
+  return i8_set_wait_limit(rounds);
 }
 
 int launch_tc_dense_contraction(int NE, int Nc, const void* Bop, const void* G, void* S, double alpha, double beta,
