@@ -479,7 +479,9 @@ int qcl_scba_promote(qcl_scba* ctx);
  * and the last seed's :initialization time.  Phases run back to back on the
  * context's stream except that the G-only part of the residual suite runs on
  * a side stream during the candidate phases; "residuals" is the time from the
- * candidate total to the end of the reduction. */
+ * candidate total to the end of the reduction.  With linear mixing the pass
+ * that assembles the candidate total mixes as well: its time is
+ * candidate_assembly, and "mixing" is empty. */
 #define QCL_PHASES 7
 int qcl_scba_use_telemetry(qcl_scba* ctx, int enable);
 int qcl_scba_phase_times(qcl_scba* ctx, double* ms, double* initialization_ms);

@@ -686,6 +686,7 @@ int qcl_current_populations(int precision, int NE, int Nk, int Nb, const double*
   if ((s = c.upload(GL, nb))) return s;
   if ((s = d.upload(GG, nb))) return s;
   if ((s = part.alloc(observables_partial_doubles(Nb) * sizeof(double)))) return s;
+  QCL_CUDA_CHECK(cudaMemset(part.p, 0, part.bytes));
   if ((s = o.alloc((2 + Nb) * sizeof(double)))) return s;
   if ((s = launch_observables(sp, NE, Nk, Nb, (const double*)dwE.p, (const double*)dwk.p, a.p, b.p, c.p, d.p, gs,
                               target, (double*)part.p, (double*)o.p, 0)))

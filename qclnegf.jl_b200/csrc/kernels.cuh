@@ -83,7 +83,15 @@ int launch_assemble_kernel(int form, int Nk, int Nb, int T, const double* W, con
 int launch_retarded_drop(int precision, size_t n, const void* SL, const void* SG, void* SR, cudaStream_t st);
 int launch_scattering_model(int precision, int NE, int Nk, int N, const double* wk, double norm, int diagonal,
                             int averaged, void* const* fields, cudaStream_t st);
-int launch_sum_fields(int precision, size_t n, const void* const* src, int count, void* out, cudaStream_t st);
+int launch_sum_fields(int precision, size_t n, const void* const (*src)[8], int count, void* const* out, int comps,
+                      cudaStream_t st);
+int launch_trace_coefficients(int NE, int Nk, const void* trL, const void* trG, const double* wE, const double* wk,
+                              double* partial, unsigned* counter, int gs, double target, double realness_limit,
+                              double* traces, double* coeffs, int* status, int scalar, int branch, cudaStream_t st);
+size_t mix_families_partial_doubles();
+int launch_mix_families(int precision, size_t n, const void* const* old, void* const* cand, int F, void* total_lesser,
+                        double alpha, double* partial, unsigned* counter, double* fam_out, double* emb_out,
+                        cudaStream_t st);
 constexpr int kMaxMixFields = 32;
 size_t residual_mix_multi_partial_doubles(int nf);
 int launch_residual_mix_multi(int precision, size_t n, const void* const* old, void* const* cand, int nf,

@@ -41,111 +41,112 @@ template <int K> __device__ __forceinline__ void cta_sum(double (&v)[K], double*
     }
 }
 
-template <typename R>
-__global__ void current_partial_kernel(int NE, int Nk, int N, const double* __restrict__ wE,
-                                       const double* __restrict__ wk, const Cx<R>* __restrict__ SG,
-                                       const Cx<R>* __restrict__ SL, const Cx<R>* __restrict__ GL,
-                                       const Cx<R>* __restrict__ GG, double* partial) {
-  const long long n = (long long)NE * Nk * N * N;
-  const long long blocks = (long long)NE * Nk;
-  double v[2] = {0, 0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long em = i % blocks, ab = i / blocks;
-    const int e = (int)(em % NE), m = (int)(em / NE);
-    const int a = (int)(ab % N), b = (int)(ab / N);
-    const long long it = em + blocks * ((long long)b + (long long)N * a);  // (e, m, b, a)
-    const Cx<R> sg = SG[i], sl = SL[i], gl = GL[it], gg = GG[it];
-    const double w = wE[e] * wk[m];
-    const double re = ((double)sg.x * gl.x - (double)sg.y * gl.y) - ((double)sl.x * gg.x - (double)sl.y * gg.y);
-    const double im = ((double)sg.x * gl.y + (double)sg.y * gl.x) - ((double)sl.x * gg.y + (double)sl.y * gg.x);
-    v[0] += w * re;
-    v[1] += w * im;
-  }
-  cta_sum<2>(v, partial + 2 * blockIdx.x);
-}
-
-template <typename R>
-__global__ void population_partial_kernel(int NE, int Nk, int N, const double* __restrict__ wE,
-                                          const double* __restrict__ wk, const Cx<R>* __restrict__ GL,
-                                          double* partial) {
-  const int a = blockIdx.y;
-  const long long blocks = (long long)NE * Nk;
-  const size_t off = (size_t)blocks * ((size_t)a + (size_t)N * a);
-  double v[2] = {0, 0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < blocks;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int e = (int)(i % NE), m = (int)(i / NE);
-    const Cx<R> g = GL[off + i];
-    const double w = wE[e] * wk[m];
-    v[0] += w * g.x;
-    v[1] += w * g.y;
-  }
-  cta_sum<2>(v, partial + 2 * ((size_t)a * gridDim.x + blockIdx.x));
-}
-
-// Combines partials into the final scalars:
+// One launch.  A CTA owns 256 consecutive (e, m): each thread's weight is read
+// once, every field access is contiguous, and the CTAs of a row of the grid
+// take slices of the (a, b) of the current (blockIdx.y < S) or the diagonal
+// of the populations (blockIdx.y = S).  The CTA that finishes last adds the
+// partial sums in CTA order:
 //   out[0] = Jbar, out[1] = Im of the complex flux (diagnostic),
 //   out[2 + a] = p_a.
-// One CTA per quantity (current, then each population), fixed-order sums.
-__global__ void observables_combine_kernel(int N, int ncta, const double* cur, const double* pop, int gs, double target,
-                                           double* out) {
-  const int q = blockIdx.x;  // 0: current, 1 + a: population a
-  const double* src = q == 0 ? cur : pop + 2 * (size_t)(q - 1) * ncta;
-  double re = 0, im = 0;
-  for (int c = threadIdx.x; c < ncta; c += blockDim.x) {
-    re += src[2 * c];
-    im += src[2 * c + 1];
+// Bound by the four field reads: 537 MB at N_E x N_k = 1024 x 32, N_b = 16,
+// complex128: 139 + 10 + 4 us in three launches with a division per element -> 94 us.
+constexpr int OBS_SLICES = 8;
+template <typename R>
+__global__ void __launch_bounds__(OBS_THREADS)
+    observables_kernel(int NE, int Nk, int N, const double* __restrict__ wE, const double* __restrict__ wk,
+                       const Cx<R>* __restrict__ SG, const Cx<R>* __restrict__ SL, const Cx<R>* __restrict__ GL,
+                       const Cx<R>* __restrict__ GG, int gs, double target, double* partial, unsigned* counter,
+                       double* out) {
+  const long long blocks = (long long)NE * Nk;
+  const int S = (int)gridDim.y - 1;
+  double* cur = partial;                                         // [gridDim.x][S][2]
+  double* pop = partial + 2 * (size_t)gridDim.x * OBS_SLICES;   // [N][gridDim.x][2]
+  const long long step = (long long)gridDim.x * OBS_THREADS;
+  if ((int)blockIdx.y < S) {
+    const int q0 = N * N * blockIdx.y / S, q1 = N * N * (blockIdx.y + 1) / S;
+    double v[2] = {0, 0};
+    for (long long em = blockIdx.x * (long long)OBS_THREADS + threadIdx.x; em < blocks; em += step) {
+      const double w = wE[em % NE] * wk[em / NE];
+      double re = 0, im = 0;
+      int a = q0 % N, b = q0 / N;
+#pragma unroll 4
+      for (int q = q0; q < q1; ++q) {
+        const size_t i = (size_t)em + (size_t)blocks * q, it = (size_t)em + (size_t)blocks * (b + N * a);
+        const Cx<R> sg = SG[i], sl = SL[i], gl = GL[it], gg = GG[it];
+        re += ((double)sg.x * gl.x - (double)sg.y * gl.y) - ((double)sl.x * gg.x - (double)sl.y * gg.y);
+        im += ((double)sg.x * gl.y + (double)sg.y * gl.x) - ((double)sl.x * gg.y + (double)sl.y * gg.x);
+        if (++a == N) {
+          a = 0;
+          ++b;
+        }
+      }
+      v[0] += w * re;
+      v[1] += w * im;
+    }
+    cta_sum<2>(v, cur + 2 * ((size_t)blockIdx.x * S + blockIdx.y));
+  } else {
+    for (int a = 0; a < N; ++a) {
+      double v[2] = {0, 0};
+      for (long long em = blockIdx.x * (long long)OBS_THREADS + threadIdx.x; em < blocks; em += step) {
+        const Cx<R> g = GL[(size_t)em + (size_t)blocks * (a + N * a)];
+        const double w = wE[em % NE] * wk[em / NE];
+        v[0] += w * g.x;
+        v[1] += w * g.y;
+      }
+      cta_sum<2>(v, pop + 2 * ((size_t)a * gridDim.x + blockIdx.x));
+      __syncthreads();  // the sum's scratch is reused
+    }
   }
-  __shared__ double red[2][32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    re += __shfl_xor_sync(0xffffffffu, re, o);
-    im += __shfl_xor_sync(0xffffffffu, im, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = re;
-    red[1][threadIdx.x >> 5] = im;
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == gridDim.x * gridDim.y - 1;
+    if (last) *counter = 0;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  re = 0;
-  im = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-    re += red[0][w];
-    im += red[1][w];
-  }
+  if (!last) return;
+  __threadfence();
   const double pre = gs / (2.0 * M_PI);
-  if (q == 0) {
-    out[0] = pre * re;
-    out[1] = pre * im;
-  } else {
-    // -i pre (re + i im) = pre (im - i re): real part = pre * im
-    out[1 + q] = pre * im / target;
+  for (int q = threadIdx.x >> 5; q < 1 + N; q += OBS_THREADS / 32) {  // one warp per quantity
+    const double* src = q == 0 ? cur : pop + 2 * (size_t)(q - 1) * gridDim.x;
+    const int count = q == 0 ? (int)gridDim.x * S : (int)gridDim.x;
+    double re = 0, im = 0;
+    for (int c = threadIdx.x & 31; c < count; c += 32) {
+      re += __ldcg(src + 2 * c);
+      im += __ldcg(src + 2 * c + 1);
+    }
+    re = wsum(re);
+    im = wsum(im);
+    if ((threadIdx.x & 31) != 0) continue;
+    if (q == 0) {
+      out[0] = pre * re;
+      out[1] = pre * im;
+    } else {
+      out[1 + q] = pre * im / target;  // -i pre (re + i im) = pre (im - i re): real part = pre * im
+    }
   }
 }
 
-size_t observables_partial_doubles(int N) { return 2 * (size_t)OBS_CTAS * (1 + N); }
+size_t observables_partial_doubles(int N) { return 2 * (size_t)OBS_CTAS * (OBS_SLICES + N) + 1; }
 
 // SG, SL: the plus-embedding family (Sigma+^>, Sigma+^<); GL, GG: the state.
+// partial: observables_partial_doubles(N), of which the last is the CTA
+// counter, zero before the first launch.
 int launch_observables(int precision, int NE, int Nk, int N, const double* wE, const double* wk, const void* SG,
                        const void* SL, const void* GL, const void* GG, int gs, double target, double* partial,
                        double* out, cudaStream_t st) {
-  double* cur = partial;
-  double* pop = partial + 2 * OBS_CTAS;
-  if (precision == QCL_C128) {
-    current_partial_kernel<double><<<OBS_CTAS, OBS_THREADS, 0, st>>>(NE, Nk, N, wE, wk, (const Cx<double>*)SG,
-                                                                     (const Cx<double>*)SL, (const Cx<double>*)GL,
-                                                                     (const Cx<double>*)GG, cur);
-    population_partial_kernel<double><<<dim3(OBS_CTAS, N), OBS_THREADS, 0, st>>>(NE, Nk, N, wE, wk,
-                                                                                 (const Cx<double>*)GL, pop);
-  } else {
-    current_partial_kernel<float><<<OBS_CTAS, OBS_THREADS, 0, st>>>(NE, Nk, N, wE, wk, (const Cx<float>*)SG,
-                                                                    (const Cx<float>*)SL, (const Cx<float>*)GL,
-                                                                    (const Cx<float>*)GG, cur);
-    population_partial_kernel<float><<<dim3(OBS_CTAS, N), OBS_THREADS, 0, st>>>(NE, Nk, N, wE, wk,
-                                                                                (const Cx<float>*)GL, pop);
-  }
-  observables_combine_kernel<<<1 + N, 128, 0, st>>>(N, OBS_CTAS, cur, pop, gs, target, out);
+  const long long g = ((long long)NE * Nk + OBS_THREADS - 1) / OBS_THREADS;
+  const dim3 grid((unsigned)(g < OBS_CTAS ? g : OBS_CTAS), (N * N < OBS_SLICES ? N * N : OBS_SLICES) + 1);
+  unsigned* counter = (unsigned*)(partial + observables_partial_doubles(N) - 1);
+  if (precision == QCL_C128)
+    observables_kernel<double><<<grid, OBS_THREADS, 0, st>>>(NE, Nk, N, wE, wk, (const Cx<double>*)SG,
+                                                             (const Cx<double>*)SL, (const Cx<double>*)GL,
+                                                             (const Cx<double>*)GG, gs, target, partial, counter, out);
+  else
+    observables_kernel<float><<<grid, OBS_THREADS, 0, st>>>(NE, Nk, N, wE, wk, (const Cx<float>*)SG,
+                                                            (const Cx<float>*)SL, (const Cx<float>*)GL,
+                                                            (const Cx<float>*)GG, gs, target, partial, counter, out);
   QCL_LAUNCH_CHECK("observables");
   return QCL_OK;
 }

@@ -103,9 +103,8 @@ int launch_weighted_trace(int NE, int Nk, const void* tr, const double* wE, cons
 // move G> weight into it); 1 or 2 forces the first or the second form (its
 // formula continued across the switch), for a derivative whose explicit part
 // must stay on the branch of the fixed point.
-__global__ void paired_coefficients_kernel(const double* trL, const double* trG, int gs, double target,
-                                           double limit, double* coeffs, int* status, int scalar, int branch) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ void paired_coefficients(const double* trL, const double* trG, int gs, double target, double limit,
+                                    double* coeffs, int* status, int scalar, int branch) {
   const double pre = gs / (2.0 * M_PI);
   // -i * pre * (x + i y) = pre * (y - i x)
   const double Nre = pre * trL[1], Nim = -pre * trL[0];
@@ -149,6 +148,69 @@ __global__ void paired_coefficients_kernel(const double* trL, const double* trG,
   coeffs[0] = a;
   coeffs[1] = c;
   coeffs[2] = lam;
+}
+
+__global__ void paired_coefficients_kernel(const double* trL, const double* trG, int gs, double target,
+                                           double limit, double* coeffs, int* status, int scalar, int branch) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  paired_coefficients(trL, trG, gs, target, limit, coeffs, status, scalar, branch);
+}
+
+// Both weighted traces and the coefficients in one launch: every CTA leaves
+// its partial sums, and the CTA that finishes last adds them in CTA order (so
+// the result does not depend on which one that is) and forms the
+// coefficients.  `counter` is zero before and after.
+__device__ __forceinline__ bool last_cta(unsigned* counter, unsigned count) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == count - 1;
+    if (last) *counter = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+__global__ void __launch_bounds__(REDUCE_THREADS)
+    trace_coefficients_kernel(int NE, int Nk, const Cx<double>* __restrict__ trL, const Cx<double>* __restrict__ trG,
+                              const double* __restrict__ wE, const double* __restrict__ wk, double* partial,
+                              unsigned* counter, int gs, double target, double limit, double* traces, double* coeffs,
+                              int* status, int scalar, int branch) {
+  const long long n = (long long)NE * Nk;
+  double v[4] = {0, 0, 0, 0};
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double w = wE[i % NE] * wk[i / NE];
+    const Cx<double> l = trL[i], g = trG[i];
+    v[0] += w * l.x;
+    v[1] += w * l.y;
+    v[2] += w * g.x;
+    v[3] += w * g.y;
+  }
+  block_sum<4>(v);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 4; ++k) partial[4 * blockIdx.x + k] = v[k];
+  if (!last_cta(counter, gridDim.x)) return;
+  for (int k = 0; k < 4; ++k) v[k] = 0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+    for (int k = 0; k < 4; ++k) v[k] += __ldcg(partial + 4 * i + k);
+  block_sum<4>(v);
+  if (threadIdx.x != 0) return;
+  for (int k = 0; k < 4; ++k) traces[k] = v[k];
+  paired_coefficients(traces, traces + 2, gs, target, limit, coeffs, status, scalar, branch);
+}
+
+// traces: 4 doubles (sum wE wk tr G<, then G>); partial: 4 x 296 doubles.
+int launch_trace_coefficients(int NE, int Nk, const void* trL, const void* trG, const double* wE, const double* wk,
+                              double* partial, unsigned* counter, int gs, double target, double realness_limit,
+                              double* traces, double* coeffs, int* status, int scalar, int branch, cudaStream_t st) {
+  const long long n = (long long)NE * Nk, g = (n + REDUCE_THREADS - 1) / REDUCE_THREADS;
+  trace_coefficients_kernel<<<(unsigned)(g < REDUCE_CTAS ? g : REDUCE_CTAS), REDUCE_THREADS, 0, st>>>(
+      NE, Nk, (const Cx<double>*)trL, (const Cx<double>*)trG, wE, wk, partial, counter, gs, target, realness_limit,
+      traces, coeffs, status, scalar, branch);
+  QCL_LAUNCH_CHECK("trace_coefficients");
+  return QCL_OK;
 }
 
 // realness_limit: _NUMBER_FUNCTIONAL_REALNESS_LIMIT = 1e-10 (domain/
@@ -261,61 +323,93 @@ int launch_density_matrix(int precision, int NE, int Nk, int N, const void* GL, 
 // production_operators.jl:1447-1473): out = sum_j src[j].
 // ---------------------------------------------------------------------------
 template <typename R> struct SumArgs {
-  const Cx<R>* src[8];
-  int count;
-  Cx<R>* out;
+  const Cx<R>* src[3][8];
+  Cx<R>* out[3];
   size_t n;
 };
 
-template <typename R> __global__ void sum_fields_kernel(SumArgs<R> p) {
+// COUNT sources (compile time: all loads of an element in flight at once) and
+// up to three outputs, one per blockIdx.y.
+template <typename R, int COUNT> __global__ void sum_fields_kernel(const __grid_constant__ SumArgs<R> p) {
+  const Cx<R>* const* src = p.src[blockIdx.y];
+  Cx<R>* out = p.out[blockIdx.y];
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < p.n; i += (size_t)gridDim.x * blockDim.x) {
-    Cx<R> v = p.src[0][i];
-    for (int j = 1; j < p.count; ++j) v = v + p.src[j][i];
-    p.out[i] = v;
+    Cx<R> x[COUNT];
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) x[j] = src[j][i];
+    Cx<R> v = x[0];
+#pragma unroll
+    for (int j = 1; j < COUNT; ++j) v = v + x[j];
+    out[i] = v;
   }
 }
 // complex64 with 16-byte aligned fields and even n: two elements per 16-byte
 // access (the same per-element sums)
-__global__ void sum_fields_pair_kernel(SumArgs<float> p) {
+template <int COUNT> __global__ void sum_fields_pair_kernel(const __grid_constant__ SumArgs<float> p) {
   const size_t n2 = p.n / 2;
+  const Cx<float>* const* src = p.src[blockIdx.y];
+  float4* out = reinterpret_cast<float4*>(p.out[blockIdx.y]);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n2; i += (size_t)gridDim.x * blockDim.x) {
-    float4 v = reinterpret_cast<const float4*>(p.src[0])[i];
-    for (int j = 1; j < p.count; ++j) {
-      const float4 w = reinterpret_cast<const float4*>(p.src[j])[i];
-      v.x += w.x;
-      v.y += w.y;
-      v.z += w.z;
-      v.w += w.w;
+    float4 x[COUNT];
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) x[j] = reinterpret_cast<const float4*>(src[j])[i];
+    float4 v = x[0];
+#pragma unroll
+    for (int j = 1; j < COUNT; ++j) {
+      v.x += x[j].x;
+      v.y += x[j].y;
+      v.z += x[j].z;
+      v.w += x[j].w;
     }
-    reinterpret_cast<float4*>(p.out)[i] = v;
+    out[i] = v;
   }
 }
 static bool aligned16(const void* q) { return ((uintptr_t)q & 15u) == 0; }
 
-int launch_sum_fields(int precision, size_t n, const void* const* src, int count, void* out, cudaStream_t st) {
-  if (count < 1 || count > 8) {
-    set_last_error("sum_fields: 1..8 inputs supported, got %d", count);
+template <int COUNT>
+static void sum_fields_t(int precision, size_t n, const void* const (*src)[8], void* const* out, int comps,
+                         cudaStream_t st) {
+  if (precision == QCL_C128) {
+    SumArgs<double> a{};
+    for (int k = 0; k < comps; ++k) {
+      for (int j = 0; j < COUNT; ++j) a.src[k][j] = (const Cx<double>*)src[k][j];
+      a.out[k] = (Cx<double>*)out[k];
+    }
+    a.n = n;
+    sum_fields_kernel<double, COUNT><<<dim3(grid_for(n, 256), comps), 256, 0, st>>>(a);
+    return;
+  }
+  SumArgs<float> a{};
+  bool pairs = n % 2 == 0;
+  for (int k = 0; k < comps; ++k) {
+    for (int j = 0; j < COUNT; ++j) {
+      a.src[k][j] = (const Cx<float>*)src[k][j];
+      pairs = pairs && aligned16(src[k][j]);
+    }
+    a.out[k] = (Cx<float>*)out[k];
+    pairs = pairs && aligned16(out[k]);
+  }
+  a.n = n;
+  if (pairs) sum_fields_pair_kernel<COUNT><<<dim3(grid_for(n / 2, 256), comps), 256, 0, st>>>(a);
+  else sum_fields_kernel<float, COUNT><<<dim3(grid_for(n, 256), comps), 256, 0, st>>>(a);
+}
+
+// out[k] = sum_j src[k][j], j < count, for the `comps` components.
+int launch_sum_fields(int precision, size_t n, const void* const (*src)[8], int count, void* const* out, int comps,
+                      cudaStream_t st) {
+  if (count < 1 || count > 8 || comps < 1 || comps > 3) {
+    set_last_error("sum_fields: 1..8 inputs and 1..3 components supported, got %d, %d", count, comps);
     return QCL_ARG;
   }
-  if (precision == QCL_C128) {
-    SumArgs<double> a;
-    for (int j = 0; j < count; ++j) a.src[j] = (const Cx<double>*)src[j];
-    a.count = count;
-    a.out = (Cx<double>*)out;
-    a.n = n;
-    sum_fields_kernel<double><<<grid_for(n, 256), 256, 0, st>>>(a);
-  } else {
-    SumArgs<float> a;
-    bool pairs = n % 2 == 0 && aligned16(out);
-    for (int j = 0; j < count; ++j) {
-      a.src[j] = (const Cx<float>*)src[j];
-      pairs = pairs && aligned16(src[j]);
-    }
-    a.count = count;
-    a.out = (Cx<float>*)out;
-    a.n = n;
-    if (pairs) sum_fields_pair_kernel<<<grid_for(n / 2, 256), 256, 0, st>>>(a);
-    else sum_fields_kernel<float><<<grid_for(n, 256), 256, 0, st>>>(a);
+  switch (count) {
+    case 1: sum_fields_t<1>(precision, n, src, out, comps, st); break;
+    case 2: sum_fields_t<2>(precision, n, src, out, comps, st); break;
+    case 3: sum_fields_t<3>(precision, n, src, out, comps, st); break;
+    case 4: sum_fields_t<4>(precision, n, src, out, comps, st); break;
+    case 5: sum_fields_t<5>(precision, n, src, out, comps, st); break;
+    case 6: sum_fields_t<6>(precision, n, src, out, comps, st); break;
+    case 7: sum_fields_t<7>(precision, n, src, out, comps, st); break;
+    default: sum_fields_t<8>(precision, n, src, out, comps, st);
   }
   QCL_LAUNCH_CHECK("sum_fields");
   return QCL_OK;
@@ -486,6 +580,162 @@ int launch_residual_mix_multi(int precision, size_t n, const void* const* old, v
   combine_segments_kernel<<<nf, REDUCE_THREADS, 0, st>>>(partial, MIX_CTAS, out);
   QCL_LAUNCH_CHECK("residual_mix_multi");
   return QCL_OK;
+}
+
+// ---------------------------------------------------------------------------
+// The end of an iteration with linear mixing, one pass over the F families'
+// state and candidate fields (blockIdx.y: component):
+//   per family   (|new - old|^2, |new|^2)              (residual_mix_multi_kernel)
+//   plus + minus (|d(n1 + n2)|^2, |n1 + n2|^2)         (the embedding total)
+//   sum_f new, for the component of total_out[], before mixing
+//   new <- (1 - alpha) old + alpha new
+// in place of a pass for each: 2F + 1 field reads and writes fewer per
+// component than the separate sum, pair-residual and mixing passes took (at
+// 7 families of 134 MB: 1.93 -> 1.36 ms).  HBM bound.  VEC elements of 16 bytes
+// per access.  The last CTA adds the partial sums in CTA order.
+// ---------------------------------------------------------------------------
+template <typename R> struct FamilyArgs {
+  const Cx<R>* old[3][7];
+  Cx<R>* cand[3][7];
+  Cx<R>* total[3];  // may be NULL
+  size_t n;
+  double alpha;
+  double* partial;  // [3][gridDim.x][2 F + 2]
+  unsigned* counter;
+  double* fam_out;  // [F][3][2]
+  double* emb_out;  // [3][2]
+};
+template <typename R, int VEC> struct __align__(sizeof(Cx<R>) * VEC) CxVec {
+  Cx<R> v[VEC];
+};
+
+template <typename R, int VEC, int F>
+__global__ void __launch_bounds__(REDUCE_THREADS) mix_families_kernel(const __grid_constant__ FamilyArgs<R> p) {
+  using V = CxVec<R, VEC>;
+  constexpr int Q = 2 * F + 2;
+  const int k = blockIdx.y;
+  double v[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) v[q] = 0;
+  const R al = (R)p.alpha, be = (R)(1.0 - p.alpha);
+  V* total = reinterpret_cast<V*>(p.total[k]);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < p.n / VEC; i += (size_t)gridDim.x * blockDim.x) {
+    V o[F], c[F];
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      o[f] = reinterpret_cast<const V*>(p.old[k][f])[i];
+      c[f] = reinterpret_cast<const V*>(p.cand[k][f])[i];
+    }
+#pragma unroll
+    for (int h = 0; h < VEC; ++h) {
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const Cx<R> a = o[f].v[h], b = c[f].v[h];
+        const double dx = (double)b.x - a.x, dy = (double)b.y - a.y;
+        const double d2 = dx * dx + dy * dy, n2 = (double)b.x * b.x + (double)b.y * b.y;
+        if (isfinite(d2) && isfinite(n2) && isfinite((double)a.x) && isfinite((double)a.y)) {
+          v[2 * f] += d2;
+          v[2 * f + 1] += n2;
+        } else {
+          v[2 * f] = INFINITY;
+        }
+      }
+      const Cx<R> o1 = o[F - 2].v[h], o2 = o[F - 1].v[h], n1 = c[F - 2].v[h], n2 = c[F - 1].v[h];
+      const double nx = (double)n1.x + n2.x, ny = (double)n1.y + n2.y;
+      const double dx = nx - ((double)o1.x + o2.x), dy = ny - ((double)o1.y + o2.y);
+      const double d2 = dx * dx + dy * dy, s2 = nx * nx + ny * ny;
+      if (isfinite(d2) && isfinite(s2)) {
+        v[Q - 2] += d2;
+        v[Q - 1] += s2;
+      } else {
+        v[Q - 2] = INFINITY;
+      }
+    }
+    if (total) {
+      V t = c[0];
+#pragma unroll
+      for (int f = 1; f < F; ++f)
+#pragma unroll
+        for (int h = 0; h < VEC; ++h) t.v[h] = t.v[h] + c[f].v[h];
+      total[i] = t;
+    }
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+#pragma unroll
+      for (int h = 0; h < VEC; ++h) {
+        const Cx<R> a = o[f].v[h], b = c[f].v[h];
+        c[f].v[h] = cx<R>(be * a.x + al * b.x, be * a.y + al * b.y);
+      }
+      reinterpret_cast<V*>(p.cand[k][f])[i] = c[f];
+    }
+  }
+  block_sum<Q>(v);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < Q; ++q) p.partial[((size_t)k * gridDim.x + blockIdx.x) * Q + q] = v[q];
+  if (!last_cta(p.counter, gridDim.x * gridDim.y)) return;
+  for (int j = threadIdx.x >> 5; j < 3 * Q; j += REDUCE_THREADS / 32) {  // one warp per sum
+    const int kk = j / Q, q = j % Q;
+    double s = 0;
+    for (int i = threadIdx.x & 31; i < (int)gridDim.x; i += 32)
+      s += __ldcg(p.partial + ((size_t)kk * gridDim.x + i) * Q + q);
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) {
+      if (q < 2 * F) p.fam_out[2 * (3 * (q / 2) + kk) + q % 2] = s;
+      else p.emb_out[2 * kk + q - 2 * F] = s;
+    }
+  }
+}
+
+constexpr int MIX_FAMILY_CTAS = 296;  // per component
+size_t mix_families_partial_doubles() { return 3 * (size_t)MIX_FAMILY_CTAS * 16; }
+
+template <typename R, int VEC>
+static int mix_families_t(const FamilyArgs<R>& a, int F, cudaStream_t st) {
+  const size_t g = (a.n / VEC + REDUCE_THREADS - 1) / REDUCE_THREADS;
+  const dim3 grid((unsigned)(g < MIX_FAMILY_CTAS ? (g > 0 ? g : 1) : MIX_FAMILY_CTAS), 3);
+  switch (F) {
+    case 2: mix_families_kernel<R, VEC, 2><<<grid, REDUCE_THREADS, 0, st>>>(a); break;
+    case 3: mix_families_kernel<R, VEC, 3><<<grid, REDUCE_THREADS, 0, st>>>(a); break;
+    case 4: mix_families_kernel<R, VEC, 4><<<grid, REDUCE_THREADS, 0, st>>>(a); break;
+    case 5: mix_families_kernel<R, VEC, 5><<<grid, REDUCE_THREADS, 0, st>>>(a); break;
+    case 6: mix_families_kernel<R, VEC, 6><<<grid, REDUCE_THREADS, 0, st>>>(a); break;
+    case 7: mix_families_kernel<R, VEC, 7><<<grid, REDUCE_THREADS, 0, st>>>(a); break;
+    default: set_last_error("mix_families: 2..7 families supported, got %d", F); return QCL_ARG;
+  }
+  QCL_LAUNCH_CHECK("mix_families");
+  return QCL_OK;
+}
+
+// old / cand: [3 f + k]; total: component 1 (the candidate total lesser).
+int launch_mix_families(int precision, size_t n, const void* const* old, void* const* cand, int F, void* total_lesser,
+                        double alpha, double* partial, unsigned* counter, double* fam_out, double* emb_out,
+                        cudaStream_t st) {
+  auto fill = [&](auto& a, auto tag) {
+    using C = decltype(tag);
+    a.n = n;
+    a.alpha = alpha;
+    a.partial = partial;
+    a.counter = counter;
+    a.fam_out = fam_out;
+    a.emb_out = emb_out;
+    for (int f = 0; f < F && f < 7; ++f)
+      for (int k = 0; k < 3; ++k) {
+        a.old[k][f] = (const C*)old[3 * f + k];
+        a.cand[k][f] = (C*)cand[3 * f + k];
+      }
+    a.total[1] = (C*)total_lesser;
+  };
+  if (precision == QCL_C128) {
+    FamilyArgs<double> a{};
+    fill(a, Cx<double>{});
+    return mix_families_t<double, 1>(a, F, st);
+  }
+  FamilyArgs<float> a{};
+  fill(a, Cx<float>{});
+  bool pairs = n % 2 == 0 && aligned16(total_lesser);
+  for (int i = 0; i < 3 * F; ++i) pairs = pairs && aligned16(old[i]) && aligned16(cand[i]);
+  return pairs ? mix_families_t<float, 2>(a, F, st) : mix_families_t<float, 1>(a, F, st);
 }
 
 int launch_combine(const double* partial, int count, int K, double* out, cudaStream_t st) {

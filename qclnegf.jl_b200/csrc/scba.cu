@@ -81,7 +81,10 @@ enum {
   SC_OBS = 20,     // 2 + N: Jbar, Im, populations
   SC_FAM = 20 + 2 + 48,  // (M + 2) families x 3 components x (num, den)
   SC_ROUND = SC_FAM + 7 * 3 * 2,  // M x (num, den) Hilbert roundoff
-  SC_TOTAL = SC_ROUND + 5 * 2
+  SC_STATUS = SC_ROUND + 5 * 2,   // the status words (two ints)
+  SC_TOTAL = SC_STATUS + 1,
+  SC_COUNTERS = SC_TOTAL,         // CTA counters of the one-launch reductions (not downloaded)
+  SC_ALLOC = SC_COUNTERS + 1
 };
 
 // Phases of an iteration, in the reference's names (production_solver.jl:438-590,
@@ -136,7 +139,8 @@ struct ScbaCtx {
   double* obspartial = nullptr;
   double* scal = nullptr;
   double* scal_h = nullptr;  // pinned
-  int* status = nullptr;
+  int* status = nullptr;        // in scal (SC_STATUS)
+  unsigned* counters = nullptr;  // in scal (SC_COUNTERS): traces, mixing
   HilbertTables hil;
   // graph of one iteration (two parities: state/cand swap)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -297,7 +301,6 @@ void scba_destroy(ScbaCtx* c) {
   cudaFree(c->obspartial);
   cudaFree(c->scal);
   cudaFreeHost(c->scal_h);
-  cudaFree(c->status);
   cudaFree(c->Xh);
   cudaFree(c->Rh);
   cudaFree(c->ameta);
@@ -382,8 +385,8 @@ static int plan_memory(const qcl_scba_problem* p, const qcl_mechanism* mechs, Me
     if (p->refinement && !c128) cwork = std::max(cwork, op_work_elems(q, QCL_C128, NE, Nk, N) * 16);
   }
   const int L = next_pow2(2 * NE - 1);
-  mp->workspace = cwork + 2 * (size_t)NE * Nk * 16 + (size_t)kReduceCtas * 2 * 8 +
-                  residual_mix_multi_partial_doubles(3 * (M + 2)) * 8 + residual_work_doubles(NE, Nk) * 8 +
+  mp->workspace = cwork + 2 * (size_t)NE * Nk * 16 + (size_t)kReduceCtas * 4 * 8 +
+                  std::max(residual_mix_multi_partial_doubles(3 * (M + 2)), mix_families_partial_doubles()) * 8 + residual_work_doubles(NE, Nk) * 8 +
                   observables_partial_doubles(N) * 8 + 4096 /* scalars, status */ +
                   (size_t)16 * 16 * L /* FFT tables */ + (size_t)Nk * N * N * 2 * 8 /* per-column partials */;
   if (p->mixing)
@@ -627,19 +630,21 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
   c->cwork_bytes = cwork;
   TRY(dalloc((void**)&c->trL, (size_t)c->NE * c->Nk * 16));
   TRY(dalloc((void**)&c->trG, (size_t)c->NE * c->Nk * 16));
-  TRY(dalloc((void**)&c->rpartial, kReduceCtas * 2 * sizeof(double)));
-  TRY(dalloc((void**)&c->mpartial, residual_mix_multi_partial_doubles(3 * (c->M + 2)) * sizeof(double)));
+  TRY(dalloc((void**)&c->rpartial, kReduceCtas * 4 * sizeof(double)));
+  TRY(dalloc((void**)&c->mpartial, std::max(residual_mix_multi_partial_doubles(3 * (c->M + 2)),
+                                            mix_families_partial_doubles()) * sizeof(double)));
   TRY(dalloc((void**)&c->reswork, residual_work_doubles(c->NE, c->Nk) * sizeof(double)));
   TRY(dalloc((void**)&c->obspartial, observables_partial_doubles(c->N) * sizeof(double)));
-  TRY(dalloc((void**)&c->scal, SC_TOTAL * sizeof(double)));
+  QCL_CUDA_CHECK(cudaMemsetAsync(c->obspartial, 0, observables_partial_doubles(c->N) * sizeof(double), c->st));
+  TRY(dalloc((void**)&c->scal, SC_ALLOC * sizeof(double)));
   {
     cudaError_t e = cudaMallocHost((void**)&c->scal_h, SC_TOTAL * sizeof(double));
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaMallocHost"));
   }
-  TRY(dalloc((void**)&c->status, 2 * sizeof(int)));
-  QCL_CUDA_CHECK(cudaMemsetAsync(c->status, 0, 2 * sizeof(int), c->st));
+  QCL_CUDA_CHECK(cudaMemsetAsync(c->scal, 0, SC_ALLOC * sizeof(double), c->st));
+  c->status = (int*)(c->scal + SC_STATUS);
+  c->counters = (unsigned*)(c->scal + SC_COUNTERS);
   for (auto& m : c->mech) m.status = c->status;
-  QCL_CUDA_CHECK(cudaMemsetAsync(c->scal, 0, SC_TOTAL * sizeof(double), c->st));
   if (c->mixing) {
     const size_t nf = 3 * (size_t)(c->M + 2);
     TRY(dalloc(&c->Xh, (size_t)c->and_depth * nf * c->fcap));
@@ -733,30 +738,24 @@ static int embedding_candidates(ScbaCtx* c, std::vector<void*>& dst, const void*
   return launch_sandwich(cp, c->NE, c->Nk, c->N, jobs, 2, c->st);
 }
 
-static int totals(ScbaCtx* c, const std::vector<void*>& fam, void* const* out, int comps_mask) {
+static int totals(ScbaCtx* c, const std::vector<void*>& fam, void* const* out) {
   const int F = c->M + 2;
-  for (int k = 0; k < 3; ++k) {
-    if (!(comps_mask & (1 << k))) continue;
-    const void* src[8];
-    for (int f = 0; f < F; ++f) src[f] = field_of(fam, f, k);
-    int s = launch_sum_fields(c->precision == QCL_MIXED ? QCL_C64 : c->precision, c->nfield, src, F, out[k], c->st);
-    if (s) return s;
-  }
-  return QCL_OK;
+  const void* src[3][8];
+  for (int k = 0; k < 3; ++k)
+    for (int f = 0; f < F; ++f) src[k][f] = field_of(fam, f, k);
+  return launch_sum_fields(c->precision == QCL_MIXED ? QCL_C64 : c->precision, c->nfield, src, F, out, 3, c->st);
 }
 
 // The current Green state from the state families (_current_green_production).
 static int current_green(ScbaCtx* c, const std::vector<void*>& fam) {
   int s;
-  if ((s = totals(c, fam, c->tot, 7))) return s;
+  if ((s = totals(c, fam, c->tot))) return s;
   if ((s = launch_dyson_keldysh(c->precision, c->NE, c->Nk, c->N, c->eps, 0.0, c->h, c->tot[0], c->tot[1], c->tot[2],
                                 c->GR, c->GL, c->GG, nullptr, c->trL, c->trG, c->status, c->st)))
     return s;
-  if ((s = launch_weighted_trace(c->NE, c->Nk, c->trL, c->wE, c->wk, c->rpartial, c->scal + SC_TRL, c->st))) return s;
-  if ((s = launch_weighted_trace(c->NE, c->Nk, c->trG, c->wE, c->wk, c->rpartial, c->scal + SC_TRG, c->st))) return s;
-  if ((s = launch_paired_coefficients(c->scal + SC_TRL, c->scal + SC_TRG, c->gs, c->target, c->scal + SC_COEF,
-                                      c->status, c->st, c->precision == QCL_C128 ? 1e-10 : 1e-5, c->scalar_lesser,
-                                      c->norm_branch)))
+  if ((s = launch_trace_coefficients(c->NE, c->Nk, c->trL, c->trG, c->wE, c->wk, c->rpartial, c->counters, c->gs,
+                                     c->target, c->precision == QCL_C128 ? 1e-10 : 1e-5, c->scal + SC_TRL,
+                                     c->scal + SC_COEF, c->status, c->scalar_lesser, c->norm_branch, c->st)))
     return s;
   const int sp = c->precision == QCL_MIXED ? QCL_C64 : c->precision;
   if (c->scalar_lesser) return launch_scalar_lesser(sp, c->NE, c->Nk, c->N, c->GR, c->GL, c->GG, c->scal + SC_COEF, c->st);
@@ -798,32 +797,6 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
   if ((s = phase_mark(c, 2))) return s;
   if ((s = embedding_candidates(c, cand))) return s;
   if ((s = phase_mark(c, 3))) return s;
-  // candidate total lesser for r_K
-  {
-    const void* src[8];
-    const int F = c->M + 2;
-    for (int f = 0; f < F; ++f) src[f] = field_of(cand, f, 1);
-    if ((s = launch_sum_fields(sp, c->nfield, src, F, c->candSL, c->st))) return s;
-  }
-  if ((s = phase_mark(c, 4))) return s;
-  if ((s = launch_residual_blocks(c->precision, RES_PART_RK, c->NE, c->Nk, c->N, c->eps, c->h, c->GR, c->GL, c->GG,
-                                  c->tot[0], c->tot[1], c->tot[2], c->candSL, c->reswork, c->st)))
-    return s;
-  QCL_CUDA_CHECK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
-  if ((s = launch_residual_reduce(c->NE, c->Nk, c->reswork, c->scal + SC_RES, c->st))) return s;
-  // embedding-total residual (before the plus/minus candidates are mixed over)
-  for (int k = 0; k < 3; ++k)
-    if ((s = launch_residual_pair(sp, c->nfield, field_of(state, c->M, k), field_of(state, c->M + 1, k),
-                                  field_of(cand, c->M, k), field_of(cand, c->M + 1, k), c->rpartial,
-                                  c->scal + SC_EMB + 2 * k, c->st)))
-      return s;
-  if ((s = phase_mark(c, 5))) return s;
-  // J from the (unmixed) plus family and the state's G
-  if ((s = launch_observables(sp, c->NE, c->Nk, c->N, c->wE, c->wk, field_of(state, c->M, 2), field_of(state, c->M, 1),
-                              c->GL, c->GG, c->gs, c->target, c->obspartial, c->scal + SC_OBS, c->st)))
-    return s;
-  if ((s = phase_mark(c, 6))) return s;
-  // per-family residual + speculative linear mixing into the candidate buffers
   const int F = c->M + 2;
   const void* olds[kMaxMixFields];
   void* cands[kMaxMixFields];
@@ -832,7 +805,45 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
       olds[3 * f + k] = field_of(state, f, k);
       cands[3 * f + k] = field_of(cand, f, k);
     }
-  if (c->mixing) {
+  // r_K against the candidate total lesser, the reduction of the suite, J and
+  // populations (from the unmixed plus family and the state's G)
+  const auto residuals = [&]() -> int {
+    if ((s = launch_residual_blocks(c->precision, RES_PART_RK, c->NE, c->Nk, c->N, c->eps, c->h, c->GR, c->GL, c->GG,
+                                    c->tot[0], c->tot[1], c->tot[2], c->candSL, c->reswork, c->st)))
+      return s;
+    QCL_CUDA_CHECK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
+    return launch_residual_reduce(c->NE, c->Nk, c->reswork, c->scal + SC_RES, c->st);
+  };
+  const auto observables = [&](cudaStream_t st) {
+    return launch_observables(sp, c->NE, c->Nk, c->N, c->wE, c->wk, field_of(state, c->M, 2), field_of(state, c->M, 1),
+                              c->GL, c->GG, c->gs, c->target, c->obspartial, c->scal + SC_OBS, st);
+  };
+  if (!c->mixing) {
+    // the candidate total, the residuals of every family and of the embedding
+    // total, and the speculative mixing into the candidate buffers: one pass
+    if ((s = launch_mix_families(sp, c->nfield, olds, cands, F, c->candSL, c->alpha, c->mpartial, c->counters + 1,
+                                 c->scal + SC_FAM, c->scal + SC_EMB, c->st)))
+      return s;
+    if ((s = phase_mark(c, 4))) return s;
+    if ((s = residuals())) return s;
+    if ((s = phase_mark(c, 5))) return s;
+    if ((s = observables(c->st))) return s;
+    if ((s = phase_mark(c, 6))) return s;
+  } else {
+    const void* src[1][8];
+    for (int f = 0; f < F; ++f) src[0][f] = field_of(cand, f, 1);
+    if ((s = launch_sum_fields(sp, c->nfield, src, F, &c->candSL, 1, c->st))) return s;
+    if ((s = phase_mark(c, 4))) return s;
+    if ((s = residuals())) return s;
+    // embedding-total residual (before the plus/minus candidates are mixed over)
+    for (int k = 0; k < 3; ++k)
+      if ((s = launch_residual_pair(sp, c->nfield, field_of(state, c->M, k), field_of(state, c->M + 1, k),
+                                    field_of(cand, c->M, k), field_of(cand, c->M + 1, k), c->rpartial,
+                                    c->scal + SC_EMB + 2 * k, c->st)))
+        return s;
+    if ((s = phase_mark(c, 5))) return s;
+    if ((s = observables(c->st))) return s;
+    if ((s = phase_mark(c, 6))) return s;
     // Anderson mixing with the causality guard (production_mixing.jl:224-317)
     const int nf = 3 * F;
     if ((s = launch_anderson_plan(c->ameta, c->and_depth, c->st))) return s;
@@ -851,9 +862,6 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
       if ((s = launch_anderson_after_guard(c->ameta, pass, c->status, c->st))) return s;
     }
     QCL_CUDA_CHECK(cudaMemcpyAsync(c->ameta_h, c->ameta, sizeof(AndersonMeta), cudaMemcpyDeviceToHost, c->st));
-  } else if ((s = launch_residual_mix_multi(sp, c->nfield, olds, cands, 3 * F, c->alpha, c->mpartial,
-                                            c->scal + SC_FAM, c->st))) {
-    return s;
   }
   if ((s = phase_mark(c, 7))) return s;
   QCL_CUDA_CHECK(cudaMemcpyAsync(c->scal_h, c->scal, SC_TOTAL * sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -1045,9 +1053,9 @@ int scba_step_finish(ScbaCtx* c, qcl_scba_row* row) {
       QCL_CUDA_CHECK(cudaEventElapsedTime(&ms, c->pev[i], c->pev[i + 1]));
       c->phase_ms[i] = ms;
     }
-  int hst[2];
-  QCL_CUDA_CHECK(cudaMemcpy(hst, c->status, sizeof(hst), cudaMemcpyDeviceToHost));
   const double* h = c->scal_h;
+  int hst[2];
+  memcpy(hst, h + SC_STATUS, sizeof(hst));
   c->nu += 1;
   memset(row, 0, sizeof(*row));
   row->nu = c->nu;
@@ -1690,7 +1698,7 @@ int scba_tangent_step(ScbaCtx* c, double* out) {
   const int F = c->M + 2, nf = 3 * F, NE = c->NE, Nk = c->Nk, N = c->N;
   std::vector<void*>& st = c->parity == 0 ? c->state : c->cand;  // the linearisation point
   // tangent totals
-  if ((s = totals(c, c->tv, c->ttot, 7))) return s;
+  if ((s = totals(c, c->tv, c->ttot))) return s;
   // Dyson + Keldysh tangent
   void *X = c->tG[0], *dL = c->tG[1], *dG = c->tG[2];
   if ((s = launch_block_triple(NE, Nk, N, c->GR, c->ttot[0], c->GR, 0, 1.0, 0.0, X, nullptr, c->st))) return s;
