@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <chrono>
 #include <map>
+#include <mutex>
 #include <vector>
 
 #include "kernels.cuh"
@@ -52,6 +53,11 @@ struct Mech {
   int* status = nullptr;
   void* i8_work = nullptr;  // the context's work area of the integer tensor path
   size_t i8_bytes = 0;
+  // the stream its candidate is built on (-1: the context's own) with its own
+  // contraction scratch and per-column Hilbert sums
+  int branch = -1;
+  void* work = nullptr;
+  double* hpartial = nullptr;
   KernelOpDev view() const {
     KernelOpDev k;
     k.i8_work = i8_work;
@@ -92,6 +98,8 @@ enum {
 // candidate_assembly, residuals, observables, mixing.
 constexpr int kPhases = 7;
 
+constexpr int kBranches = 3;  // the mechanisms take turns on all but the last, the embedding has the last
+
 struct ScbaCtx {
   int NE, Nk, N, M, precision, gs, verify;
   int refinement = 0;  // FP64-sized state and complex128 operator copies for qcl_scba_promote
@@ -114,6 +122,7 @@ struct ScbaCtx {
   size_t nfield, fbytes;  // elements per field, bytes per field at the active precision
   size_t fcap = 0;        // allocated bytes per field (complex128 size in refinement contexts)
   cudaStream_t st = nullptr;
+  int dev = 0;
   // grids and operators
   double *eps = nullptr, *wE = nullptr, *wk = nullptr;
   void *h = nullptr, *Tp = nullptr, *Tm = nullptr;
@@ -126,6 +135,7 @@ struct ScbaCtx {
   void *tot[3] = {nullptr, nullptr, nullptr};
   void* candSL = nullptr;
   void* tmp = nullptr;
+  void* slab = nullptr;  // small fields share one allocation
   void* cwork = nullptr;
   size_t cwork_bytes = 0;
   void* i8_work = nullptr;  // complex128: work area of the integer tensor path, where the budget has room
@@ -147,6 +157,12 @@ struct ScbaCtx {
   cudaGraph_t gtpl[2] = {nullptr, nullptr};  // the captured iterations (child graphs of a batched sweep)
   cudaStream_t st2 = nullptr;  // side stream of an iteration (forked from st, joined back)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // branches of the candidate construction (mechanisms, embedding), forked
+  // from st and joined back; br_area holds the branches' scratch
+  cudaStream_t br_st[kBranches] = {};
+  cudaEvent_t br_done[kBranches] = {}, br_fork = nullptr;
+  void* br_area = nullptr;
+  size_t br_bytes = 0;
   bool use_graph = false;
   // phase telemetry: device time between CUDA events at the phase boundaries of an
   // iteration (the :phase_begin / :phase_end events of production_telemetry.jl:81-200)
@@ -172,6 +188,45 @@ struct ScbaCtx {
   bool have_residual = false;  // reswork holds the per-block residual outputs of the last step
   double green_eta = 0;
 };
+
+// Streams of closed contexts, kept for the next one on the same device (a
+// stream costs more to create than a small iteration takes to run).  At most
+// kIdleStreams are kept; they are idle and carry no capture.
+constexpr int kIdleStreams = 16;
+static std::mutex g_streams_mutex;
+static std::vector<std::pair<int, cudaStream_t>> g_streams;
+
+static cudaError_t take_stream(cudaStream_t* st) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  {
+    std::lock_guard<std::mutex> lock(g_streams_mutex);
+    for (size_t i = 0; i < g_streams.size(); ++i)
+      if (g_streams[i].first == dev) {
+        *st = g_streams[i].second;
+        g_streams.erase(g_streams.begin() + i);
+        return cudaSuccess;
+      }
+  }
+  return cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+}
+
+// Gives a stream of the context on device `dev` back.
+static void give_stream(int dev, cudaStream_t st) {
+  if (!st) return;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+      cudaStreamQuery(st) == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(g_streams_mutex);
+    if (g_streams.size() < kIdleStreams) {
+      g_streams.push_back({dev, st});
+      return;
+    }
+  }
+  cudaGetLastError();
+  cudaStreamDestroy(st);
+}
 
 static void* field_of(const std::vector<void*>& v, int f, int c) { return v[3 * f + c]; }
 int scba_step_launch(ScbaCtx* c, cudaGraph_t* child);
@@ -273,8 +328,12 @@ void scba_destroy(ScbaCtx* c) {
     for (void* q : m.tc_stage1) cudaFree(q);
     for (void* q : {m.block64, m.matrix64, m.left64, m.right64, m.radial64}) cudaFree(q);
   }
-  for (void* p : c->state) cudaFree(p);
-  for (void* p : c->cand) cudaFree(p);
+  if (!c->slab) {
+    for (void* p : c->state) cudaFree(p);
+    for (void* p : c->cand) cudaFree(p);
+    for (void* p : {c->GR, c->GL, c->GG, c->tot[0], c->tot[1], c->tot[2], c->candSL, c->tmp}) cudaFree(p);
+  }
+  cudaFree(c->slab);
   for (auto* v : {&c->tv, &c->tw, &c->tsrc})
     for (void* p : *v) cudaFree(p);
   for (int k = 0; k < 3; ++k) {
@@ -285,14 +344,9 @@ void scba_destroy(ScbaCtx* c) {
   cudaFree(c->ttrG);
   cudaFree(c->tscal);
   if (c->tscal_h) cudaFreeHost(c->tscal_h);
-  cudaFree(c->GR);
-  cudaFree(c->GL);
-  cudaFree(c->GG);
-  for (auto p : c->tot) cudaFree(p);
-  cudaFree(c->candSL);
-  cudaFree(c->tmp);
   cudaFree(c->cwork);
   cudaFree(c->i8_work);
+  cudaFree(c->br_area);
   cudaFree(c->trL);
   cudaFree(c->trG);
   cudaFree(c->rpartial);
@@ -311,8 +365,13 @@ void scba_destroy(ScbaCtx* c) {
     if (e) cudaEventDestroy(e);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
-  if (c->st2) cudaStreamDestroy(c->st2);
-  if (c->st) cudaStreamDestroy(c->st);
+  for (int i = 0; i < kBranches; ++i) {
+    if (c->br_done[i]) cudaEventDestroy(c->br_done[i]);
+    give_stream(c->dev, c->br_st[i]);
+  }
+  if (c->br_fork) cudaEventDestroy(c->br_fork);
+  give_stream(c->dev, c->st2);
+  give_stream(c->dev, c->st);
   delete c;
 }
 
@@ -435,6 +494,71 @@ static void i8_area(ScbaCtx* c) {
   }
 }
 
+// Scratch and streams for building the mechanisms' candidates side by side.
+// They are independent given G, and at small sizes each is a chain of kernels
+// that leaves most of the GPU idle; at large ones the branches only fill the
+// ends of each other's launches.  The LO mechanism (whose shifted fields have
+// one buffer), maps on the integer path (one work area) and the largest of the
+// rest stay on the context's stream.  Optional, like i8_area: at most 64 MB
+// (or half a field) and what the budget leaves over; without it the
+// mechanisms run one after another.
+static void branch_area(ScbaCtx* c) {
+  const size_t ncols = (size_t)c->Nk * c->N * c->N;
+  std::vector<size_t> need(c->M, 0);
+  auto align = [](size_t n) { return (n + 255) / 256 * 256; };
+  int keep = -1;
+  bool main_used = false;
+  for (int i = 0; i < c->M; ++i) {
+    const KernelOpDev op = c->mech[i].view();
+    if (c->mech[i].is_LO || (op.i8_work && contraction_i8_bytes(op, c->NE, c->Nk, c->N) > 0)) {
+      main_used = true;
+      continue;
+    }
+    size_t work = contraction_work_elems(op, c->NE, c->Nk, c->N) * (c->precision == QCL_C128 ? 16 : 8);
+    if (c->refinement) {
+      KernelOpDev k64;
+      k64.kind = op.kind;
+      k64.J = op.J;
+      work = std::max(work, contraction_work_elems(k64, c->NE, c->Nk, c->N) * 16);
+    }
+    need[i] = align(work) + align(ncols * 2 * sizeof(double));
+    if (keep < 0 || need[i] > need[keep]) keep = i;
+  }
+  if (!main_used && keep >= 0) need[keep] = 0;
+  size_t cap = std::max<size_t>((size_t)64 << 20, c->fbytes / 2), total = 0, room = 0;
+  const size_t i8 = c->mech.empty() ? 0 : c->mech[0].i8_bytes;
+  if (c->budget) room = c->budget > c->base_peak + i8 ? c->budget - c->base_peak - i8 : 0;
+  else room = cap;  // a failed allocation means one after another
+  cap = std::min(cap, room);
+  int next = 0;
+  for (int i = 0; i < c->M; ++i) {
+    if (need[i] == 0 || total + need[i] > cap) continue;
+    c->mech[i].branch = next++ % (kBranches - 1);
+    total += need[i];
+  }
+  bool ok = total == 0 || cudaMalloc(&c->br_area, total) == cudaSuccess;
+  ok = ok && cudaEventCreateWithFlags(&c->br_fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int i = 0; i < kBranches && ok; ++i)
+    ok = take_stream(&c->br_st[i]) == cudaSuccess &&
+         cudaEventCreateWithFlags(&c->br_done[i], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {  // one after another
+    cudaGetLastError();
+    for (auto& m : c->mech) m.branch = -1;
+    if (c->br_fork) cudaEventDestroy(c->br_fork);
+    c->br_fork = nullptr;
+    return;
+  }
+  c->br_bytes = total;
+  char* q = (char*)c->br_area;
+  for (int i = 0; i < c->M; ++i) {
+    if (c->mech[i].branch < 0) continue;
+    const size_t hp = align(ncols * 2 * sizeof(double));
+    c->mech[i].hpartial = (double*)q;
+    c->mech[i].work = q + hp;
+    q += need[i];
+  }
+}
+
 int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx** out) {
   *out = nullptr;
   if (!p || p->NE < 2 || p->Nk < 1 || p->Nb < 1) {
@@ -550,10 +674,11 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
                             "low-rank operator does not preserve adjoints and positivity"),
              QCL_ARG));
   {
-    cudaError_t e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
+    cudaError_t e = cudaGetDevice(&c->dev);
+    if (e == cudaSuccess) e = take_stream(&c->st);
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaStreamCreate"));
     // the residual suite's G-only part runs beside the candidate construction
-    e = cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking);
+    e = take_stream(&c->st2);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaStreamCreate"));
@@ -616,16 +741,24 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
   const int F = c->M + 2;
   c->state.assign(3 * F, nullptr);
   c->cand.assign(3 * F, nullptr);
-  for (int i = 0; i < 3 * F; ++i) {
-    TRY(dalloc(&c->state[i], c->fcap));
-    TRY(dalloc(&c->cand[i], c->fcap));
+  {
+    // the fields: one allocation each, or, where each would be small (an
+    // allocation costs more than the field's use of it), one for all
+    std::vector<void**> fields;
+    for (int i = 0; i < 3 * F; ++i) {
+      fields.push_back(&c->state[i]);
+      fields.push_back(&c->cand[i]);
+    }
+    for (void** f : {&c->GR, &c->GL, &c->GG, &c->tot[0], &c->tot[1], &c->tot[2], &c->candSL, &c->tmp})
+      fields.push_back(f);
+    const size_t step = (c->fcap + 511) / 512 * 512;
+    if (step <= ((size_t)1 << 20)) {
+      TRY(dalloc(&c->slab, step * fields.size()));
+      for (size_t i = 0; i < fields.size(); ++i) *fields[i] = (char*)c->slab + i * step;
+    } else {
+      for (void** f : fields) TRY(dalloc(f, c->fcap));
+    }
   }
-  TRY(dalloc(&c->GR, c->fcap));
-  TRY(dalloc(&c->GL, c->fcap));
-  TRY(dalloc(&c->GG, c->fcap));
-  for (auto& t : c->tot) TRY(dalloc(&t, c->fcap));
-  TRY(dalloc(&c->candSL, c->fcap));
-  TRY(dalloc(&c->tmp, c->fcap));
   TRY(dalloc(&c->cwork, cwork));
   c->cwork_bytes = cwork;
   TRY(dalloc((void**)&c->trL, (size_t)c->NE * c->Nk * 16));
@@ -661,6 +794,7 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
   c->budget = p->memory_budget_bytes;
   c->base_peak = base_peak;
   i8_area(c);
+  branch_area(c);
 #undef TRY
   QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));
   c->pops.assign(c->N, 0.0);
@@ -671,6 +805,10 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
 // ---------------------------------------------------------------------------
 // Candidate maps (stream-ordered launches; no host synchronisation)
 // ---------------------------------------------------------------------------
+// Whether candidates are built on several streams (phase telemetry times the
+// phases one after another).
+static bool branching(const ScbaCtx* c) { return c->br_fork && !c->telemetry; }
+
 static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, const void* GG, std::vector<void*>& dst,
                                  bool verify) {
   int s;
@@ -678,9 +816,21 @@ static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, con
   // contractions run at storage precision (mixed: FP32 with FP64 k-sums)
   const int cp = p == QCL_MIXED ? QCL_C64 : p;
   const long long ncols = (long long)c->Nk * c->N * c->N;
+  const bool fork = branching(c);
+  unsigned used = 0;  // branches taken
+  if (fork) QCL_CUDA_CHECK(cudaEventRecord(c->br_fork, c->st));
   for (int i = 0; i < c->M; ++i) {
     const Mech& m = c->mech[i];
     const KernelOpDev op = m.view();
+    const bool side = fork && m.branch >= 0;
+    const cudaStream_t st = side ? c->br_st[m.branch] : c->st;
+    void* work = side ? m.work : c->cwork;
+    HilbertTables hil = c->hil;  // shares the tables; the per-column sums are the branch's own
+    if (side) {
+      hil.partial = m.hpartial;
+      if (!(used >> m.branch & 1u)) QCL_CUDA_CHECK(cudaStreamWaitEvent(st, c->br_fork, 0));
+      used |= 1u << m.branch;
+    }
     void* SL = field_of(dst, i, 1);
     void* SG = field_of(dst, i, 2);
     const void* X[2] = {GL, GG};
@@ -702,28 +852,33 @@ static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, con
       X[0] = c->tmp;
       X[1] = c->candSL;
     }
-    if ((s = launch_contraction_pair(cp, op, c->NE, c->Nk, c->N, c->wk, X, Y, m.q, c->cwork, c->st))) return s;
+    if ((s = launch_contraction_pair(cp, op, c->NE, c->Nk, c->N, c->wk, X, Y, m.q, work, st))) return s;
     void* SR = field_of(dst, i, 0);
     if (c->drop_real) {
       // Sigma^R = -i Gamma / 2 (production_operators.jl:1174-1177); no roundoff estimate
-      if ((s = launch_retarded_drop(cp, c->nfield, SL, SG, SR, c->st))) return s;
+      if ((s = launch_retarded_drop(cp, c->nfield, SL, SG, SR, st))) return s;
     } else if (c->direct_green && !m.is_LO) {
       // elastic closure Sigma^R = K[G^R] (production_operators.jl:1311-1316)
-      if ((s = launch_contraction(cp, op, c->NE, c->Nk, c->N, c->wk, GR, SR, m.q, 0.0, c->cwork, c->st))) return s;
+      if ((s = launch_contraction(cp, op, c->NE, c->Nk, c->N, c->wk, GR, SR, m.q, 0.0, work, st))) return s;
     } else {
-      if ((s = launch_hilbert(c->hil, cp, ncols, c->wE, nullptr, SL, SG, nullptr, SR, nullptr, verify, c->st)))
+      if ((s = launch_hilbert(hil, cp, ncols, c->wE, nullptr, SL, SG, nullptr, SR, nullptr, verify, st)))
         return s;
-      if (verify && (s = launch_combine(c->hil.partial, (int)ncols, 2, c->scal + SC_ROUND + 2 * i, c->st))) return s;
+      if (verify && (s = launch_combine(hil.partial, (int)ncols, 2, c->scal + SC_ROUND + 2 * i, st))) return s;
     }
     // _apply_scattering_model! (production_operators.jl:1240-1256)
     void* fam[3] = {SR, SL, SG};
-    if ((s = launch_scattering_model(cp, c->NE, c->Nk, c->N, c->wk, c->wk_sum, c->diagonal, c->averaged, fam, c->st)))
+    if ((s = launch_scattering_model(cp, c->NE, c->Nk, c->N, c->wk, c->wk_sum, c->diagonal, c->averaged, fam, st)))
       return s;
   }
+  for (int q = 0; q < kBranches; ++q)
+    if (used >> q & 1u) {
+      QCL_CUDA_CHECK(cudaEventRecord(c->br_done[q], c->br_st[q]));
+      QCL_CUDA_CHECK(cudaStreamWaitEvent(c->st, c->br_done[q], 0));
+    }
   return QCL_OK;
 }
 
-static int embedding_candidates(ScbaCtx* c, std::vector<void*>& dst, const void* GR = nullptr,
+static int embedding_candidates(ScbaCtx* c, std::vector<void*>& dst, cudaStream_t st, const void* GR = nullptr,
                                 const void* GL = nullptr, const void* GG = nullptr) {
   const int cp = c->precision == QCL_MIXED ? QCL_C64 : c->precision;
   SandwichJob jobs[2];
@@ -735,7 +890,7 @@ static int embedding_candidates(ScbaCtx* c, std::vector<void*>& dst, const void*
     jobs[sgn].T = sgn == 0 ? c->Tp : c->Tm;
     jobs[sgn].plan = c->shift[sgn].view();
   }
-  return launch_sandwich(cp, c->NE, c->Nk, c->N, jobs, 2, c->st);
+  return launch_sandwich(cp, c->NE, c->Nk, c->N, jobs, 2, st);
 }
 
 static int totals(ScbaCtx* c, const std::vector<void*>& fam, void* const* out) {
@@ -792,10 +947,24 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
   if ((s = launch_residual_blocks(c->precision, RES_PART_MAIN, c->NE, c->Nk, c->N, c->eps, c->h, c->GR, c->GL, c->GG,
                                   c->tot[0], c->tot[1], c->tot[2], nullptr, c->reswork, c->st2)))
     return s;
+  // J and populations come from the unmixed plus family and the state's G
+  const auto observables = [&](cudaStream_t st) {
+    return launch_observables(sp, c->NE, c->Nk, c->N, c->wE, c->wk, field_of(state, c->M, 2), field_of(state, c->M, 1),
+                              c->GL, c->GG, c->gs, c->target, c->obspartial, c->scal + SC_OBS, st);
+  };
+  const bool fork = branching(c);  // the embedding has a branch of its own, observables follow the residuals
+  const int eb = kBranches - 1;
+  if (fork) {
+    if ((s = observables(c->st2))) return s;
+    QCL_CUDA_CHECK(cudaStreamWaitEvent(c->br_st[eb], c->ev_fork, 0));
+    if ((s = embedding_candidates(c, cand, c->br_st[eb]))) return s;
+    QCL_CUDA_CHECK(cudaEventRecord(c->br_done[eb], c->br_st[eb]));
+  }
   QCL_CUDA_CHECK(cudaEventRecord(c->ev_join, c->st2));
   if ((s = scattering_candidates(c, c->GR, c->GL, c->GG, cand, c->verify != 0))) return s;
   if ((s = phase_mark(c, 2))) return s;
-  if ((s = embedding_candidates(c, cand))) return s;
+  if (fork) QCL_CUDA_CHECK(cudaStreamWaitEvent(c->st, c->br_done[eb], 0));
+  else if ((s = embedding_candidates(c, cand, c->st))) return s;
   if ((s = phase_mark(c, 3))) return s;
   const int F = c->M + 2;
   const void* olds[kMaxMixFields];
@@ -805,18 +974,13 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
       olds[3 * f + k] = field_of(state, f, k);
       cands[3 * f + k] = field_of(cand, f, k);
     }
-  // r_K against the candidate total lesser, the reduction of the suite, J and
-  // populations (from the unmixed plus family and the state's G)
+  // r_K against the candidate total lesser and the reduction of the suite
   const auto residuals = [&]() -> int {
     if ((s = launch_residual_blocks(c->precision, RES_PART_RK, c->NE, c->Nk, c->N, c->eps, c->h, c->GR, c->GL, c->GG,
                                     c->tot[0], c->tot[1], c->tot[2], c->candSL, c->reswork, c->st)))
       return s;
     QCL_CUDA_CHECK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
     return launch_residual_reduce(c->NE, c->Nk, c->reswork, c->scal + SC_RES, c->st);
-  };
-  const auto observables = [&](cudaStream_t st) {
-    return launch_observables(sp, c->NE, c->Nk, c->N, c->wE, c->wk, field_of(state, c->M, 2), field_of(state, c->M, 1),
-                              c->GL, c->GG, c->gs, c->target, c->obspartial, c->scal + SC_OBS, st);
   };
   if (!c->mixing) {
     // the candidate total, the residuals of every family and of the embedding
@@ -827,7 +991,7 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
     if ((s = phase_mark(c, 4))) return s;
     if ((s = residuals())) return s;
     if ((s = phase_mark(c, 5))) return s;
-    if ((s = observables(c->st))) return s;
+    if (!fork && (s = observables(c->st))) return s;
     if ((s = phase_mark(c, 6))) return s;
   } else {
     const void* src[1][8];
@@ -842,7 +1006,7 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
                                     c->scal + SC_EMB + 2 * k, c->st)))
         return s;
     if ((s = phase_mark(c, 5))) return s;
-    if ((s = observables(c->st))) return s;
+    if (!fork && (s = observables(c->st))) return s;
     if ((s = phase_mark(c, 6))) return s;
     // Anderson mixing with the causality guard (production_mixing.jl:224-317)
     const int nf = 3 * F;
@@ -940,7 +1104,7 @@ int scba_seed(ScbaCtx* c, double* mu_out) {
   if ((s = launch_seed_green(sp, c->NE, c->Nk, c->N, c->GR, f_d, c->GL, c->GG, c->st))) return s;
   // initial candidates (no roundoff verification), straight into the state
   if ((s = scattering_candidates(c, c->GR, c->GL, c->GG, c->state, false))) return s;
-  if ((s = embedding_candidates(c, c->state))) return s;
+  if ((s = embedding_candidates(c, c->state, c->st))) return s;
   QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));
   QCL_CUDA_CHECK(cudaMemcpy(hst, c->status, sizeof(hst), cudaMemcpyDeviceToHost));
   if (hst[0]) {
@@ -1407,6 +1571,8 @@ int scba_promote(ScbaCtx* c) {
   }
   c->precision = QCL_C128;
   i8_area(c);
+  for (auto& m : c->mech)  // maps on the integer path share its work area
+    if (m.i8_work && contraction_i8_bytes(m.view(), c->NE, c->Nk, c->N) > 0) m.branch = -1;
   c->guard_roundoff = 1.1920928955078125e-07;  // the promoted state's FP32 rounding
   c->fbytes = c->nfield * 16;
   if ((s = prepare_hilbert_tables(c->hil, c->NE, c->de, QCL_C128))) return s;
@@ -1535,7 +1701,7 @@ int sweep_run(Sweep* sw, int max_iter, double tol, qcl_scba_row* last, int* iter
     bool changed = false;
     while (next < n && used + peak[next] <= budget) {
       qcl_scba_problem p = sw->points[next].problem;
-      // what the points that fit beside this one leave over may hold its integer-path area
+      // what the points that fit beside this one leave over may hold its optional areas
       size_t rest = budget - used - peak[next];
       for (int j = next + 1; j < n && peak[j] <= rest; ++j) rest -= peak[j];
       p.memory_budget_bytes = peak[next] + rest;
@@ -1547,7 +1713,7 @@ int sweep_run(Sweep* sw, int max_iter, double tol, qcl_scba_row* last, int* iter
         scba_destroy(c);
         return fail(s);
       }
-      const size_t bytes = peak[next] + (c->mech.empty() ? 0 : c->mech[0].i8_bytes);
+      const size_t bytes = peak[next] + (c->mech.empty() ? 0 : c->mech[0].i8_bytes) + c->br_bytes;
       active.push_back({next, c, bytes});
       used += bytes;
       ++next;
@@ -1726,7 +1892,7 @@ int scba_tangent_step(ScbaCtx* c, double* out) {
     return s;
   // Phi_Sigma v: the linear candidate maps of the tangent Green's functions
   if ((s = scattering_candidates(c, X, dL, dG, c->tw, false))) return s;
-  if ((s = embedding_candidates(c, c->tw, X, dL, dG))) return s;
+  if ((s = embedding_candidates(c, c->tw, c->st, X, dL, dG))) return s;
   // w <- Phi_Sigma v + s, then the damped update into w with the residual norms
   const void* olds[kMaxMixFields];
   void* cands[kMaxMixFields];
