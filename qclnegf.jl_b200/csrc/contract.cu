@@ -146,13 +146,16 @@ int build_shift_plan_host(int NE, const double* eps, double delta, int* left, in
 // Momentum reduction: X[e + NE q] = sum_m' wk[m'] G[e + NE (m' + Nk q)]
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void momentum_sum_kernel(int NE, int Nk, int NQ, const double* __restrict__ wk,
-                                    const Cx<R>* __restrict__ G, Cx<R>* __restrict__ X) {
+__global__ void momentum_sum_kernel(int NE, int Nk, int NQ, const double* __restrict__ wk, const Cx<R>* G0,
+                                    const Cx<R>* G1, Cx<R>* X0, Cx<R>* X1) {
+  const Cx<R>* __restrict__ G = blockIdx.y ? G1 : G0;
+  Cx<R>* __restrict__ X = blockIdx.y ? X1 : X0;
   const long long n = (long long)NE * NQ;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int e = (int)(i % NE);
     const long long q = i / NE;
     double sx = 0, sy = 0;
+#pragma unroll 8
     for (int mp = 0; mp < Nk; ++mp) {
       const Cx<R> g = G[(size_t)e + (size_t)NE * ((size_t)mp + (size_t)Nk * q)];
       sx += wk[mp] * (double)g.x;
@@ -163,80 +166,112 @@ __global__ void momentum_sum_kernel(int NE, int Nk, int NQ, const double* __rest
 }
 
 // ---------------------------------------------------------------------------
-// Tiled complex GEMM over strided views:
+// Complex GEMM over strided views, of one or two fields:
 //   C[e, j] (bcast copies) = alpha * sum_k A[e,k] w(k,b) B[j,k] + beta * C
-//   A[e,k] = A[e + lda k + a_b b],  B[j,k] = B[j ldb_j + k ldb_k + b_b b],
-//   C[e,j] = C[e + ldc j + c_b b + bcast_stride r], r < bcast.
+//   A[e,k] = A[f][e + lda k + a_b b],  B[j,k] = B[j + ldb k + b_b b],
+//   C[e,j] = C[f][e + ldc j + c_b b + bcast_stride r], r < bcast,
+// b < batch, f < fields.
 // ---------------------------------------------------------------------------
 template <typename R> struct GemmArgs {
   int M, Nout, K, batch;
-  const Cx<R>* A;
+  int fields = 1;
+  const Cx<R>* A[2];
   long long lda, a_b;
   const double* wk;  // optional weight wk[k % wk_mod]
   int wk_mod;
   const double* wb;  // optional weight wb[b]
   const Cx<R>* B;
-  long long ldb_j, ldb_k, b_b;
-  Cx<R>* C;
+  long long ldb, b_b;
+  Cx<R>* C[2];
   long long ldc, c_b;
   int bcast;
   long long bcast_stride;
   double alpha, beta;
+  // tile order: 0 = row tiles fastest (the CTAs in flight share B tiles),
+  // 1 = column tiles fastest (they share A tiles: an A larger than L2 is
+  // read once); set by launch_gemm for complex128
+  int cols_fastest;
 };
 
-constexpr int GK = 16;
+template <typename R> __device__ __forceinline__ void gemm_store(const GemmArgs<R>& p, Cx<R>* C, int e, int j, Cx<R> acc) {
+  const double vx = p.alpha * (double)acc.x, vy = p.alpha * (double)acc.y;
+  for (int r = 0; r < p.bcast; ++r) {
+    const size_t idx = (size_t)e + (size_t)p.ldc * j + (size_t)p.bcast_stride * r;
+    if (p.beta == 0.0) {
+      C[idx] = cx<R>((R)vx, (R)vy);
+    } else {
+      const Cx<R> o = C[idx];
+      C[idx] = cx<R>((R)(p.beta * o.x + vx), (R)(p.beta * o.y + vy));
+    }
+  }
+}
 
-// Output tile GE x GJ per CTA of GT threads: a 16 x (GT / 16) thread grid,
-// each thread GE/16 x GJ/(GT/16) outputs.  Two shapes: 64 x 32 (256 threads)
-// and, when that gives fewer than two CTAs per SM, 32 x 16 (128 threads) --
-// the same per-output arithmetic and summation order, more CTAs in flight.
-template <typename R, int GE, int GJ, int GT> __global__ void __launch_bounds__(GT) gemm_kernel(GemmArgs<R> p) {
+// complex64: CUDA cores.  Output tile GE x GJ per CTA of GT threads: a 16 x
+// (GT / 16) thread grid, each thread GE/16 x GJ/(GT/16) outputs.  The next K
+// block is fetched into registers while the current one is multiplied, all
+// its loads in flight at once (loop by loop they were a chain of load
+// latencies: 383 x 256 x 256 took 54 us for 0.2 GFLOP).
+constexpr int GK = 16;
+template <int GE, int GJ, int GT> __global__ void __launch_bounds__(GT) gemm_kernel(const __grid_constant__ GemmArgs<float> p) {
+  using R = float;
   constexpr int TJ = GT / 16, NI = GE / 16, NU = GJ / TJ;
-  static_assert(GE % 16 == 0 && GJ % TJ == 0, "tile shape");
-  __shared__ Cx<R> As[GK][GE];
-  __shared__ Cx<R> Bs[GK][GJ];
-  const int b = blockIdx.z;
+  constexpr int NA = GE * GK / GT, NB = GJ * GK / GT;
+  static_assert(GE % 16 == 0 && GJ % TJ == 0 && NA * GT == GE * GK && NB * GT == GJ * GK, "tile shape");
+  __shared__ Cx<R> As[2][GK][GE];
+  __shared__ Cx<R> Bs[2][GK][GJ];
+  const int f = blockIdx.z / p.batch, b = blockIdx.z - f * p.batch;
   const int e0 = blockIdx.x * GE, j0 = blockIdx.y * GJ;
   const int te = threadIdx.x % 16, tj = threadIdx.x / 16;
   const double wbb = p.wb ? p.wb[b] : 1.0;
-  Cx<R> acc[NI][NU];
+  const Cx<R>* A = (f ? p.A[1] : p.A[0]) + (size_t)p.a_b * b;
+  const Cx<R>* B = p.B + (size_t)p.b_b * b;
+  Cx<R>* C = (f ? p.C[1] : p.C[0]) + (size_t)p.c_b * b;
+  Cx<R> acc[NI][NU], ra[NA], rb[NB];
 #pragma unroll
   for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int u = 0; u < NU; ++u) acc[i][u] = cx<R>(0, 0);
-  for (int k0 = 0; k0 < p.K; k0 += GK) {
-    for (int idx = threadIdx.x; idx < GE * GK; idx += GT) {
-      const int el = idx % GE, kl = idx / GE;
-      const int e = e0 + el, k = k0 + kl;
-      Cx<R> v = cx<R>(0, 0);
-      if (e < p.M && k < p.K) {
-        v = p.A[(size_t)e + (size_t)p.lda * k + (size_t)p.a_b * b];
-        double w = wbb;
-        if (p.wk) w *= p.wk[k % p.wk_mod];
-        if (w != 1.0) v = cx<R>((R)(w * v.x), (R)(w * v.y));
-      }
-      As[kl][el] = v;
+  double rw[NA];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+      const int idx = threadIdx.x + q * GT, e = e0 + idx % GE, k = k0 + idx / GE;
+      const bool ok = e < p.M && k < p.K;
+      ra[q] = ok ? A[(size_t)e + (size_t)p.lda * k] : cx<R>(0, 0);
+      rw[q] = p.wk && ok ? wbb * p.wk[k % p.wk_mod] : wbb;
     }
-    for (int idx = threadIdx.x; idx < GJ * GK; idx += GT) {
-      const int jl = idx % GJ, kl = idx / GJ;
-      const int j = j0 + jl, k = k0 + kl;
-      Bs[kl][jl] = (j < p.Nout && k < p.K) ? p.B[(size_t)p.ldb_j * j + (size_t)p.ldb_k * k + (size_t)p.b_b * b]
-                                           : cx<R>(0, 0);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const int idx = threadIdx.x + q * GT, j = j0 + idx % GJ, k = k0 + idx / GJ;
+      rb[q] = j < p.Nout && k < p.K ? B[(size_t)j + (size_t)p.ldb * k] : cx<R>(0, 0);
     }
-    __syncthreads();
+  };
+  fetch(0);
+  for (int k0 = 0, s = 0; k0 < p.K; k0 += GK, s ^= 1) {
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+      const int idx = threadIdx.x + q * GT;
+      As[s][idx / GE][idx % GE] = rw[q] == 1.0 ? ra[q] : cx<R>((R)(rw[q] * ra[q].x), (R)(rw[q] * ra[q].y));
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const int idx = threadIdx.x + q * GT;
+      Bs[s][idx / GJ][idx % GJ] = rb[q];
+    }
+    __syncthreads();  // stage s is complete; its other half was read before the last barrier
+    if (k0 + GK < p.K) fetch(k0 + GK);
 #pragma unroll
     for (int kl = 0; kl < GK; ++kl) {
       Cx<R> a[NI], bb[NU];
 #pragma unroll
-      for (int i = 0; i < NI; ++i) a[i] = As[kl][te + 16 * i];
+      for (int i = 0; i < NI; ++i) a[i] = As[s][kl][te + 16 * i];
 #pragma unroll
-      for (int u = 0; u < NU; ++u) bb[u] = Bs[kl][tj + TJ * u];
+      for (int u = 0; u < NU; ++u) bb[u] = Bs[s][kl][tj + TJ * u];
 #pragma unroll
       for (int i = 0; i < NI; ++i)
 #pragma unroll
         for (int u = 0; u < NU; ++u) cfma(acc[i][u], a[i], bb[u]);
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
@@ -245,65 +280,47 @@ template <typename R, int GE, int GJ, int GT> __global__ void __launch_bounds__(
 #pragma unroll
     for (int u = 0; u < NU; ++u) {
       const int j = j0 + tj + TJ * u;
-      if (j >= p.Nout) continue;
-      const double vx = p.alpha * (double)acc[i][u].x, vy = p.alpha * (double)acc[i][u].y;
-      for (int r = 0; r < p.bcast; ++r) {
-        const size_t idx = (size_t)e + (size_t)p.ldc * j + (size_t)p.c_b * b + (size_t)p.bcast_stride * r;
-        if (p.beta == 0.0) {
-          p.C[idx] = cx<R>((R)vx, (R)vy);
-        } else {
-          const Cx<R> o = p.C[idx];
-          p.C[idx] = cx<R>((R)(p.beta * o.x + vx), (R)(p.beta * o.y + vy));
-        }
-      }
+      if (j < p.Nout) gemm_store<R>(p, C, e, j, acc[i][u]);
     }
   }
 }
 
-template <typename R> static int launch_gemm(const GemmArgs<R>& a, cudaStream_t st) {
+// Wider tiles while they leave two CTAs per SM; narrower ones, down to 32 x 16,
+// fill the GPU at the sizes where a launch would otherwise be a few CTAs.
+static int launch_gemm(const GemmArgs<float>& a, cudaStream_t st) {
   if (a.M <= 0 || a.Nout <= 0 || a.batch <= 0) return QCL_OK;
-  const long long big = (long long)((a.M + 63) / 64) * ((a.Nout + 31) / 32) * a.batch;
-  if (big >= 2 * 148) {
-    dim3 grid((a.M + 63) / 64, (a.Nout + 31) / 32, a.batch);
-    gemm_kernel<R, 64, 32, 256><<<grid, 256, 0, st>>>(a);
+  const int z = a.batch * a.fields;
+  auto ctas = [&](int ge, int gj) { return (long long)((a.M + ge - 1) / ge) * ((a.Nout + gj - 1) / gj) * z; };
+  if (a.Nout > 32 && ctas(64, 64) >= 2 * 148) {
+    gemm_kernel<64, 64, 256><<<dim3((a.M + 63) / 64, (a.Nout + 63) / 64, z), 256, 0, st>>>(a);
+  } else if (a.Nout > 16 && ctas(64, 32) >= 2 * 148) {
+    gemm_kernel<64, 32, 256><<<dim3((a.M + 63) / 64, (a.Nout + 31) / 32, z), 256, 0, st>>>(a);
   } else {
-    dim3 grid((a.M + 31) / 32, (a.Nout + 15) / 16, a.batch);
-    gemm_kernel<R, 32, 16, 128><<<grid, 128, 0, st>>>(a);
+    gemm_kernel<32, 16, 128><<<dim3((a.M + 31) / 32, (a.Nout + 15) / 16, z), 128, 0, st>>>(a);
   }
   QCL_LAUNCH_CHECK("gemm_kernel");
   return QCL_OK;
 }
 
 // ---------------------------------------------------------------------------
-// Dense complex128 contraction on the FP64 tensor path (mma.sync m8n8k4 f64):
-//   C[e, j] = alpha sum_k A[e + lda k] w[k % wmod] B[j + ldb k] + beta C[e + ldc j].
-// CTA: 8 warps, 128 (e) x 32 (j) outputs; warp (wm, wn) owns rows 32 wm ..
-// + 31 and columns 16 wn .. + 15 as 4 x 2 tiles of 8 x 8, each accumulated as
-// four real products (Re C += Ar Br - Ai Bi, Im C += Ar Bi + Ai Br).  K
-// advances by 16 through two cp.async stages; shared rows are padded to a
-// stride of 2 (mod 8) 16-byte units so the fragment loads of a quarter warp
-// hit 8 distinct bank groups.  Fragment layouts (m8n8k4, f64): A lane l holds
-// (l / 4, l % 4), B holds (l % 4, l / 4), C holds (l / 4, 2 (l % 4) + i).
+// complex128: the FP64 tensor path (mma.sync m8n8k4 f64).  CTA: BM (e) x 32 (j)
+// outputs on BM / (8 TR) x 2 warps; warp (wm, wn) owns 8 TR rows and 16 columns
+// as TR x 2 tiles of 8 x 8, each accumulated as four real
+// products (Re C += Ar Br - Ai Bi, Im C += Ar Bi + Ai Br); tiles past the last
+// column are skipped.  K advances by 16 through 2 or 3 cp.async stages; shared
+// rows are padded to a stride of 2 (mod 8) 16-byte units so the fragment
+// loads of a quarter warp hit 8 distinct bank groups.  Fragment layouts
+// (m8n8k4, f64): A lane l holds (l / 4, l % 4), B holds (l % 4, l / 4), C holds
+// (l / 4, 2 (l % 4) + i).
 // ---------------------------------------------------------------------------
-constexpr int DM_BM = 128, DM_BN = 32, DM_BK = 16, DM_THREADS = 256;
-constexpr int DM_APAD = DM_BM + 2, DM_BPAD = DM_BN + 2;
-constexpr size_t DM_SMEM = (2 * DM_BK * DM_APAD + 2 * DM_BK * DM_BPAD) * sizeof(Cx<double>) + 2 * DM_BK * sizeof(double);
-
-struct DmArgs {
-  int M, N, K;
-  const Cx<double>* A;
-  long long lda;
-  const double* w;
-  int wmod;
-  const Cx<double>* B;
-  long long ldb;
-  Cx<double>* C;
-  long long ldc;
-  double alpha, beta;
-  // tile order: 0 = row tiles fastest (the CTAs in flight share B tiles),
-  // 1 = column tiles fastest (they share A tiles: an A larger than L2 is
-  // read once); set by launch_dmma_dense
-  int cols_fastest;
+constexpr int DM_BN = 32, DM_BK = 16;
+constexpr int DM_BPAD = DM_BN + 2;
+// at least four warps, one per scheduler: each has a quarter of the FP64 rate
+template <int BM_> struct DmShape {
+  static constexpr int BM = BM_, TR = BM == 32 ? 2 : 4, WM = BM / (8 * TR), THREADS = 64 * WM, APAD = BM + 2;
+  static constexpr int STAGES = BM == 32 ? 3 : 2;  // CTAs per SM: 2, 4, 4
+  static constexpr size_t SMEM =
+      STAGES * (DM_BK * (APAD + DM_BPAD) * sizeof(Cx<double>) + DM_BK * sizeof(double));
 };
 
 __device__ __forceinline__ void dm_cp16(Cx<double>* dst, const Cx<double>* src, bool valid) {
@@ -316,234 +333,267 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(DM_THREADS, 2) dmma_dense_kernel(DmArgs p) {
+template <int BM>
+__global__ void __launch_bounds__(DmShape<BM>::THREADS, BM == 128 ? 2 : 4) dmma_gemm_kernel(const __grid_constant__ GemmArgs<double> p) {
+  using S = DmShape<BM>;
+  constexpr int TR = S::TR, WM = S::WM, ST = S::STAGES;
   extern __shared__ __align__(16) unsigned char dm_raw[];
-  Cx<double>* As = reinterpret_cast<Cx<double>*>(dm_raw);   // [2][DM_BK][DM_APAD]
-  Cx<double>* Bs = As + 2 * DM_BK * DM_APAD;                 // [2][DM_BK][DM_BPAD]
-  double* ws = reinterpret_cast<double*>(Bs + 2 * DM_BK * DM_BPAD);  // [2][DM_BK]
-  const int m0 = (p.cols_fastest ? blockIdx.y : blockIdx.x) * DM_BM;
+  Cx<double>* As = reinterpret_cast<Cx<double>*>(dm_raw);            // [ST][DM_BK][APAD]
+  Cx<double>* Bs = As + ST * DM_BK * S::APAD;                         // [ST][DM_BK][DM_BPAD]
+  double* ws = reinterpret_cast<double*>(Bs + ST * DM_BK * DM_BPAD);  // [ST][DM_BK]
+  const int m0 = (p.cols_fastest ? blockIdx.y : blockIdx.x) * S::BM;
   const int n0 = (p.cols_fastest ? blockIdx.x : blockIdx.y) * DM_BN;
+  const int f = blockIdx.z / p.batch, b = blockIdx.z - f * p.batch;
+  const double wbb = p.wb ? p.wb[b] : 1.0;
+  const Cx<double>* A = (f ? p.A[1] : p.A[0]) + (size_t)p.a_b * b;
+  const Cx<double>* B = p.B + (size_t)p.b_b * b;
+  Cx<double>* C = (f ? p.C[1] : p.C[0]) + (size_t)p.c_b * b;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = warp & 3, wn = warp >> 2;
+  const int wm = warp % WM, wn = warp / WM;
   const int lr = lane >> 2, lc = lane & 3;
-  double cr[4][2][2], ci[4][2][2];
+  const bool col_in[2] = {n0 + wn * 16 < p.Nout, n0 + wn * 16 + 8 < p.Nout};  // warp-uniform
+  double cr[TR][2][2], ci[TR][2][2];
 #pragma unroll
-  for (int t = 0; t < 4; ++t)
+  for (int t = 0; t < TR; ++t)
 #pragma unroll
     for (int u = 0; u < 2; ++u) cr[t][u][0] = cr[t][u][1] = ci[t][u][0] = ci[t][u][1] = 0.0;
 
   const int nkb = (p.K + DM_BK - 1) / DM_BK;
   auto load = [&](int kb, int s) {
     const int k0 = kb * DM_BK;
-    Cx<double>* as = As + s * DM_BK * DM_APAD;
+    Cx<double>* as = As + s * DM_BK * S::APAD;
     Cx<double>* bs = Bs + s * DM_BK * DM_BPAD;
 #pragma unroll
-    for (int i = threadIdx.x; i < DM_BK * DM_BM; i += DM_THREADS) {
-      const int kk = i / DM_BM, el = i % DM_BM;
+    for (int i = threadIdx.x; i < DM_BK * S::BM; i += S::THREADS) {
+      const int kk = i / S::BM, el = i % S::BM;
       const int k = k0 + kk, e = m0 + el;
       const bool ok = k < p.K && e < p.M;
-      dm_cp16(as + kk * DM_APAD + el, ok ? p.A + (size_t)e + (size_t)p.lda * k : p.A, ok);
+      dm_cp16(as + kk * S::APAD + el, ok ? A + (size_t)e + (size_t)p.lda * k : A, ok);
     }
 #pragma unroll
-    for (int i = threadIdx.x; i < DM_BK * DM_BN; i += DM_THREADS) {
+    for (int i = threadIdx.x; i < DM_BK * DM_BN; i += S::THREADS) {
       const int kk = i / DM_BN, jl = i % DM_BN;
       const int k = k0 + kk, j = n0 + jl;
-      const bool ok = k < p.K && j < p.N;
-      dm_cp16(bs + kk * DM_BPAD + jl, ok ? p.B + (size_t)j + (size_t)p.ldb * k : p.B, ok);
+      const bool ok = k < p.K && j < p.Nout;
+      dm_cp16(bs + kk * DM_BPAD + jl, ok ? B + (size_t)j + (size_t)p.ldb * k : B, ok);
     }
     if (threadIdx.x < DM_BK) {
       const int k = k0 + threadIdx.x;
-      ws[s * DM_BK + threadIdx.x] = (k < p.K && p.w) ? p.w[k % p.wmod] : 1.0;
+      ws[s * DM_BK + threadIdx.x] = (k < p.K && p.wk) ? wbb * p.wk[k % p.wk_mod] : wbb;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  load(0, 0);
+  // one commit group per stage, empty past the last block, so that the wait
+  // counts stages
+#pragma unroll
+  for (int q = 0; q < ST - 1; ++q) {
+    if (q < nkb) load(q, q);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   for (int kb = 0; kb < nkb; ++kb) {
-    const int s = kb & 1;
-    if (kb + 1 < nkb) {
-      load(kb + 1, s ^ 1);  // stage s^1 was released by the barrier at the end of iteration kb-1
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
+    const int s = kb % ST;
+    // the stage being refilled was released by the barrier at the end of iteration kb - 1
+    if (kb + ST - 1 < nkb) load(kb + ST - 1, (kb + ST - 1) % ST);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(ST - 1) : "memory");
     __syncthreads();
-    const Cx<double>* as = As + s * DM_BK * DM_APAD;
+    const Cx<double>* as = As + s * DM_BK * S::APAD;
     const Cx<double>* bs = Bs + s * DM_BK * DM_BPAD;
+    if (col_in[0]) {
 #pragma unroll
-    for (int c = 0; c < DM_BK / 4; ++c) {
-      const int kk = 4 * c + lc;
-      const double w = ws[s * DM_BK + kk];
-      double ar[4], ai[4], nai[4], br[2], bi[2];
+      for (int c = 0; c < DM_BK / 4; ++c) {
+        const int kk = 4 * c + lc;
+        const double w = ws[s * DM_BK + kk];
+        double ar[TR], ai[TR], nai[TR], br[2], bi[2];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const Cx<double> a = as[kk * DM_APAD + wm * 32 + t * 8 + lr];
-        ar[t] = a.x * w;
-        ai[t] = a.y * w;
-        nai[t] = -ai[t];
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const Cx<double> b = bs[kk * DM_BPAD + wn * 16 + u * 8 + lr];
-        br[u] = b.x;
-        bi[u] = b.y;
-      }
-#pragma unroll
-      for (int t = 0; t < 4; ++t)
+        for (int t = 0; t < TR; ++t) {
+          const Cx<double> a = as[kk * S::APAD + wm * 8 * TR + t * 8 + lr];
+          ar[t] = a.x * w;
+          ai[t] = a.y * w;
+          nai[t] = -ai[t];
+        }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          dmma(cr[t][u], ar[t], br[u]);
-          dmma(cr[t][u], nai[t], bi[u]);
-          dmma(ci[t][u], ar[t], bi[u]);
-          dmma(ci[t][u], ai[t], br[u]);
+          const Cx<double> bv = bs[kk * DM_BPAD + wn * 16 + u * 8 + lr];
+          br[u] = bv.x;
+          bi[u] = bv.y;
         }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (!col_in[u]) continue;
+#pragma unroll
+          for (int t = 0; t < TR; ++t) {
+            dmma(cr[t][u], ar[t], br[u]);
+            dmma(cr[t][u], nai[t], bi[u]);
+            dmma(ci[t][u], ar[t], bi[u]);
+            dmma(ci[t][u], ai[t], br[u]);
+          }
+        }
+      }
     }
     __syncthreads();  // every warp is done with stage s before it is refilled
   }
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const int e = m0 + wm * 32 + t * 8 + lr;
+  for (int t = 0; t < TR; ++t) {
+    const int e = m0 + wm * 8 * TR + t * 8 + lr;
     if (e >= p.M) continue;
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int j = n0 + wn * 16 + u * 8 + 2 * lc + i;
-        if (j >= p.N) continue;
-        Cx<double>* dst = p.C + (size_t)e + (size_t)p.ldc * j;
-        const double vr = p.alpha * cr[t][u][i], vi = p.alpha * ci[t][u][i];
-        if (p.beta == 0.0) {
-          *dst = cx<double>(vr, vi);
-        } else {
-          const Cx<double> o = *dst;
-          *dst = cx<double>(p.beta * o.x + vr, p.beta * o.y + vi);
-        }
+        if (j < p.Nout) gemm_store<double>(p, C, e, j, cx<double>(cr[t][u][i], ci[t][u][i]));
       }
   }
 }
 
-static int launch_dmma_dense(const DmArgs& args, cudaStream_t st) {
+template <int BM> static int launch_dmma_t(const GemmArgs<double>& a, cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
-    QCL_CUDA_CHECK(cudaFuncSetAttribute(dmma_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DM_SMEM));
+    QCL_CUDA_CHECK(cudaFuncSetAttribute(dmma_gemm_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)DmShape<BM>::SMEM));
     configured = true;
   }
-  DmArgs a = args;
-  const int mt = (a.M + DM_BM - 1) / DM_BM, nt = (a.N + DM_BN - 1) / DM_BN;
+  const int mt = (a.M + BM - 1) / BM, nt = (a.Nout + DM_BN - 1) / DM_BN, z = a.batch * a.fields;
+  const dim3 grid = a.cols_fastest ? dim3(nt, mt, z) : dim3(mt, nt, z);
+  dmma_gemm_kernel<BM><<<grid, DmShape<BM>::THREADS, DmShape<BM>::SMEM, st>>>(a);
+  QCL_LAUNCH_CHECK("dmma_gemm_kernel");
+  return QCL_OK;
+}
+
+// Tile height by the rows the busiest SM works through (the FP64 rate is the
+// bound): 64 x 48^2 x 48^2 436 -> 183 us with 32 rows, 383 x 2048^2 670 -> 515 us
+// with 64, where 128 rows leave SMs without a tile.  Shorter tiles load more
+// per product, hence their handicap.
+static int launch_gemm(const GemmArgs<double>& args, cudaStream_t st) {
+  GemmArgs<double> a = args;
+  if (a.M <= 0 || a.Nout <= 0 || a.batch <= 0) return QCL_OK;
+  const int nt = (a.Nout + DM_BN - 1) / DM_BN, z = a.batch * a.fields;
+  auto ctas = [&](int bm) { return (long long)((a.M + bm - 1) / bm) * nt * z; };
   // the larger operand is read once: an A larger than B and than L2 streams
   // with the column tiles fastest
-  a.cols_fastest = a.M > a.N && (size_t)a.M * a.K * sizeof(Cx<double>) > ((size_t)96 << 20) && mt <= 65535;
-  const dim3 grid = a.cols_fastest ? dim3(nt, mt) : dim3(mt, nt);
-  dmma_dense_kernel<<<grid, DM_THREADS, DM_SMEM, st>>>(a);
-  QCL_LAUNCH_CHECK("dmma_dense_kernel");
-  return QCL_OK;
+  const int mt = (a.M + 127) / 128;
+  a.cols_fastest = a.M > a.Nout && (size_t)a.M * a.K * sizeof(Cx<double>) > ((size_t)96 << 20) && mt <= 65535;
+  auto rows = [&](int bm) { return (double)((ctas(bm) + 147) / 148 * bm); };
+  const double r128 = rows(128), r64 = 1.07 * rows(64), r32 = 1.2 * rows(32);
+  if (r128 <= r64 && r128 <= r32) return launch_dmma_t<128>(a, st);
+  if (r64 <= r32) return launch_dmma_t<64>(a, st);
+  return launch_dmma_t<32>(a, st);
 }
 
 // ---------------------------------------------------------------------------
 // Contraction dispatch
 // ---------------------------------------------------------------------------
+// One or two fields G[f] -> S[f].  work holds contraction_work_elems elements;
+// with two fields, work2 as many again.
 template <typename R>
-static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const double* wk, const void* Gv, void* Sv,
-                         double alpha_q, double beta, void* work, cudaStream_t st) {
-  const Cx<R>* G = (const Cx<R>*)Gv;
-  Cx<R>* S = (Cx<R>*)Sv;
+static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const double* wk, int fields,
+                         const void* const* Gv, void* const* Sv, double alpha_q, double beta, void* work, void* work2,
+                         cudaStream_t st) {
   const int N2 = N * N;
   const long long NEl = NE;
+  const Cx<R>* const G[2] = {(const Cx<R>*)Gv[0], fields > 1 ? (const Cx<R>*)Gv[1] : nullptr};
+  Cx<R>* const S[2] = {(Cx<R>*)Sv[0], fields > 1 ? (Cx<R>*)Sv[1] : nullptr};
+  Cx<R>* const T[2] = {(Cx<R>*)work, (Cx<R>*)work2};
   if (op.kind == QCL_KERNEL_MOMENTUM_INDEPENDENT) {
-    Cx<R>* X = (Cx<R>*)work;  // NE * N2
-    const long long n = NEl * N2;
-    momentum_sum_kernel<R><<<grid_cap(n, 256), 256, 0, st>>>(NE, Nk, N2, wk, G, X);
+    const long long n = NEl * N2;  // T[f]: NE * N2
+    momentum_sum_kernel<R><<<dim3(grid_cap(n, 256), fields), 256, 0, st>>>(NE, Nk, N2, wk, G[0], G[1], T[0], T[1]);
     QCL_LAUNCH_CHECK("momentum_sum_kernel");
     GemmArgs<R> g{};
-    g.M = NE; g.Nout = N2; g.K = N2; g.batch = 1;
-    g.A = X; g.lda = NEl; g.a_b = 0;
-    g.B = (const Cx<R>*)op.block; g.ldb_j = 1; g.ldb_k = N2; g.b_b = 0;
-    g.C = S; g.ldc = NEl * Nk; g.c_b = 0; g.bcast = Nk; g.bcast_stride = NEl;
+    g.M = NE; g.Nout = N2; g.K = N2; g.batch = 1; g.fields = fields;
+    g.B = (const Cx<R>*)op.block; g.ldb = N2;
+    g.ldc = NEl * Nk; g.bcast = Nk; g.bcast_stride = NEl;
+    g.lda = NEl;
     g.alpha = alpha_q; g.beta = beta;
-    return launch_gemm<R>(g, st);
+    for (int f = 0; f < 2; ++f) {
+      g.A[f] = T[f];
+      g.C[f] = S[f];
+    }
+    return launch_gemm(g, st);
   }
   if (op.kind == QCL_KERNEL_DENSE) {
     const int Nc = Nk * N2;
-    if (sizeof(R) == 4 && op.tc_bop)  // complex64 fields: tensor cores (scaled FP16 hi/lo)
-      return launch_tc_dense_contraction(NE, Nc, op.tc_bop, Gv, Sv, alpha_q, beta, (float*)work, op.status, st);
-    if (sizeof(R) == 8 && op.i8_work && i8_worthwhile(NE, 1, Nc, Nc)) {
-      const void* A[1] = {Gv};
-      void* C[1] = {Sv};
-      return launch_i8_gemm(NE, 1, Nc, Nc, A, NEl, wk, Nk, op.matrix, Nc, C, NEl, alpha_q, beta, op.i8_work, op.i8_bytes,
-                            op.status, st);
+    if (sizeof(R) == 4 && op.tc_bop) {  // complex64 fields: tensor cores (scaled FP16 hi/lo)
+      for (int f = 0; f < fields; ++f)
+        if (int s = launch_tc_dense_contraction(NE, Nc, op.tc_bop, Gv[f], Sv[f], alpha_q, beta, (float*)work, op.status, st))
+          return s;
+      return QCL_OK;
     }
-    if (sizeof(R) == 8) {  // complex128: FP64 tensor path (DMMA)
-      DmArgs d{NE, Nc, Nc, (const Cx<double>*)Gv, NEl, wk, Nk, (const Cx<double>*)op.matrix, Nc, (Cx<double>*)Sv, NEl,
-               alpha_q, beta};
-      return launch_dmma_dense(d, st);
-    }
+    if (sizeof(R) == 8 && op.i8_work && i8_worthwhile(NE, fields, Nc, Nc))
+      return launch_i8_gemm(NE, fields, Nc, Nc, Gv, NEl, wk, Nk, op.matrix, Nc, Sv, NEl, alpha_q, beta, op.i8_work,
+                            op.i8_bytes, op.status, st);
     GemmArgs<R> g{};
-    g.M = NE; g.Nout = Nc; g.K = Nc; g.batch = 1;
-    g.A = G; g.lda = NEl; g.wk = wk; g.wk_mod = Nk;
-    g.B = (const Cx<R>*)op.matrix; g.ldb_j = 1; g.ldb_k = Nc;
-    g.C = S; g.ldc = NEl; g.bcast = 1;
+    g.M = NE; g.Nout = Nc; g.K = Nc; g.batch = 1; g.fields = fields;
+    g.lda = NEl; g.wk = wk; g.wk_mod = Nk;
+    g.B = (const Cx<R>*)op.matrix; g.ldb = Nc;
+    g.ldc = NEl; g.bcast = 1;
     g.alpha = alpha_q; g.beta = beta;
-    return launch_gemm<R>(g, st);
+    for (int f = 0; f < 2; ++f) {
+      g.A[f] = G[f];
+      g.C[f] = S[f];
+    }
+    return launch_gemm(g, st);
   }
   if (op.kind == QCL_KERNEL_IFR) {
-    const int J = op.J;
-    Cx<R>* T = (Cx<R>*)work;                  // T[e + NE (j + J m')]
-    Cx<R>* F = T + (size_t)NE * J * Nk;       // F[e + NE (j + J m)]
+    const int J = op.J;  // T[e + NE (j + J m')], then F[e + NE (j + J m)] behind it
+    const size_t half = (size_t)NE * J * Nk;
     int s;
-    GemmArgs<R> g{};
+    GemmArgs<R> g{}, h{}, f{};
     // stage 1, batch m': T = wk[m'] right * G_m'
-    g.M = NE; g.Nout = J; g.K = N2; g.batch = Nk;
-    g.A = G; g.lda = NEl * Nk; g.a_b = NEl; g.wb = wk;
-    g.B = (const Cx<R>*)op.right; g.ldb_j = 1; g.ldb_k = J; g.b_b = 0;
-    g.C = T; g.ldc = NEl; g.c_b = NEl * J; g.bcast = 1;
+    g.M = NE; g.Nout = J; g.K = N2; g.batch = Nk; g.fields = fields;
+    g.lda = NEl * Nk; g.a_b = NEl; g.wb = wk;
+    g.B = (const Cx<R>*)op.right; g.ldb = J;
+    g.ldc = NEl; g.c_b = NEl * J; g.bcast = 1;
     g.alpha = 1.0; g.beta = 0.0;
-    if ((s = launch_gemm<R>(g, st))) return s;
     // stage 2, batch j: F[., j, m] = sum_m' radial[m, m'] T[., j, m']
-    GemmArgs<R> h{};
-    h.M = NE; h.Nout = Nk; h.K = Nk; h.batch = J;
-    h.A = T; h.lda = NEl * J; h.a_b = NEl;
-    h.B = (const Cx<R>*)op.radial; h.ldb_j = 1; h.ldb_k = Nk; h.b_b = 0;
-    h.C = F; h.ldc = NEl * J; h.c_b = NEl; h.bcast = 1;
+    h.M = NE; h.Nout = Nk; h.K = Nk; h.batch = J; h.fields = fields;
+    h.lda = NEl * J; h.a_b = NEl;
+    h.B = (const Cx<R>*)op.radial; h.ldb = Nk;
+    h.ldc = NEl * J; h.c_b = NEl; h.bcast = 1;
     h.alpha = 1.0; h.beta = 0.0;
-    if ((s = launch_gemm<R>(h, st))) return s;
     // stage 3, batch m: S[., m, p] = alpha q sum_j left[p, j] F[., j, m] + beta S
-    GemmArgs<R> f{};
-    f.M = NE; f.Nout = N2; f.K = J; f.batch = Nk;
-    f.A = F; f.lda = NEl; f.a_b = NEl * J;
-    f.B = (const Cx<R>*)op.left; f.ldb_j = 1; f.ldb_k = N2; f.b_b = 0;
-    f.C = S; f.ldc = NEl * Nk; f.c_b = NEl; f.bcast = 1;
+    f.M = NE; f.Nout = N2; f.K = J; f.batch = Nk; f.fields = fields;
+    f.lda = NEl; f.a_b = NEl * J;
+    f.B = (const Cx<R>*)op.left; f.ldb = N2;
+    f.ldc = NEl * Nk; f.c_b = NEl; f.bcast = 1;
     f.alpha = alpha_q; f.beta = beta;
-    return launch_gemm<R>(f, st);
+    for (int q = 0; q < 2; ++q) {
+      Cx<R>* F = T[q] ? T[q] + half : nullptr;
+      g.A[q] = G[q];
+      g.C[q] = T[q];
+      h.A[q] = T[q];
+      h.C[q] = F;
+      f.A[q] = F;
+      f.C[q] = S[q];
+    }
+    if ((s = launch_gemm(g, st))) return s;
+    if ((s = launch_gemm(h, st))) return s;
+    return launch_gemm(f, st);
   }
   if (op.kind == QCL_KERNEL_LOW_RANK) {
     // LowRankProductionKernel (production_operators.jl:597-658):
     //   T[e, r] = sum_q right_adjoint[r, q] wk[q % Nk] G[e, q]      (NE x rank)
     //   S[e, q] = alpha q^K sum_r left[q, r] T[e, r] + beta S[e, q]
     const int Nc = Nk * N2, r = op.J;
-    Cx<R>* T = (Cx<R>*)work;
-    int s;
-    if (sizeof(R) == 8) {
-      DmArgs d1{NE, r, Nc, (const Cx<double>*)Gv, NEl, wk, Nk, (const Cx<double>*)op.right, r, (Cx<double>*)work,
-                NEl, 1.0, 0.0};
-      if ((s = launch_dmma_dense(d1, st))) return s;
-      DmArgs d2{NE, Nc, r, (const Cx<double>*)work, NEl, nullptr, 1, (const Cx<double>*)op.left, Nc,
-                (Cx<double>*)Sv, NEl, alpha_q, beta};
-      return launch_dmma_dense(d2, st);
-    }
-    GemmArgs<R> g{};
-    g.M = NE; g.Nout = r; g.K = Nc; g.batch = 1;
-    g.A = G; g.lda = NEl; g.wk = wk; g.wk_mod = Nk;
-    g.B = (const Cx<R>*)op.right; g.ldb_j = 1; g.ldb_k = r;
-    g.C = T; g.ldc = NEl; g.bcast = 1;
+    GemmArgs<R> g{}, f{};
+    g.M = NE; g.Nout = r; g.K = Nc; g.batch = 1; g.fields = fields;
+    g.lda = NEl; g.wk = wk; g.wk_mod = Nk;
+    g.B = (const Cx<R>*)op.right; g.ldb = r;
+    g.ldc = NEl; g.bcast = 1;
     g.alpha = 1.0; g.beta = 0.0;
-    if ((s = launch_gemm<R>(g, st))) return s;
-    GemmArgs<R> f{};
-    f.M = NE; f.Nout = Nc; f.K = r; f.batch = 1;
-    f.A = T; f.lda = NEl;
-    f.B = (const Cx<R>*)op.left; f.ldb_j = 1; f.ldb_k = Nc;
-    f.C = S; f.ldc = NEl; f.bcast = 1;
+    f.M = NE; f.Nout = Nc; f.K = r; f.batch = 1; f.fields = fields;
+    f.lda = NEl;
+    f.B = (const Cx<R>*)op.left; f.ldb = Nc;
+    f.ldc = NEl; f.bcast = 1;
     f.alpha = alpha_q; f.beta = beta;
-    return launch_gemm<R>(f, st);
+    for (int q = 0; q < 2; ++q) {
+      g.A[q] = G[q];
+      g.C[q] = T[q];
+      f.A[q] = T[q];
+      f.C[q] = S[q];
+    }
+    if (int s = launch_gemm(g, st)) return s;
+    return launch_gemm(f, st);
   }
   if (op.kind == QCL_KERNEL_SEPARABLE_SUM) {
     // K(m,m') = sum_i radial_i(m,m') block_i: a Kronecker sum of J terms (the
@@ -557,6 +607,7 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
     //            S[(e,m), (a,b)] = alpha q sum_k Z[(e,m), k] block[(a,b), k] + beta S
     // The rows of stage 2 are the (e, m) pairs, contiguous in the E-fastest
     // layout, so S and Z are plain column-major (NE Nk) x N^2 matrices.
+    for (int fi = 0; fi < fields; ++fi) {
     const int J = op.J;
     const long long Mr = NEl * Nk;                // stage-2 rows
     const size_t zfield = (size_t)Mr * N2;        // one intermediate field
@@ -567,7 +618,7 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
     // rows (e, (c,d)), K = m', behind the stage-2 work area
     float* gwork = awork + tc_a_work_floats2((int)Mr, jmax * N2);
     int s;
-    if (sizeof(R) == 4 && op.tc_stage1 && (s = tc_split_rows(NE * N2, Nk, Gv, NEl, NEl * Nk, gwork, st))) return s;
+    if (sizeof(R) == 4 && op.tc_stage1 && (s = tc_split_rows(NE * N2, Nk, Gv[fi], NEl, NEl * Nk, gwork, st))) return s;
     for (int c = 0, i0 = 0; i0 < J; ++c, i0 += kSepChunk) {
       const int jc = min(kSepChunk, J - i0);
       if (sizeof(R) == 4 && op.tc_stage1) {
@@ -580,38 +631,35 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
       for (int i = i0; i < i0 + jc; ++i) {
         GemmArgs<R> g{};
         g.M = NE; g.Nout = Nk; g.K = Nk; g.batch = N2;
-        g.A = G; g.lda = NEl; g.a_b = Mr; g.wk = wk; g.wk_mod = Nk;
-        g.B = (const Cx<R>*)op.radial + (size_t)Nk * Nk * i; g.ldb_j = 1; g.ldb_k = Nk; g.b_b = 0;
-        g.C = Z + zfield * (i - i0); g.ldc = NEl; g.c_b = Mr; g.bcast = 1;
+        g.A[0] = G[fi]; g.lda = NEl; g.a_b = Mr; g.wk = wk; g.wk_mod = Nk;
+        g.B = (const Cx<R>*)op.radial + (size_t)Nk * Nk * i; g.ldb = Nk;
+        g.C[0] = Z + zfield * (i - i0); g.ldc = NEl; g.c_b = Mr; g.bcast = 1;
         g.alpha = 1.0; g.beta = 0.0;
-        if ((s = launch_gemm<R>(g, st))) return s;
+        if ((s = launch_gemm(g, st))) return s;
       }
       const double bc = c == 0 ? beta : 1.0;
       const Cx<R>* blk = (const Cx<R>*)op.block + (size_t)N2 * N2 * i0;
       if (sizeof(R) == 8 && op.i8_work && i8_worthwhile((int)Mr, 1, N2, jc * N2)) {
         const void* A[1] = {Z};
-        void* C[1] = {Sv};
+        void* C[1] = {Sv[fi]};
         if ((s = launch_i8_gemm((int)Mr, 1, N2, jc * N2, A, Mr, nullptr, 1, blk, N2, C, Mr, alpha_q, bc, op.i8_work,
                                 op.i8_bytes, op.status, st)))
           return s;
-      } else if (sizeof(R) == 8) {
-        DmArgs d{(int)Mr, N2, jc * N2, (const Cx<double>*)Z, Mr, nullptr, 1, (const Cx<double>*)blk, N2,
-                 (Cx<double>*)Sv, Mr, alpha_q, bc};
-        if ((s = launch_dmma_dense(d, st))) return s;
       } else if (op.tc_chunks) {
-        if ((s = launch_tc_contraction2((int)Mr, N2, jc * N2, op.tc_chunks[c], Z, Sv, alpha_q, bc, awork, op.status,
+        if ((s = launch_tc_contraction2((int)Mr, N2, jc * N2, op.tc_chunks[c], Z, Sv[fi], alpha_q, bc, awork, op.status,
                                         st)))
           return s;
       } else {
         GemmArgs<R> f{};
         f.M = (int)Mr; f.Nout = N2; f.K = jc * N2; f.batch = 1;
-        f.A = Z; f.lda = Mr;
-        f.B = blk; f.ldb_j = 1; f.ldb_k = N2;
-        f.C = S; f.ldc = Mr; f.bcast = 1;
+        f.A[0] = Z; f.lda = Mr;
+        f.B = blk; f.ldb = N2;
+        f.C[0] = S[fi]; f.ldc = Mr; f.bcast = 1;
         f.alpha = alpha_q; f.beta = bc;
-        if ((s = launch_gemm<R>(f, st))) return s;
+        if ((s = launch_gemm(f, st))) return s;
       }
     }
+    }  // fields
     return QCL_OK;
   }
   set_last_error("unknown kernel operator kind %d", op.kind);
@@ -695,21 +743,27 @@ size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N) {
   return 0;
 }
 
+// The second field's scratch is as large as the first's; where it is not given
+// (work2 == NULL) or an operator's maps gain nothing, the fields go one by one.
 int launch_contraction_pair(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk,
-                            const void* const* G, void* const* S, double alpha_q, void* work, cudaStream_t st) {
-  const int Nc = Nk * N * N;
-  if (precision == QCL_C128 && op.kind == QCL_KERNEL_DENSE && op.i8_work && i8_worthwhile(NE, 2, Nc, Nc))
-    return launch_i8_gemm(NE, 2, Nc, Nc, G, NE, wk, Nk, op.matrix, Nc, S, NE, alpha_q, 0.0, op.i8_work, op.i8_bytes,
-                          op.status, st);
-  for (int f = 0; f < 2; ++f)
-    if (int s = launch_contraction(precision, op, NE, Nk, N, wk, G[f], S[f], alpha_q, 0.0, work, st)) return s;
-  return QCL_OK;
+                            const void* const* G, void* const* S, double alpha_q, void* work, void* work2,
+                            cudaStream_t st) {
+  const bool scratch = op.kind != QCL_KERNEL_DENSE && op.kind != QCL_KERNEL_SEPARABLE_SUM;
+  if (scratch && !work2) {
+    for (int f = 0; f < 2; ++f)
+      if (int s = launch_contraction(precision, op, NE, Nk, N, wk, G[f], S[f], alpha_q, 0.0, work, st)) return s;
+    return QCL_OK;
+  }
+  if (precision == QCL_C128) return contraction_t<double>(op, NE, Nk, N, wk, 2, G, S, alpha_q, 0.0, work, work2, st);
+  return contraction_t<float>(op, NE, Nk, N, wk, 2, G, S, alpha_q, 0.0, work, work2, st);
 }
 
 int launch_contraction(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk, const void* G,
                        void* S, double alpha_q, double beta, void* work, cudaStream_t st) {
-  if (precision == QCL_C128) return contraction_t<double>(op, NE, Nk, N, wk, G, S, alpha_q, beta, work, st);
-  return contraction_t<float>(op, NE, Nk, N, wk, G, S, alpha_q, beta, work, st);
+  const void* Gv[1] = {G};
+  void* Sv[1] = {S};
+  if (precision == QCL_C128) return contraction_t<double>(op, NE, Nk, N, wk, 1, Gv, Sv, alpha_q, beta, work, nullptr, st);
+  return contraction_t<float>(op, NE, Nk, N, wk, 1, Gv, Sv, alpha_q, beta, work, nullptr, st);
 }
 
 }  // namespace qcl

@@ -172,7 +172,8 @@ int i8_set_wait_limit(long long rounds);
 size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N);
 // Two fields through one operator: S[f] = alpha_q K[wk G[f]].
 int launch_contraction_pair(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk,
-                            const void* const* G, void* const* S, double alpha_q, void* work, cudaStream_t st);
+                            const void* const* G, void* const* S, double alpha_q, void* work, void* work2,
+                            cudaStream_t st);
 int launch_contraction(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk, const void* G,
                        void* S, double alpha_q, double beta, void* work, cudaStream_t st);
 

@@ -852,7 +852,10 @@ static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, con
       X[0] = c->tmp;
       X[1] = c->candSL;
     }
-    if ((s = launch_contraction_pair(cp, op, c->NE, c->Nk, c->N, c->wk, X, Y, m.q, work, st))) return s;
+    // the retarded candidate is formed after the maps: its field serves as the
+    // second component's scratch where that fits
+    void* work2 = contraction_work_elems(op, c->NE, c->Nk, c->N) <= c->nfield ? field_of(dst, i, 0) : nullptr;
+    if ((s = launch_contraction_pair(cp, op, c->NE, c->Nk, c->N, c->wk, X, Y, m.q, work, work2, st))) return s;
     void* SR = field_of(dst, i, 0);
     if (c->drop_real) {
       // Sigma^R = -i Gamma / 2 (production_operators.jl:1174-1177); no roundoff estimate
