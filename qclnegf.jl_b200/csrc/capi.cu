@@ -8,6 +8,8 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "staging.cuh"
+#include <initializer_list>
 
 namespace qcl {
 
@@ -109,8 +111,29 @@ struct Grow {
   }
 };
 
+// Slots of a staged call: slab k uses slot k % kSlots of the pinned buffer.
+constexpr int kSlots = 3;
+constexpr size_t kStageBytes = (size_t)4 << 20;  // one field's part of a slab
+
 struct Pipeline {
   cudaStream_t st[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t done[kSlots] = {nullptr, nullptr, nullptr};
+  char* pinned = nullptr;
+  size_t pinned_cap = 0;
+  // Pinned memory for staged calls (at most kSlots slots of 6 fields' slab
+  // parts), kept like the device workspace.
+  int ensure_pinned(size_t n) {
+    for (auto& e : done)
+      if (!e) QCL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (n <= pinned_cap) return QCL_OK;
+    if (pinned) cudaFreeHost(pinned);
+    pinned = nullptr;
+    pinned_cap = 0;
+    cudaError_t e = cudaMallocHost((void**)&pinned, n);
+    if (e != cudaSuccess) return cuda_status(e, "cudaMallocHost (staging)");
+    pinned_cap = n;
+    return QCL_OK;
+  }
   Grow eps, h, in[3], out[3], scale, trL, trG, status, wE, sum, gam;
   int init() {
     for (auto& s : st)
@@ -121,6 +144,94 @@ struct Pipeline {
     return QCL_OK;
   }
 };
+// One field's part of a slab on either side: `rows` runs of `width` bytes.
+struct SlabPart {
+  char* host;
+  char* dev;
+  size_t pitch, width, rows;  // the same pitch on both sides
+};
+
+// Runs `slabs` slabs with their inputs and outputs staged through pinned
+// slots: while the device works on a slab, the copy team fills the next one's
+// inputs and empties the outputs of the one before.  parts(k, in, out) lists a
+// slab's parts, launch(k, stream) enqueues its work.
+template <typename Parts, typename Launch>
+static int run_staged_slabs(Pipeline& P, int slabs, size_t slot_bytes, CopyTeam& team, Parts&& parts, Launch&& launch) {
+  int s;
+  if ((s = P.ensure_pinned(kSlots * slot_bytes))) return s;
+  std::vector<SlabPart> in, out, done_out[kSlots];
+  std::vector<CopyPiece> pieces;
+  for (int k = 0; k < slabs + 2; ++k) {
+    pieces.clear();
+    if (k >= 2) {  // slab k - 2 is on the host side of the link: empty its outputs
+      const int q = (k - 2) % kSlots;
+      QCL_CUDA_CHECK(cudaEventSynchronize(P.done[q]));
+      size_t off = q * slot_bytes;
+      for (const SlabPart& p : done_out[q]) {
+        pieces.push_back({p.host, P.pinned + off, p.pitch, p.width, p.width, p.rows});
+        off += p.width * p.rows;
+      }
+    }
+    if (k < slabs) {
+      // slot k % kSlots was last slab k - 3's, emptied in the step before
+      const int q = k % kSlots;
+      const cudaStream_t st = P.st[q];
+      in.clear();
+      out.clear();
+      parts(k, in, out);
+      size_t off = q * slot_bytes;
+      for (const SlabPart& p : out) off += p.width * p.rows;  // outputs first, inputs behind them
+      const size_t in_off = off;
+      for (const SlabPart& p : in) {
+        pieces.push_back({P.pinned + off, p.host, p.width, p.pitch, p.width, p.rows});
+        off += p.width * p.rows;
+      }
+      team.copy(pieces);
+      off = in_off;
+      for (const SlabPart& p : in) {
+        QCL_CUDA_CHECK(cudaMemcpy2DAsync(p.dev, p.pitch, P.pinned + off, p.width, p.width, p.rows,
+                                         cudaMemcpyHostToDevice, st));
+        off += p.width * p.rows;
+      }
+      if ((s = launch(k, st))) return s;
+      off = q * slot_bytes;
+      for (const SlabPart& p : out) {
+        QCL_CUDA_CHECK(cudaMemcpy2DAsync(P.pinned + off, p.width, p.dev, p.pitch, p.width, p.rows,
+                                         cudaMemcpyDeviceToHost, st));
+        off += p.width * p.rows;
+      }
+      QCL_CUDA_CHECK(cudaEventRecord(P.done[q], st));
+      done_out[q] = out;
+    } else {
+      team.copy(pieces);
+    }
+  }
+  return QCL_OK;
+}
+
+template <typename Parts, typename Launch>
+static int run_staged(Pipeline& P, int slabs, size_t slot_bytes, CopyTeam& team, Parts&& parts, Launch&& launch) {
+  const int s = run_staged_slabs(P, slabs, slot_bytes, team, parts, launch);
+  if (s)  // nothing of a failed call may still use the slots
+    for (auto st : P.st) cudaStreamSynchronize(st);
+  return s;
+}
+
+// Threads for a call on these host arrays (NULL entries are skipped): 0 unless
+// one of them is pageable and all are host memory.
+static int staged_threads(std::initializer_list<const void*> ptrs, size_t field_bytes, int* fields) {
+  bool pageable = false, host = true;
+  *fields = 0;
+  for (const void* p : ptrs)
+    if (p) {
+      ++*fields;
+      const HostKind k = host_kind(p);
+      pageable = pageable || k == HOST_PAGEABLE;
+      host = host && k != HOST_NOT;
+    }
+  return pageable && host ? copy_threads(field_bytes * *fields) : 0;
+}
+
 static std::mutex g_pipe_mutex;
 static Pipeline& pipeline() {
   static Pipeline p;
@@ -252,32 +363,25 @@ int qcl_dyson_keldysh(int precision, int NE, int Nk, int Nb, const double* eps, 
   QCL_CUDA_CHECK(cudaMemcpyAsync(P.h.p, h, (size_t)Nk * Nb * Nb * 16, cudaMemcpyHostToDevice, P.st[0]));
   QCL_CUDA_CHECK(cudaMemsetAsync(P.status.p, 0, 2 * sizeof(int), P.st[0]));
   QCL_CUDA_CHECK(cudaStreamSynchronize(P.st[0]));
-  // momentum slabs of ~64 MiB per field, round-robin over three streams so
-  // that the upload of one slab, the kernel of the previous one and the
-  // download of the one before overlap
+  // momentum slabs, round-robin over three streams so that the upload of one
+  // slab, the kernel of the previous one and the download of the one before
+  // overlap: ~64 MiB per field, or, through pinned slots where a field is in
+  // pageable memory, ~4 MiB
   const size_t slab_bytes = (size_t)NE * Nb * Nb * es;
-  int ms = (int)std::max<size_t>(1, (64u << 20) / std::max<size_t>(slab_bytes, 1));
+  int fields;
+  int threads = staged_threads({hin[0], hin[1], hin[2], hout[0], hout[1], hout[2]}, nf, &fields);
+  if (slab_bytes > 2 * kStageBytes) threads = 0;  // a momentum is the smallest slab
+  int ms = (int)std::max<size_t>(1, (threads > 0 ? kStageBytes : (64u << 20)) / std::max<size_t>(slab_bytes, 1));
   ms = std::min(ms, Nk);
   const size_t pitch = (size_t)NE * Nk * es;
-  int k = 0;
-  for (int m0 = 0; m0 < Nk; m0 += ms, ++k) {
-    const int cnt = std::min(ms, Nk - m0);
-    cudaStream_t st = P.st[k % 3];
-    const size_t off = (size_t)NE * m0 * es, width = (size_t)NE * cnt * es;
-    for (int i = 0; i < 3; ++i)
-      if (hin[i])
-        QCL_CUDA_CHECK(cudaMemcpy2DAsync((char*)P.in[i].p + off, pitch, (const char*)hin[i] + off, pitch, width,
-                                         (size_t)Nb * Nb, cudaMemcpyHostToDevice, st));
-    s = launch_dyson_keldysh(precision, NE, Nk, Nb, (const double*)P.eps.p, eta, P.h.p, P.in[0].p,
-                             sigL ? P.in[1].p : nullptr, sigG ? P.in[2].p : nullptr, GR ? P.out[0].p : nullptr,
-                             hout[1] ? P.out[1].p : nullptr, hout[2] ? P.out[2].p : nullptr,
-                             scale ? (double*)P.scale.p : nullptr, (traceL && sigL) ? P.trL.p : nullptr,
-                             (traceG && sigG) ? P.trG.p : nullptr, (int*)P.status.p, st, m0, cnt);
-    if (s) return s;
-    for (int i = 0; i < 3; ++i)
-      if (hout[i])
-        QCL_CUDA_CHECK(cudaMemcpy2DAsync((char*)hout[i] + off, pitch, (const char*)P.out[i].p + off, pitch, width,
-                                         (size_t)Nb * Nb, cudaMemcpyDeviceToHost, st));
+  const auto launch = [&](int m0, int cnt, cudaStream_t st) {
+    return launch_dyson_keldysh(precision, NE, Nk, Nb, (const double*)P.eps.p, eta, P.h.p, P.in[0].p,
+                                sigL ? P.in[1].p : nullptr, sigG ? P.in[2].p : nullptr, GR ? P.out[0].p : nullptr,
+                                hout[1] ? P.out[1].p : nullptr, hout[2] ? P.out[2].p : nullptr,
+                                scale ? (double*)P.scale.p : nullptr, (traceL && sigL) ? P.trL.p : nullptr,
+                                (traceG && sigG) ? P.trG.p : nullptr, (int*)P.status.p, st, m0, cnt);
+  };
+  const auto rows = [&](int m0, int cnt, cudaStream_t st) -> int {  // the per-block outputs
     const size_t boff = (size_t)NE * m0, bcnt = (size_t)NE * cnt;
     if (scale)
       QCL_CUDA_CHECK(cudaMemcpyAsync(scale + boff, (double*)P.scale.p + boff, bcnt * sizeof(double),
@@ -288,6 +392,40 @@ int qcl_dyson_keldysh(int precision, int NE, int Nk, int Nb, const double* eps, 
     if (traceG && sigG)
       QCL_CUDA_CHECK(cudaMemcpyAsync((char*)traceG + boff * 16, (char*)P.trG.p + boff * 16, bcnt * 16,
                                      cudaMemcpyDeviceToHost, st));
+    return QCL_OK;
+  };
+  if (threads > 0) {
+    CopyTeam team(threads);
+    const auto parts = [&](int k, std::vector<SlabPart>& in, std::vector<SlabPart>& out) {
+      const int m0 = k * ms, cnt = std::min(ms, Nk - m0);
+      const size_t off = (size_t)NE * m0 * es, width = (size_t)NE * cnt * es;
+      for (int i = 0; i < 3; ++i) {
+        if (hin[i]) in.push_back({(char*)hin[i] + off, (char*)P.in[i].p + off, pitch, width, (size_t)Nb * Nb});
+        if (hout[i]) out.push_back({(char*)hout[i] + off, (char*)P.out[i].p + off, pitch, width, (size_t)Nb * Nb});
+      }
+    };
+    s = run_staged(P, (Nk + ms - 1) / ms, slab_bytes * ms * fields, team, parts, [&](int k, cudaStream_t st) {
+      return launch(k * ms, std::min(ms, Nk - k * ms), st);
+    });
+    if (s) return s;
+    if ((s = rows(0, Nk, P.st[0]))) return s;
+  } else {
+    int k = 0;
+    for (int m0 = 0; m0 < Nk; m0 += ms, ++k) {
+      const int cnt = std::min(ms, Nk - m0);
+      cudaStream_t st = P.st[k % 3];
+      const size_t off = (size_t)NE * m0 * es, width = (size_t)NE * cnt * es;
+      for (int i = 0; i < 3; ++i)
+        if (hin[i])
+          QCL_CUDA_CHECK(cudaMemcpy2DAsync((char*)P.in[i].p + off, pitch, (const char*)hin[i] + off, pitch, width,
+                                           (size_t)Nb * Nb, cudaMemcpyHostToDevice, st));
+      if ((s = launch(m0, cnt, st))) return s;
+      for (int i = 0; i < 3; ++i)
+        if (hout[i])
+          QCL_CUDA_CHECK(cudaMemcpy2DAsync((char*)hout[i] + off, pitch, (const char*)P.out[i].p + off, pitch, width,
+                                           (size_t)Nb * Nb, cudaMemcpyDeviceToHost, st));
+      if ((s = rows(m0, cnt, st))) return s;
+    }
   }
   for (int i = 0; i < 3; ++i) QCL_CUDA_CHECK(cudaStreamSynchronize(P.st[i]));
   return read_status((int*)P.status.p, "dyson_keldysh");
@@ -341,25 +479,51 @@ static int hilbert_host(int precision, int NE, size_t ncols, const double* eps, 
   if ((s = P.sum.ensure(2 * sizeof(double)))) return s;
   QCL_CUDA_CHECK(cudaMemcpyAsync(P.wE.p, wE, NE * sizeof(double), cudaMemcpyHostToDevice, P.st[0]));
   QCL_CUDA_CHECK(cudaStreamSynchronize(P.st[0]));
-  // column slabs of ~64 MiB, three streams
-  size_t cs = std::max<size_t>(1, (64u << 20) / ((size_t)NE * es));
-  cs = std::min(cs, ncols);
-  int k = 0;
-  for (size_t c0 = 0; c0 < ncols; c0 += cs, ++k) {
-    const size_t cnt = std::min(cs, ncols - c0);
-    cudaStream_t st = P.st[k % 3];
-    const size_t off = c0 * NE * es, bytes = cnt * NE * es;
-    if (Gam) QCL_CUDA_CHECK(cudaMemcpyAsync((char*)P.in[0].p + off, (const char*)Gam + off, bytes, cudaMemcpyHostToDevice, st));
-    if (SL) QCL_CUDA_CHECK(cudaMemcpyAsync((char*)P.in[1].p + off, (const char*)SL + off, bytes, cudaMemcpyHostToDevice, st));
-    if (SG) QCL_CUDA_CHECK(cudaMemcpyAsync((char*)P.in[2].p + off, (const char*)SG + off, bytes, cudaMemcpyHostToDevice, st));
-    s = launch_hilbert(t, sp, (long long)cnt, (const double*)P.wE.p, Gam ? (char*)P.in[0].p + off : nullptr,
-                       SL ? (char*)P.in[1].p + off : nullptr, SG ? (char*)P.in[2].p + off : nullptr,
-                       out_lam ? (char*)P.out[0].p + off : nullptr, out_SR ? (char*)P.out[0].p + off : nullptr,
-                       out_gam ? (char*)P.gam.p + off : nullptr, verify, st, (long long)c0);
+  const auto slab = [&](size_t c0, size_t cnt, cudaStream_t st) {
+    const size_t off = c0 * NE * es;
+    return launch_hilbert(t, sp, (long long)cnt, (const double*)P.wE.p, Gam ? (char*)P.in[0].p + off : nullptr,
+                          SL ? (char*)P.in[1].p + off : nullptr, SG ? (char*)P.in[2].p + off : nullptr,
+                          out_lam ? (char*)P.out[0].p + off : nullptr, out_SR ? (char*)P.out[0].p + off : nullptr,
+                          out_gam ? (char*)P.gam.p + off : nullptr, verify, st, (long long)c0);
+  };
+  void* const hin[3] = {(void*)Gam, (void*)SL, (void*)SG};
+  void* const hout[2] = {out_lam ? out_lam : out_SR, out_gam};
+  void* const dout[2] = {P.out[0].p, P.gam.p};
+  int fields;
+  const int threads = staged_threads({hin[0], hin[1], hin[2], hout[0], hout[1]}, nf, &fields);
+  if (threads > 0) {
+    CopyTeam team(threads);
+    const size_t per = std::max<size_t>(1, kStageBytes / ((size_t)NE * es));
+    const int slabs = (int)((ncols + per - 1) / per);
+    const auto parts = [&](int k, std::vector<SlabPart>& in, std::vector<SlabPart>& out) {
+      const size_t c0 = (size_t)k * per, off = c0 * NE * es, bytes = std::min(per, ncols - c0) * NE * es;
+      for (int i = 0; i < 3; ++i)
+        if (hin[i]) in.push_back({(char*)hin[i] + off, (char*)P.in[i].p + off, bytes, bytes, 1});
+      for (int i = 0; i < 2; ++i)
+        if (hout[i]) out.push_back({(char*)hout[i] + off, (char*)dout[i] + off, bytes, bytes, 1});
+    };
+    s = run_staged(P, slabs, per * NE * es * fields, team, parts, [&](int k, cudaStream_t st) {
+      return slab((size_t)k * per, std::min(per, ncols - (size_t)k * per), st);
+    });
     if (s) return s;
-    QCL_CUDA_CHECK(cudaMemcpyAsync((char*)(out_lam ? out_lam : out_SR) + off, (char*)P.out[0].p + off, bytes,
-                                   cudaMemcpyDeviceToHost, st));
-    if (out_gam) QCL_CUDA_CHECK(cudaMemcpyAsync((char*)out_gam + off, (char*)P.gam.p + off, bytes, cudaMemcpyDeviceToHost, st));
+  } else {
+    // column slabs of ~64 MiB, three streams
+    size_t cs = std::max<size_t>(1, (64u << 20) / ((size_t)NE * es));
+    cs = std::min(cs, ncols);
+    int k = 0;
+    for (size_t c0 = 0; c0 < ncols; c0 += cs, ++k) {
+      const size_t cnt = std::min(cs, ncols - c0);
+      cudaStream_t st = P.st[k % 3];
+      const size_t off = c0 * NE * es, bytes = cnt * NE * es;
+      for (int i = 0; i < 3; ++i)
+        if (hin[i])
+          QCL_CUDA_CHECK(cudaMemcpyAsync((char*)P.in[i].p + off, (const char*)hin[i] + off, bytes,
+                                         cudaMemcpyHostToDevice, st));
+      if ((s = slab(c0, cnt, st))) return s;
+      for (int i = 0; i < 2; ++i)
+        if (hout[i])
+          QCL_CUDA_CHECK(cudaMemcpyAsync((char*)hout[i] + off, (char*)dout[i] + off, bytes, cudaMemcpyDeviceToHost, st));
+    }
   }
   for (int i = 0; i < 3; ++i) QCL_CUDA_CHECK(cudaStreamSynchronize(P.st[i]));
   if (verify) {

@@ -271,30 +271,24 @@ static int upload_op(ScbaCtx* c, void** dst, const void* host_c128, size_t n, vo
   return s;
 }
 
-static int build_plan(ScbaCtx* c, DevShift& d, double delta) {
-  std::vector<int> l(c->NE), r(c->NE);
-  std::vector<double> th(c->NE);
-  std::vector<unsigned char> v(c->NE);
-  int s = build_shift_plan_host(c->NE, c->eps_h.data(), delta, l.data(), r.data(), th.data(), v.data());
+// Fills a shift plan's device arrays, which share one allocation (theta, left,
+// right, valid), made on first use.
+static int fill_plan(ScbaCtx* c, DevShift& d, double delta) {
+  const size_t NE = c->NE;
+  std::vector<char> host(NE * 17);
+  double* th = (double*)host.data();
+  int *l = (int*)(th + NE), *r = l + NE;
+  unsigned char* v = (unsigned char*)(r + NE);
+  int s = build_shift_plan_host(c->NE, c->eps_h.data(), delta, l, r, th, v);
   if (s) return s;
-  if ((s = dupload(&d.left, l.data(), c->NE * sizeof(int), c->st))) return s;
-  if ((s = dupload(&d.right, r.data(), c->NE * sizeof(int), c->st))) return s;
-  if ((s = dupload(&d.theta, th.data(), c->NE * sizeof(double), c->st))) return s;
-  return dupload(&d.valid, v.data(), c->NE, c->st);
-}
-
-// Rebuilds a shift plan into its existing device arrays.
-static int refill_plan(ScbaCtx* c, DevShift& d, double delta) {
-  std::vector<int> l(c->NE), r(c->NE);
-  std::vector<double> th(c->NE);
-  std::vector<unsigned char> v(c->NE);
-  int s = build_shift_plan_host(c->NE, c->eps_h.data(), delta, l.data(), r.data(), th.data(), v.data());
-  if (s) return s;
-  QCL_CUDA_CHECK(cudaMemcpyAsync(d.left, l.data(), c->NE * sizeof(int), cudaMemcpyHostToDevice, c->st));
-  QCL_CUDA_CHECK(cudaMemcpyAsync(d.right, r.data(), c->NE * sizeof(int), cudaMemcpyHostToDevice, c->st));
-  QCL_CUDA_CHECK(cudaMemcpyAsync(d.theta, th.data(), c->NE * sizeof(double), cudaMemcpyHostToDevice, c->st));
-  QCL_CUDA_CHECK(cudaMemcpyAsync(d.valid, v.data(), c->NE, cudaMemcpyHostToDevice, c->st));
-  QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));  // the host vectors are temporaries
+  if (!d.theta) {
+    if ((s = dalloc((void**)&d.theta, host.size()))) return s;
+    d.left = (int*)(d.theta + NE);
+    d.right = d.left + NE;
+    d.valid = (unsigned char*)(d.right + NE);
+  }
+  QCL_CUDA_CHECK(cudaMemcpyAsync(d.theta, host.data(), host.size(), cudaMemcpyHostToDevice, c->st));
+  QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));  // the host vector is a temporary
   return QCL_OK;
 }
 
@@ -311,12 +305,7 @@ void scba_destroy(ScbaCtx* c) {
   cudaFree(c->h);
   cudaFree(c->Tp);
   cudaFree(c->Tm);
-  for (auto& d : c->shift) {
-    cudaFree(d.left);
-    cudaFree(d.right);
-    cudaFree(d.theta);
-    cudaFree(d.valid);
-  }
+  for (auto& d : c->shift) cudaFree(d.theta);  // the plan's one allocation
   for (auto& m : c->mech) {
     cudaFree(m.block);
     cudaFree(m.matrix);
@@ -689,10 +678,10 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
   TRY(dupload(&c->h, p->h, (size_t)c->Nk * c->N * c->N * 16, c->st));
   TRY(dupload(&c->Tp, p->Tplus, (size_t)c->N * c->N * 16, c->st));
   TRY(dupload(&c->Tm, p->Tminus, (size_t)c->N * c->N * 16, c->st));
-  TRY(build_plan(c, c->shift[0], +c->Ep));
-  TRY(build_plan(c, c->shift[1], -c->Ep));
-  TRY(build_plan(c, c->shift[2], +c->hw_LO));
-  TRY(build_plan(c, c->shift[3], -c->hw_LO));
+  TRY(fill_plan(c, c->shift[0], +c->Ep));
+  TRY(fill_plan(c, c->shift[1], -c->Ep));
+  TRY(fill_plan(c, c->shift[2], +c->hw_LO));
+  TRY(fill_plan(c, c->shift[3], -c->hw_LO));
   size_t cwork = 0;
   const int N2 = c->N * c->N;
   for (int i = 0; i < c->M; ++i) {
@@ -1431,8 +1420,8 @@ int scba_retarget(ScbaCtx* c, double Ep, double N_LO, double kBT, const void* h,
       }
   QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));
   int s;
-  if ((s = refill_plan(c, c->shift[0], +Ep))) return s;
-  if ((s = refill_plan(c, c->shift[1], -Ep))) return s;
+  if ((s = fill_plan(c, c->shift[0], +Ep))) return s;
+  if ((s = fill_plan(c, c->shift[1], -Ep))) return s;
   if (h) {
     QCL_CUDA_CHECK(cudaMemcpyAsync(c->h, h, (size_t)c->Nk * c->N * c->N * 16, cudaMemcpyHostToDevice, c->st));
     QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));

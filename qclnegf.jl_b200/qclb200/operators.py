@@ -74,9 +74,10 @@ def dyson_keldysh(eps, h, sigR, sigL=None, sigG=None, *, eta=0.0, precision="c12
     sigR = _field(sigR, cdt, shape)
     sigL = None if sigL is None else _field(sigL, cdt, shape)
     sigG = None if sigG is None else _field(sigG, cdt, shape)
-    GR = np.zeros(shape, dtype=cdt, order="F") if want_retarded else None
-    GL = np.zeros(shape, dtype=cdt, order="F") if sigL is not None else None
-    GG = np.zeros(shape, dtype=cdt, order="F") if sigG is not None else None
+    # every entry is written by the call
+    GR = np.empty(shape, dtype=cdt, order="F") if want_retarded else None
+    GL = np.empty(shape, dtype=cdt, order="F") if sigL is not None else None
+    GG = np.empty(shape, dtype=cdt, order="F") if sigG is not None else None
     scale = np.zeros((NE, Nk), order="F")
     trL = np.zeros((NE, Nk), dtype=np.complex128, order="F") if (return_traces and sigL is not None) else None
     trG = np.zeros((NE, Nk), dtype=np.complex128, order="F") if (return_traces and sigG is not None) else None
@@ -112,7 +113,7 @@ def fft_hilbert_transform(Gam, eps, wE, *, precision="c128", return_roundoff=Fal
     eps, wE = _real(eps), _real(wE)
     if eps.shape[0] != NE or wE.shape[0] != NE:
         raise _lib.DimensionMismatch(_lib.QCL_DIM, "energy data differ")
-    Lam = np.zeros_like(Gam, order="F")
+    Lam = np.empty_like(Gam, order="F")
     r = ctypes.c_double()
     check(lib().qcl_fft_hilbert_transform(p, NE, ncols, _ptr(eps), _ptr(wE), _ptr(Gam), _ptr(Lam),
                                           ctypes.byref(r) if return_roundoff else None))
@@ -129,8 +130,8 @@ def retarded_self_energy_fft(SL, SG, eps, wE, *, precision="c128", return_roundo
     NE = SL.shape[0]
     ncols = SL.size // NE
     eps, wE = _real(eps), _real(wE)
-    SR = np.zeros_like(SL, order="F")
-    Gam = np.zeros_like(SL, order="F")
+    SR = np.empty_like(SL, order="F")
+    Gam = np.empty_like(SL, order="F")
     r = ctypes.c_double()
     check(lib().qcl_retarded_self_energy(p, NE, ncols, _ptr(eps), _ptr(wE), _ptr(SL), _ptr(SG), _ptr(SR), _ptr(Gam),
                                          ctypes.byref(r) if return_roundoff else None))
