@@ -92,8 +92,9 @@ template <int NP> struct GjUnroll {
 };
 
 template <typename RS, typename RL, int NP, int TT, int BPC> constexpr size_t dyson_smem() {
-  static_assert(2 * (NP + 1) * sizeof(Cx<RL>) <= NP * NP * sizeof(Cx<RS>), "pivot rows fit the G tile");
-  return 2 * (size_t)BPC * NP * NP * sizeof(Cx<RS>) + BPC * sizeof(DysonScratch<TT>);
+  static_assert(2 * (NP * sizeof(Cx<RL>) + (Tile<NP>::CPR + 1) * 16) <= NP * NP * sizeof(Cx<RS>),
+                "pivot rows fit the G tile");
+  return 2 * (size_t)BPC * tile_stride<RS, NP, BPC>() * sizeof(Cx<RS>) + BPC * sizeof(DysonScratch<TT>);
 }
 
 // CTAs per SM that the shared memory allows (228 KB per SM, 1 KB reserved per
@@ -157,7 +158,7 @@ __device__ __forceinline__ void dyson_gj_2d24(const DysonArgs<RS>& p, Cx<RS>* X,
   }
   __syncthreads();  // every team has read its SigmaR tile: bufX is free
   // prefetch the first Keldysh input while the inversion runs
-  if (first_sig && (first_is_L ? p.GL : p.GG)) load_blocks_async<RS, NP, BPC>(first_sig, bufX, NP * NP, e0, m, NE, Nk, N);
+  if (first_sig && (first_is_L ? p.GL : p.GG)) load_blocks_async<RS, NP, BPC>(first_sig, bufX, tile_stride<RS, NP, BPC>(), e0, m, NE, Nk, N);
   const double s = team_max<32>(rmax, tt, S.red, team);
   const RL inv_s = (RL)(1.0 / s);
   const bool scale_ok = s > 0.0 && isfinite(s);
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (dyson_min_ctas<RS, RL, NP,
   constexpr int CPR = Tile<NP>::CPR, TT = Tile<NP>::TT, COLS = NP / CPR;
   constexpr int U = GjUnroll<NP>::U, GROUPS = COLS / U;
   static_assert(COLS % U == 0, "group width must divide the row chunk");
-  constexpr size_t MSZ = (size_t)NP * NP;
+  constexpr size_t MSZ = tile_stride<RS, NP, BPC>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx<RS>* bufX = reinterpret_cast<Cx<RS>*>(smem_raw);  // BPC tiles: Sigma^R, then Sigma^<,> and products
   Cx<RS>* bufG = bufX + BPC * MSZ;                    // BPC tiles: pivot rows, then G^R
@@ -288,7 +289,13 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (dyson_min_ctas<RS, RL, NP,
   const bool live = e < NE;
   Cx<RS>* X = bufX + team * MSZ;
   Cx<RS>* G = bufG + team * MSZ;
-  Cx<RL>* rowbuf = reinterpret_cast<Cx<RL>*>(G);  // 2 x (NP + 1): row chunks + pivot reciprocal
+  // two step buffers: the pivot row's chunks and its reciprocal.  One spare
+  // 16-byte slot per chunk: all lanes of a chunk read the same entry of theirs, and
+  // chunks that start a multiple of 128 bytes apart would read it from the
+  // same bank (N_b = 32, 1024 x 32 blocks, G^R alone: c128 1293 -> 1157 us,
+  // mixed 1175 -> 1010 us).
+  constexpr int CST = COLS + 16 / (int)sizeof(Cx<RL>), RBW = CPR * CST + 16 / (int)sizeof(Cx<RL>);
+  Cx<RL>* rowbuf = reinterpret_cast<Cx<RL>*>(G);
   DysonScratch<TT>& S = scr[team];
   const Cx<RS>* first_sig = p.sigL ? p.sigL : p.sigG;
   const bool first_is_L = p.sigL != nullptr;
@@ -387,9 +394,9 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (dyson_min_ctas<RS, RL, NP,
           }
           const bool is_pivot = row == best;
           if (chunk == kc) w[u] = is_pivot ? cx<RL>(1, 0) : cx<RL>(0, 0);
-          Cx<RL>* rb = rowbuf + (k & 1) * (NP + 1);
+          Cx<RL>* rb = rowbuf + (k & 1) * RBW;
   #pragma unroll
-          for (int j = 0; j < COLS; ++j) st_shared_if(rb + chunk * COLS + j, w[j], is_pivot);
+          for (int j = 0; j < COLS; ++j) st_shared_if(rb + chunk * CST + j, w[j], is_pivot);
           Cx<RL> rp;
           if (TT == 32) {
             const int plane = (best * CPR + kc) & 31;
@@ -397,9 +404,9 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (dyson_min_ctas<RS, RL, NP,
             rp.y = __shfl_sync(0xffffffffu, rc.y, plane);
             team_sync<TT>(team);
           } else {
-            st_shared_if(rb + NP, rc, is_pivot && chunk == kc);
+            st_shared_if(rb + RBW - 1, rc, is_pivot && chunk == kc);
             team_sync<TT>(team);
-            rp = rb[NP];
+            rp = rb[RBW - 1];
           }
           if (zero) rp = cx<RL>(0, 0);
           used |= is_pivot;
@@ -407,7 +414,7 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (dyson_min_ctas<RS, RL, NP,
           myrc = is_pivot ? rp : myrc;
           const Cx<RL> fp = is_pivot ? cx<RL>(0, 0) : f * rp;
   #pragma unroll
-          for (int j = 0; j < COLS; ++j) cfms(w[j], fp, rb[chunk * COLS + j]);
+          for (int j = 0; j < COLS; ++j) cfms(w[j], fp, rb[chunk * CST + j]);
         }
         if (GROUPS > 1) {  // rotate the chunk so that the next group is at w[0..U)
           Cx<RL> t[U];

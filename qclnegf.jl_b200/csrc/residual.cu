@@ -716,7 +716,7 @@ __device__ void posdef_rounds(unsigned kinds, int count, const Cx<double>* G, co
 }
 
 // Loads the tiles of `count` fields with all their accesses in flight.
-template <typename RS, int NP, int BPC, int COUNT>
+template <typename RS, int NP, int BPC, size_t STRIDE, int COUNT>
 __device__ __forceinline__ void load_tiles(const Cx<RS>* const (&src)[COUNT], Cx<double>* const (&dst)[COUNT], int e0,
                                            int m, int NE, int Nk, int N) {
   constexpr int IT = NP * NP / Tile<NP>::TT;
@@ -741,7 +741,7 @@ __device__ __forceinline__ void load_tiles(const Cx<RS>* const (&src)[COUNT], Cx
 #pragma unroll
       for (int q = 0; q < G; ++q) {
         const int el = (threadIdx.x + (q0 + q) * BPC * Tile<NP>::TT) / BPC;
-        dst[f][(size_t)eloc * NP * NP + sw<NP>(el % NP, el / NP)] = cvt<double>(v[f][q]);
+        dst[f][eloc * STRIDE + sw<NP>(el % NP, el / NP)] = cvt<double>(v[f][q]);
       }
   }
 }
@@ -785,7 +785,7 @@ __device__ void keldysh_defect(const Cx<double>* G, Cx<double>* T, const Cx<doub
 template <typename RS, int NP, int BPC>
 __global__ void __launch_bounds__(BPC* Tile<NP>::TT) residual_rk_kernel(ResidualArgs<RS> p) {
   constexpr int TT = Tile<NP>::TT;
-  constexpr size_t MSZ = (size_t)NP * NP;
+  constexpr size_t MSZ = tile_stride<double, NP, BPC>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx<double>* bG = reinterpret_cast<Cx<double>*>(smem_raw);
   Cx<double>* bX = bG + BPC * MSZ;
@@ -793,7 +793,7 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT) residual_rk_kernel(Residual
   double* red = reinterpret_cast<double*>(bW + BPC * MSZ);
   const int N = p.N, NE = p.NE, Nk = p.Nk, m = blockIdx.y, e0 = blockIdx.x * BPC;
   const int team = threadIdx.x / TT, tt = threadIdx.x % TT, e = e0 + team;
-  load_tiles<RS, NP, BPC, 3>({p.GR, p.GL, p.SLc}, {bG, bX, bW}, e0, m, NE, Nk, N);
+  load_tiles<RS, NP, BPC, MSZ, 3>({p.GR, p.GL, p.SLc}, {bG, bX, bW}, e0, m, NE, Nk, N);
   __syncthreads();
   double kNum, kDen;
   keldysh_defect<NP, TT>(bG + team * MSZ, bW + team * MSZ, bX + team * MSZ, N, tt, red + 4 * team, team, kNum, kDen);
@@ -837,8 +837,8 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (rows_min_ctas<NP>())) resi
   auto kinds = [](int a, int b = 0, int c = 0, int d = 0) { return (unsigned)(a | b << 4 | c << 8 | d << 12); };
 
   // ---- causality, A ---------------------------------------------------------
-  if constexpr (FOUR) load_tiles<RS, NP, BPC, 4>({p.GR, p.SR, p.GL, p.GG}, {bG, bX, bW, bH}, e0, m, NE, Nk, N);
-  else load_tiles<RS, NP, BPC, 3>({p.GR, p.SR, p.GL}, {bG, bX, bW}, e0, m, NE, Nk, N);
+  if constexpr (FOUR) load_tiles<RS, NP, BPC, MSZ, 4>({p.GR, p.SR, p.GL, p.GG}, {bG, bX, bW, bH}, e0, m, NE, Nk, N);
+  else load_tiles<RS, NP, BPC, MSZ, 3>({p.GR, p.SR, p.GL}, {bG, bX, bW}, e0, m, NE, Nk, N);
   __syncthreads();
   posdef_rounds<NP, TT>(kinds(HK_CAUS, HK_A, HK_GL, HK_GG), FOUR ? 4 : 2, G, X, W, H, N, tt, R, team, fail, bad);
   team_sync<TT>(team);
@@ -874,7 +874,7 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (rows_min_ctas<NP>())) resi
   double kNum = 0, kDen = 0;
   if (with_rk) {
     __syncthreads();
-    load_tiles<RS, NP, BPC, 1>({p.SLc}, {bX}, e0, m, NE, Nk, N);
+    load_tiles<RS, NP, BPC, MSZ, 1>({p.SLc}, {bX}, e0, m, NE, Nk, N);
     __syncthreads();
     keldysh_defect<NP, TT>(G, X, W, N, tt, S.red, team, kNum, kDen);
   }
@@ -882,12 +882,12 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (rows_min_ctas<NP>())) resi
   // ---- G<, G>, Gamma, then the raw products ---------------------------------
   __syncthreads();
   if constexpr (!FOUR) {
-    load_tiles<RS, NP, BPC, 1>({p.GG}, {bX}, e0, m, NE, Nk, N);
+    load_tiles<RS, NP, BPC, MSZ, 1>({p.GG}, {bX}, e0, m, NE, Nk, N);
     __syncthreads();
     posdef_rounds<NP, TT>(kinds(HK_GL, HK_GG), 2, G, X, W, H, N, tt, R, team, fail, bad);
     __syncthreads();
   }
-  load_tiles<RS, NP, BPC, 2>({p.SL, p.SG}, {bX, bW}, e0, m, NE, Nk, N);
+  load_tiles<RS, NP, BPC, MSZ, 2>({p.SL, p.SG}, {bX, bW}, e0, m, NE, Nk, N);
   __syncthreads();
   posdef_rounds<NP, TT>(kinds(HK_GAM), 1, G, X, W, H, N, tt, R, team, fail, bad);
   team_sync<TT>(team);
@@ -926,8 +926,8 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (rows_min_ctas<NP>())) resi
     const bool need = (fail >> kind & 1u) && live;
     if (__syncthreads_or(need)) {
       const Cx<RS>* src = kind == HK_A ? p.GR : kind == HK_GL ? p.GL : kind == HK_GG ? p.GG : kind == HK_RAWG ? p.SG : p.SL;
-      load_tiles<RS, NP, BPC, 1>({src}, {bX}, e0, m, NE, Nk, N);
-      if (kind == HK_GAM) load_tiles<RS, NP, BPC, 1>({p.SG}, {bW}, e0, m, NE, Nk, N);
+      load_tiles<RS, NP, BPC, MSZ, 1>({src}, {bX}, e0, m, NE, Nk, N);
+      if (kind == HK_GAM) load_tiles<RS, NP, BPC, MSZ, 1>({p.SG}, {bW}, e0, m, NE, Nk, N);
       __syncthreads();
       if (need) {
         if (kind == HK_RAWL || kind == HK_RAWG) sandwich(X);
@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (rows_min_ctas<NP>())) resi
   }
   const bool need = (fail >> HK_CAUS & 1u) && live;
   if (__syncthreads_or(need)) {
-    load_tiles<RS, NP, BPC, 1>({p.SR}, {bX}, e0, m, NE, Nk, N);
+    load_tiles<RS, NP, BPC, MSZ, 1>({p.SR}, {bX}, e0, m, NE, Nk, N);
     __syncthreads();
     if (need) {
       tile_for<NP, TT>(N, tt, [&](int i, int j) {
@@ -1071,7 +1071,7 @@ template <typename RS, int NP, int BPC> static int launch_residual_rows_t(const 
   constexpr int TT = Tile<NP>::TT;
   constexpr size_t tile = (size_t)BPC * NP * NP * sizeof(Cx<double>);
   constexpr size_t smem = (rows_four_tiles<NP>() ? 4 : 3) * tile + BPC * (sizeof(RowScratch<NP>) + sizeof(ResScratch<NP>));
-  constexpr size_t smem_rk = 3 * tile + BPC * 4 * sizeof(double);
+  constexpr size_t smem_rk = 3 * BPC * tile_stride<double, NP, BPC>() * sizeof(Cx<double>) + BPC * 4 * sizeof(double);
   static bool configured = false;
   if (!configured) {
     QCL_CUDA_CHECK(cudaFuncSetAttribute(residual_rows_kernel<RS, NP, BPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
