@@ -388,31 +388,45 @@ __device__ __forceinline__ void split_f16(float x, __half& hi, __half& lo) {
   lo = __float2half_rn(x - __half2float(hi));
 }
 
-// Row maxima of A: max_kk |A[e][kk]| into rowmax[e] as FP32 bits (non-negative
-// values order as unsigned integers; a non-finite entry gives +inf), which
-// the caller zeroes first.  A CTA covers 32 rows x 256 values of k (coalesced
-// along e); the atomic maximum is independent of the order.
+// |x| as an unsigned integer: non-negative FP32 bits order as integers, with
+// infinities and NaN above every finite value.
+__device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned max_bits(unsigned mx, Cx<float> g) {
+  return max(mx, max(abs_bits(g.x), abs_bits(g.y)));
+}
+
+// Row maxima of A: max_kk |A[e][kk]| into rowmax[e] as FP32 bits (a non-finite
+// entry gives +inf), which the caller zeroes first.  A CTA covers 32 rows x 256
+// values of k (coalesced along e); the atomic maximum is independent of the
+// order.  Bound by HBM: with eight loads in flight per thread 2.1 GB
+// (32768 x 8192) take 296 us, 7.3 TB/s (one at a time: 567 us).
 // Rows of A address G at (e mod P) + P k + Bs (e / P): P = NE, Bs = 0 is the
 // plain column-major matrix; P = N_E, Bs = N_E N_k reads a field with rows
 // (e, (c,d)) and columns m' (the first stage of a separable-sum contraction).
 __global__ void tc_row_max_kernel(int NE, int Nc, long long P, long long Bs, const Cx<float>* __restrict__ G,
                                   unsigned* __restrict__ rowmax) {
-  __shared__ float red[8][32];
+  __shared__ unsigned red[8][32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
   const int e = blockIdx.x * 32 + tx;
   const int k0 = blockIdx.y * 256, k1 = min(Nc, k0 + 256);
-  float mx = 0.0f;
-  if (e < NE)
-    for (int k = k0 + ty; k < k1; k += 8) {
-      const Cx<float> g = G[(size_t)(e % P) + (size_t)P * k + (size_t)Bs * (size_t)(e / P)];
-      const float a = fmaxf(fabsf(g.x), fabsf(g.y));
-      mx = (isfinite(g.x) && isfinite(g.y)) ? fmaxf(mx, a) : INFINITY;
+  unsigned mx = 0;
+  if (e < NE) {
+    const Cx<float>* row = G + (size_t)(e % P) + (size_t)Bs * (size_t)(e / P);
+    int k = k0 + ty;
+    for (; k + 56 < k1; k += 64) {
+      Cx<float> g[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) g[q] = row[(size_t)P * (k + 8 * q)];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) mx = max_bits(mx, g[q]);
     }
+    for (; k < k1; k += 8) mx = max_bits(mx, row[(size_t)P * k]);
+  }
   red[ty][tx] = mx;
   __syncthreads();
   if (ty == 0 && e < NE) {
-    for (int q = 1; q < 8; ++q) mx = fmaxf(mx, red[q][tx]);
-    atomicMax(rowmax + e, __float_as_uint(mx));
+    for (int q = 1; q < 8; ++q) mx = max(mx, red[q][tx]);
+    atomicMax(rowmax + e, min(mx, 0x7f800000u));
   }
 }
 
@@ -422,29 +436,48 @@ __global__ void tc_row_max_kernel(int NE, int Nc, long long P, long long Bs, con
 // and walks K in tiles of 64 complex columns (128 real), gridDim.y tiles
 // apart: each complex value is read once (coalesced along e), the tile is
 // transposed through shared memory, and each row's 128 values are written as
-// half2 pairs (coalesced along K).
+// half2 pairs (coalesced along K).  ONE: K fits one tile, so the CTA holds
+// whole rows, takes their maxima itself and rowmax is not read (2^20 rows x 32:
+// 138 us; the two passes: 80 + 130 us).
 constexpr int TC_SPLIT_KK = 128;
+template <bool ONE>
 __global__ void tc_split_a_kernel(int NE, int Nc, int Mpad, int Kpad, long long P, long long Bs,
                                   const Cx<float>* __restrict__ G,
                                   const unsigned* __restrict__ rowmax, __half* __restrict__ Ahi,
                                   __half* __restrict__ Alo, float* __restrict__ ainv) {
+  constexpr int Q = TC_SPLIT_KK / 16;
   __shared__ float tile[TC_SPLIT_KK][33];
   const int e0 = blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
   const int er = e0 + tx;  // this thread's row in the read phase
   const bool rin = er < NE;
-  const float sc = rin ? tc_scale_for(__uint_as_float(rowmax[er])) : 1.0f;
-  if (blockIdx.y == 0 && ty == 0 && er < Mpad) ainv[er] = 1.0f / sc;
   const size_t rowbase = rin ? (size_t)(er % P) + (size_t)Bs * (size_t)(er / P) : 0;
   for (int kk0 = blockIdx.y * TC_SPLIT_KK; kk0 < Kpad; kk0 += gridDim.y * TC_SPLIT_KK) {
+    Cx<float> g[Q];
+    unsigned mx = 0;
 #pragma unroll
-    for (int q = 0; q < TC_SPLIT_KK / 16; ++q) {
+    for (int q = 0; q < Q; ++q) {
+      const int k = (kk0 >> 1) + ty + 8 * q;
+      g[q] = rin && k < Nc ? G[rowbase + (size_t)P * k] : cx<float>(0.0f, 0.0f);
+      mx = max_bits(mx, g[q]);
+    }
+    if constexpr (ONE) {
+      __shared__ unsigned red[8][32];
+      red[ty][tx] = mx;
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) mx = max(mx, red[q][tx]);
+      mx = min(mx, 0x7f800000u);
+    } else {
+      mx = rin ? rowmax[er] : 0u;
+    }
+    const float sc = rin ? tc_scale_for(__uint_as_float(mx)) : 1.0f;
+    if (kk0 == 0 && ty == 0 && er < Mpad) ainv[er] = 1.0f / sc;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
       const int kl = ty + 8 * q;  // complex column within the tile
-      const int k = (kk0 >> 1) + kl;
-      Cx<float> g = cx<float>(0.0f, 0.0f);
-      if (rin && k < Nc) g = G[rowbase + (size_t)P * k];
-      tile[2 * kl][tx] = g.x * sc;
-      tile[2 * kl + 1][tx] = g.y * sc;
+      tile[2 * kl][tx] = g[q].x * sc;
+      tile[2 * kl + 1][tx] = g[q].y * sc;
     }
     __syncthreads();
     for (int r = ty; r < 32; r += 8) {
@@ -676,11 +709,17 @@ int tc_split_rows(int M, int Kc, const void* A, long long P, long long Bs, float
   __half* Alo = Ahi + (size_t)Mpad * Kpad;
   unsigned* rowmax = (unsigned*)(Alo + (size_t)Mpad * Kpad);
   float* ainv = (float*)(rowmax + Mpad);
-  QCL_CUDA_CHECK(cudaMemsetAsync(rowmax, 0, (size_t)Mpad * sizeof(unsigned), st));
-  tc_row_max_kernel<<<dim3(Mpad / 32, (Kc + 255) / 256), 256, 0, st>>>(M, Kc, P, Bs, (const Cx<float>*)A, rowmax);
-  QCL_LAUNCH_CHECK("tc_row_max_kernel");
-  dim3 sg((Mpad + 31) / 32, std::min((Kpad + TC_SPLIT_KK - 1) / TC_SPLIT_KK, 32));
-  tc_split_a_kernel<<<sg, 256, 0, st>>>(M, Kc, Mpad, Kpad, P, Bs, (const Cx<float>*)A, rowmax, Ahi, Alo, ainv);
+  if (Kpad <= TC_SPLIT_KK) {  // whole rows per CTA: one pass
+    tc_split_a_kernel<true><<<(Mpad + 31) / 32, 256, 0, st>>>(M, Kc, Mpad, Kpad, P, Bs, (const Cx<float>*)A, rowmax,
+                                                             Ahi, Alo, ainv);
+  } else {
+    QCL_CUDA_CHECK(cudaMemsetAsync(rowmax, 0, (size_t)Mpad * sizeof(unsigned), st));
+    tc_row_max_kernel<<<dim3(Mpad / 32, (Kc + 255) / 256), 256, 0, st>>>(M, Kc, P, Bs, (const Cx<float>*)A, rowmax);
+    QCL_LAUNCH_CHECK("tc_row_max_kernel");
+    const dim3 sg((Mpad + 31) / 32, std::min((Kpad + TC_SPLIT_KK - 1) / TC_SPLIT_KK, 32));
+    tc_split_a_kernel<false><<<sg, 256, 0, st>>>(M, Kc, Mpad, Kpad, P, Bs, (const Cx<float>*)A, rowmax, Ahi, Alo,
+                                                 ainv);
+  }
   QCL_LAUNCH_CHECK("tc_split_a_kernel");
   return QCL_OK;
 }
