@@ -134,6 +134,13 @@ struct Pipeline {
     pinned_cap = n;
     return QCL_OK;
   }
+  // Whether a staged call has its slots; without them the caller copies
+  // directly, as from pinned arrays.
+  bool can_stage(size_t slot_bytes) {
+    if (ensure_pinned(kSlots * slot_bytes) == QCL_OK) return true;
+    cudaGetLastError();
+    return false;
+  }
   Grow eps, h, in[3], out[3], scale, trL, trG, status, wE, sum, gam;
   int init() {
     for (auto& s : st)
@@ -371,8 +378,12 @@ int qcl_dyson_keldysh(int precision, int NE, int Nk, int Nb, const double* eps, 
   int fields;
   int threads = staged_threads({hin[0], hin[1], hin[2], hout[0], hout[1], hout[2]}, nf, &fields);
   if (slab_bytes > 2 * kStageBytes) threads = 0;  // a momentum is the smallest slab
-  int ms = (int)std::max<size_t>(1, (threads > 0 ? kStageBytes : (64u << 20)) / std::max<size_t>(slab_bytes, 1));
-  ms = std::min(ms, Nk);
+  const auto slab_momenta = [&](size_t bytes) {
+    return std::min((int)std::max<size_t>(1, bytes / std::max<size_t>(slab_bytes, 1)), Nk);
+  };
+  int ms = slab_momenta(kStageBytes);
+  if (threads > 0 && !P.can_stage(slab_bytes * ms * fields)) threads = 0;
+  if (threads == 0) ms = slab_momenta(64u << 20);
   const size_t pitch = (size_t)NE * Nk * es;
   const auto launch = [&](int m0, int cnt, cudaStream_t st) {
     return launch_dyson_keldysh(precision, NE, Nk, Nb, (const double*)P.eps.p, eta, P.h.p, P.in[0].p,
@@ -490,10 +501,11 @@ static int hilbert_host(int precision, int NE, size_t ncols, const double* eps, 
   void* const hout[2] = {out_lam ? out_lam : out_SR, out_gam};
   void* const dout[2] = {P.out[0].p, P.gam.p};
   int fields;
-  const int threads = staged_threads({hin[0], hin[1], hin[2], hout[0], hout[1]}, nf, &fields);
+  int threads = staged_threads({hin[0], hin[1], hin[2], hout[0], hout[1]}, nf, &fields);
+  const size_t per = std::max<size_t>(1, kStageBytes / ((size_t)NE * es));
+  if (threads > 0 && !P.can_stage(per * NE * es * fields)) threads = 0;
   if (threads > 0) {
     CopyTeam team(threads);
-    const size_t per = std::max<size_t>(1, kStageBytes / ((size_t)NE * es));
     const int slabs = (int)((ncols + per - 1) / per);
     const auto parts = [&](int k, std::vector<SlabPart>& in, std::vector<SlabPart>& out) {
       const size_t c0 = (size_t)k * per, off = c0 * NE * es, bytes = std::min(per, ncols - c0) * NE * es;
