@@ -1067,22 +1067,42 @@ template <typename RS, int NP, int BPC> static int launch_residual_t(const Resid
   return QCL_OK;
 }
 
+// r_K alone has no tests and is bound by its loads, where longer runs of
+// energies help: N_b = 32, 1024 x 32 blocks, mixed, 2 per CTA instead of 1: 1.52
+// -> 0.98 ms; N_b = 12 and 16, 4 instead of 2: 6400 blocks, c128, 37 -> 30 us,
+// 3064 blocks, mixed, 30 -> 24 us, but 22 us more at 32768 blocks, which fill
+// the SMs with the smaller CTAs.
+constexpr long long kFewRkBlocks = 8192;
+template <typename RS, int NP, int BPC> static int launch_residual_rk_t(const ResidualArgs<RS>& a, cudaStream_t st) {
+  constexpr size_t smem = BPC * (3 * tile_stride<double, NP, BPC>() * sizeof(Cx<double>) + 4 * sizeof(double));
+  static bool configured = false;
+  if (!configured) {
+    QCL_CUDA_CHECK(cudaFuncSetAttribute(residual_rk_kernel<RS, NP, BPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem));
+    configured = true;
+  }
+  residual_rk_kernel<RS, NP, BPC><<<dim3((a.NE + BPC - 1) / BPC, a.Nk), BPC * Tile<NP>::TT, smem, st>>>(a);
+  QCL_LAUNCH_CHECK("residual_rk_kernel");
+  return QCL_OK;
+}
+
 template <typename RS, int NP, int BPC> static int launch_residual_rows_t(const ResidualArgs<RS>& a, cudaStream_t st) {
   constexpr int TT = Tile<NP>::TT;
   constexpr size_t tile = (size_t)BPC * NP * NP * sizeof(Cx<double>);
   constexpr size_t smem = (rows_four_tiles<NP>() ? 4 : 3) * tile + BPC * (sizeof(RowScratch<NP>) + sizeof(ResScratch<NP>));
-  constexpr size_t smem_rk = 3 * BPC * tile_stride<double, NP, BPC>() * sizeof(Cx<double>) + BPC * 4 * sizeof(double);
   static bool configured = false;
   if (!configured) {
     QCL_CUDA_CHECK(cudaFuncSetAttribute(residual_rows_kernel<RS, NP, BPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
-    QCL_CUDA_CHECK(cudaFuncSetAttribute(residual_rk_kernel<RS, NP, BPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem_rk));
     configured = true;
   }
+  if (a.part == RES_PART_RK) {
+    if (NP == 32) return launch_residual_rk_t<RS, NP, 2>(a, st);
+    if (NP == 16 && (long long)a.NE * a.Nk <= kFewRkBlocks) return launch_residual_rk_t<RS, NP, 4>(a, st);
+    return launch_residual_rk_t<RS, NP, BPC>(a, st);
+  }
   const dim3 grid((a.NE + BPC - 1) / BPC, a.Nk);
-  if (a.part == RES_PART_RK) residual_rk_kernel<RS, NP, BPC><<<grid, BPC * TT, smem_rk, st>>>(a);
-  else residual_rows_kernel<RS, NP, BPC><<<grid, BPC * TT, smem, st>>>(a);
+  residual_rows_kernel<RS, NP, BPC><<<grid, BPC * TT, smem, st>>>(a);
   QCL_LAUNCH_CHECK("residual_rows_kernel");
   return QCL_OK;
 }
