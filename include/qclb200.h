@@ -80,7 +80,8 @@ int qcl_max_basis(void);
  * GL = GR sigL GR^H; GG = GR sigG GR^H.  sigL/sigG/GR/GL/GG/scale/traceL/
  * traceG may be NULL (the matching product or output is skipped).  scale is
  * (N_E, N_k) float64; traceL/traceG are (N_E, N_k) complex128 raw block
- * traces (unweighted).  A singular block returns QCL_SINGULAR. */
+ * traces (unweighted).  A singular block returns QCL_SINGULAR.  Device
+ * variant: GL may be sigL and GG may be sigG (in place). */
 int qcl_dyson_keldysh(int precision, int NE, int Nk, int Nb, const double* eps, double eta, const void* h,
                       const void* sigR, const void* sigL, const void* sigG, void* GR, void* GL, void* GG,
                       double* scale, void* traceL, void* traceG);

@@ -533,6 +533,19 @@ constexpr int kSmallThreads = 64;
 static bool dyson_small(int N, long long blocks) {
   return N <= 4 || (N == 5 && blocks >= 2048) || (N == 6 && blocks >= 4096);
 }
+// The kernel reads a block's Sigma^< and Sigma^> row by row between its
+// stores; the team kernel has them in shared memory before it stores, so a
+// call that writes a Green function over one of them takes that kernel.
+template <typename RS> static bool dyson_in_place(const DysonArgs<RS>& a) {
+  const size_t bytes = (size_t)a.NE * a.Nk * a.N * a.N * sizeof(Cx<RS>);
+  const auto overlap = [&](const void* x, const void* y) {
+    return x && y && (const char*)x < (const char*)y + bytes && (const char*)y < (const char*)x + bytes;
+  };
+  const Cx<RS>* const outs[3] = {a.GR, a.GL, a.GG};
+  for (const Cx<RS>* out : outs)
+    if (overlap(a.sigL, out) || overlap(a.sigG, out)) return true;
+  return false;
+}
 
 template <typename RS, typename RL, typename RM, int N>
 __global__ void __launch_bounds__(kSmallThreads) dyson_small_kernel(DysonArgs<RS> p) {
@@ -783,7 +796,8 @@ static int launch_dyson_np(const DysonArgs<RS>& a, int bpc, cudaStream_t st) {
 
 template <typename RS, typename RL, typename RM>
 static int launch_dyson_prec(const DysonArgs<RS>& a, int precision, int bpc_override, cudaStream_t st) {
-  if (bpc_override <= 0 && dyson_small(a.N, (long long)a.NE * a.mcount)) return launch_dyson_small<RS, RL, RM>(a, st);
+  if (bpc_override <= 0 && dyson_small(a.N, (long long)a.NE * a.mcount) && !dyson_in_place(a))
+    return launch_dyson_small<RS, RL, RM>(a, st);
   const int NP = padded_size(a.N);
   const int bpc = bpc_override > 0 ? bpc_override : dyson_bpc(precision, NP);
   switch (NP) {
