@@ -55,6 +55,12 @@ __device__ __forceinline__ unsigned pivot_key(float mag, int row) {
   return (__float_as_uint(mag) & ~63u) | (unsigned)(63 - row);
 }
 __device__ __forceinline__ bool pivot_key_zero(unsigned key) { return (key >> 6) == 0u; }
+// The magnitude's bits as one integer, for exact comparisons, and the same
+// test for zero.
+__device__ __forceinline__ unsigned long long mag_bits(double mag) { return (unsigned long long)__double_as_longlong(mag); }
+__device__ __forceinline__ unsigned mag_bits(float mag) { return __float_as_uint(mag); }
+__device__ __forceinline__ bool mag_zero(unsigned long long bits) { return (bits >> 38) == 0u; }
+__device__ __forceinline__ bool mag_zero(unsigned bits) { return (bits >> 6) == 0u; }
 
 // Shared-memory store under a predicate, without a branch.
 __device__ __forceinline__ void st_shared_if(Cx<double>* ptr, Cx<double> v, bool pred) {
@@ -581,18 +587,19 @@ __global__ void __launch_bounds__(kSmallThreads) dyson_small_kernel(DysonArgs<RS
   int piv[N], zstep = -1;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
+    // by the bits of the magnitudes, as pivot_key: a NaN ranks above any number
     int best = k;
-    RL mag = cabs1(w[k][k]);
+    auto mag = mag_bits(cabs1(w[k][k]));
 #pragma unroll
     for (int r = k + 1; r < N; ++r) {
-      const RL q = cabs1(w[r][k]);
+      const auto q = mag_bits(cabs1(w[r][k]));
       if (q > mag) {
         mag = q;
         best = r;
       }
     }
     piv[k] = best;
-    const bool zero = pivot_key_zero(pivot_key(mag, 0));
+    const bool zero = mag_zero(mag);
     if (zero && zstep < 0) zstep = k;
 #pragma unroll
     for (int r = k + 1; r < N; ++r)
