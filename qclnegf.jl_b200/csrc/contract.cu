@@ -744,12 +744,13 @@ size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N) {
 }
 
 // The second field's scratch is as large as the first's; where it is not given
-// (work2 == NULL) or an operator's maps gain nothing, the fields go one by one.
+// (work2 == NULL), an operator's maps gain nothing, or the momenta of both
+// fields exceed a grid's z extent, the fields go one by one.
 int launch_contraction_pair(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk,
                             const void* const* G, void* const* S, double alpha_q, void* work, void* work2,
                             cudaStream_t st) {
   const bool scratch = op.kind != QCL_KERNEL_DENSE && op.kind != QCL_KERNEL_SEPARABLE_SUM;
-  if (scratch && !work2) {
+  if (scratch && (!work2 || 2ll * Nk > 65535)) {
     for (int f = 0; f < 2; ++f)
       if (int s = launch_contraction(precision, op, NE, Nk, N, wk, G[f], S[f], alpha_q, 0.0, work, st)) return s;
     return QCL_OK;
