@@ -15,7 +15,9 @@
  * interleaved (re, im) pairs, energy fastest: element (e, m, a, b) (0-based)
  * is at e + N_E*(m + N_k*(a + N_b*b)).  h is (N_k, N_b, N_b) complex128.
  * Matrices are column-major.  `precision` selects the storage/arithmetic:
- *   QCL_C128  complex128 fields, FP64 arithmetic (the reference's precision);
+ *   QCL_C128  complex128 fields, FP64 arithmetic (the reference's precision; the
+ *             products of large dense and separable operators run on exact
+ *             integer digits where every output is at least as accurate so);
  *   QCL_C64   complex64 fields, FP32 arithmetic;
  *   QCL_MIXED complex64 fields, FP64 Dyson inversion, FP32 products,
  *             FP64 reductions.

@@ -191,6 +191,8 @@ template <typename R> struct GemmArgs {
   // 1 = column tiles fastest (they share A tiles: an A larger than L2 is
   // read once); set by launch_gemm for complex128
   int cols_fastest;
+  // complex128: run only if the integer path rejected the product (NULL: always)
+  const int* i8_level;
 };
 
 template <typename R> __device__ __forceinline__ void gemm_store(const GemmArgs<R>& p, Cx<R>* C, int e, int j, Cx<R> acc) {
@@ -337,6 +339,7 @@ template <int BM>
 __global__ void __launch_bounds__(DmShape<BM>::THREADS, BM == 128 ? 2 : 4) dmma_gemm_kernel(const __grid_constant__ GemmArgs<double> p) {
   using S = DmShape<BM>;
   constexpr int TR = S::TR, WM = S::WM, ST = S::STAGES;
+  if (p.i8_level && *p.i8_level != kI8Rejected) return;  // launch-uniform
   extern __shared__ __align__(16) unsigned char dm_raw[];
   Cx<double>* As = reinterpret_cast<Cx<double>*>(dm_raw);            // [ST][DM_BK][APAD]
   Cx<double>* Bs = As + ST * DM_BK * S::APAD;                         // [ST][DM_BK][DM_BPAD]
@@ -519,10 +522,13 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
           return s;
       return QCL_OK;
     }
-    if (sizeof(R) == 8 && op.i8_work && i8_worthwhile(NE, fields, Nc, Nc))
-      return launch_i8_gemm(NE, fields, Nc, Nc, Gv, NEl, wk, Nk, op.matrix, Nc, Sv, NEl, alpha_q, beta, op.i8_work,
-                            op.i8_bytes, op.status, st);
     GemmArgs<R> g{};
+    if (sizeof(R) == 8 && op.i8_work && i8_worthwhile(NE, fields, Nc, Nc)) {
+      if (int s = launch_i8_gemm(NE, fields, Nc, Nc, Gv, NEl, wk, Nk, op.matrix, Nc, Sv, NEl, alpha_q, beta, op.i8_work,
+                                 op.i8_bytes, op.status, st))
+        return s;
+      g.i8_level = (const int*)op.i8_work;
+    }
     g.M = NE; g.Nout = Nc; g.K = Nc; g.batch = 1; g.fields = fields;
     g.lda = NEl; g.wk = wk; g.wk_mod = Nk;
     g.B = (const Cx<R>*)op.matrix; g.ldb = Nc;
@@ -639,13 +645,15 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
       }
       const double bc = c == 0 ? beta : 1.0;
       const Cx<R>* blk = (const Cx<R>*)op.block + (size_t)N2 * N2 * i0;
-      if (sizeof(R) == 8 && op.i8_work && i8_worthwhile((int)Mr, 1, N2, jc * N2)) {
+      const bool i8 = sizeof(R) == 8 && op.i8_work && i8_worthwhile((int)Mr, 1, N2, jc * N2);
+      if (i8) {
         const void* A[1] = {Z};
         void* C[1] = {Sv[fi]};
         if ((s = launch_i8_gemm((int)Mr, 1, N2, jc * N2, A, Mr, nullptr, 1, blk, N2, C, Mr, alpha_q, bc, op.i8_work,
                                 op.i8_bytes, op.status, st)))
           return s;
-      } else if (op.tc_chunks) {
+      }
+      if (op.tc_chunks) {
         if ((s = launch_tc_contraction2((int)Mr, N2, jc * N2, op.tc_chunks[c], Z, Sv[fi], alpha_q, bc, awork, op.status,
                                         st)))
           return s;
@@ -656,6 +664,7 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
         f.B = blk; f.ldb = N2;
         f.C[0] = S[fi]; f.ldc = Mr; f.bcast = 1;
         f.alpha = alpha_q; f.beta = bc;
+        if (i8) f.i8_level = (const int*)op.i8_work;
         if ((s = launch_gemm(f, st))) return s;
       }
     }
@@ -738,7 +747,7 @@ size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N) {
   if (op.kind == QCL_KERNEL_SEPARABLE_SUM) {
     const long long Mr = (long long)NE * Nk;
     const int K = (op.J < kSepChunk ? op.J : kSepChunk) * N2;
-    return i8_worthwhile((int)Mr, 1, N2, K) ? i8_work_bytes((int)(Mr < 4736 ? Mr : 4736), 1, N2, K) : 0;
+    return i8_worthwhile((int)Mr, 1, N2, K) ? i8_work_bytes((int)Mr, 1, N2, K, 4736) : 0;
   }
   return 0;
 }

@@ -15,34 +15,56 @@
 // products left out,
 //   P0 = Re A Re B,  P1 = Im A Im B,  P2 = (Re A + Im A)(Re B + Im B),
 //   Re C = P0 - P1,  Im C = P2 - P0 - P1,
-// each the digit products with s + t <= 7: 36 of 64 int8 GEMMs.  What is left
-// out lies under 2^-64 of a product of row maxima.  On the kernels and Green
-// functions of an SCBA (row rms 0.05 to 0.2 of the row maximum) the error
-// against 64-bit arithmetic with exact sums is 1e-16 of the result, against
-// 5e-16 to 1.5e-15 for FP64 accumulation at K = 216 to 640, which grows with
-// K.  A row with a non-finite value gives NaN in its row (column) of C.
+// each the digit products with s + t <= 7 (36 of 64 int8 GEMMs) or, where the
+// accuracy asks for it, s + t <= 8 (43).  The family of methods is that of
+// Ozaki, Ogita, Oishi and Rump (Numer. Algorithms 59, 2012).
+//
+// Accuracy.  Let MA and MB be the powers of two above the largest parts of the
+// two rows.  The 7 digit products of the first diagonal left out are at most
+// 2^14 each, in units of 2^(48-122): per term of K the error of one part of C
+// is at most 3 x 2^-57.2 = 2^-55.6 of MA MB (three products in Im C) and, the
+// digits being spread over their range, 2^-59.4 rms (1.2e-18 measured), which
+// adds up as sqrt(K).  This is relative to the rows' maxima; an FP64 sum's error
+// is relative to sum_k |a_k| |b_k|: 2K x 2^-53 of it at most, 0.6 to 29e-16 rms
+// measured (least where few terms dominate).  So what decides is
+//   S = sum_k |a_k| |b_k| / (MA MB):
+// by the bounds the two meet at S = 0.08, by the rms at S = 1.2e-18 sqrt(K) /
+// 1.2e-16 = sqrt(K) / 100.  The path runs only where every output lies above
+// that: before it, the leading 7 bits of all entries (rounded down, so that
+// their sum is a lower bound of S) go through one int8 product, 1/108 of the
+// work.  One output below the line adds the diagonal s + t = 8 to the product;
+// what is left then is the rounding of the operands, 2^-62.8 rms of the maxima
+// per entry, whose line is sqrt(K) / 1500.  One output below that rejects the
+// product, which then takes the FP64 tensor path.  Outputs of a zero row are
+// exact and exempt; a non-finite entry rejects.  Errors in units of sum |a| |b|,
+// here / FP64 path:
+//   normal entries, K = 1024 ... 8192: 3.4 ... 1.3e-18 / 6e-17
+//   random form factors with SCBA fields, K = 8192 (S >= 1.5): 1.1e-17 / 5e-16
+//   entries of one sign, K = 1024 ... 8192: 4e-17 / 9 ... 29e-16
+// The screened kernels of a real stack, whose far couplings meet small entries
+// only, go down to S = 1e-8 and are rejected.
 //
 // Sums.  The digit products of one diagonal s + t share an int32 accumulator:
-// at most 8 of them at s + t = 7, so K <= 16320 per accumulation keeps
-// 8 * K * 2^14 below 2^31; a longer K takes several.  Four diagonals of a
-// 128 x BN tile (BN <= 128) fill the 512 columns of tensor memory: two passes
-// over K per product, diagonals 4..7 (26 MMAs per 32 of K) and 0..3 (10).
-// The four sums are combined exactly in 64 bits, converted once and added to
-// C in FP64.
+// at most 8 of them, so K <= 16320 per accumulation keeps 8 * K * 2^14 below
+// 2^31; a longer K takes several.  Four diagonals of a 128 x BN tile (BN <= 128)
+// fill the 512 columns of tensor memory, so a product takes passes over K:
+// diagonals 4..7 (26 MMAs per 32 of K) and 0..3 (10), or 5..8 (28), 1..4 (14)
+// and 0 (1).  The sums of a pass are combined exactly in 64 bits, converted once
+// and added to C in FP64.
 //
 // Kernel: persistent CTAs (one per SM) of 320 threads walk the tiles.  Warp 8
 // streams operand blocks with untiled bulk copies into a 3-stage ring (the
 // split kernels write the operands in the order the MMA reads them: 16-byte
 // K chunks of consecutive rows), warp 9 issues the MMAs, warps 0-7 add the
-// sums to C.  A stage holds 8 digit tiles of A and B: one 32-wide block of K
-// with all 8 digits, or two with the 4 leading ones.
+// sums to C.  A stage holds up to 8 digit tiles of A and B: one 32-wide block of
+// K with all 8 digits, two with the 4 leading ones, eight with one.
 //
 // Bound: the int8 rate and the power limit (980 of 1000 W drawn).  2048 x 8192
 // x 8192 (both Keldysh components of an operator with 32 momenta and 16
 // states): 9.9 ms = 3.0 POP/s of the 4.2 POP/s that resident operands reach,
 // plus 1.2 ms for the split; the FP64 tensor path takes 36 ms.
 #include <algorithm>
-#include <climits>
+#include <cmath>
 
 #include "kernels.cuh"
 #include "tc_prims.cuh"
@@ -54,7 +76,7 @@ constexpr int I8_STAGES = 3, I8_DRAIN = 8, I8_THREADS = 32 * (I8_DRAIN + 2);
 constexpr int I8_A_TILE = I8_BM * I8_KB;            // bytes of one digit tile of A
 constexpr int I8_SEG_KB = 16320 / I8_KB;            // K blocks per accumulation (even)
 constexpr int I8_TOP = 61;                          // |x| < 2^61
-constexpr int I8_BAD = 1 << 20;                     // exponent of a row with a non-finite value
+constexpr int I8_BOUND_MAX_KB = 4096;               // further ones are left out of the bound (int32: 2^17 x 127^2 < 2^31)
 static_assert(8ll * I8_SEG_KB * I8_KB * 128 * 128 < (1ll << 31), "int32 accumulation");
 
 __device__ long long g_i8_main_wait_limit = TC_WAIT_LIMIT;
@@ -102,36 +124,79 @@ struct I8Args {
   int M, mpad;                   // rows of C per field, padded rows per field
   int N;                         // columns of C
   const int *ea, *eb;            // row exponents
+  const unsigned long long *amax, *bmax;  // row maxima (FP64 bits)
+  int* level;                    // of the product: I8_PLAIN, I8_WIDE or kI8Rejected
+  int wide_line, reject_line;    // least sums of leading bits of the first two
   Cx<double>* C[2];              // output fields: rows [f mpad, f mpad + M)
   long long ldc;
   double alpha, beta;
   int* status;
 };
 
-// The digit products of a stage.  PASS 0 (diagonals 4..7, one K block): as
-// digits arrive in the order 0 7 1 6 2 5 3 4; PASS 1 (diagonals 0..3).
-// Accumulator i holds diagonal 4 + i or i.
-template <int BN, int PASS>
-__device__ __forceinline__ void i8_issue(uint32_t st, uint32_t tmem, bool first) {
+// What a launch computes, and its passes over K: blocks of K and digits per
+// stage, the lowest diagonal and the number of diagonals.
+enum { I8_PLAIN = 0, I8_WIDE = 1, I8_BOUND = 3 };
+static_assert(I8_PLAIN < I8_WIDE && I8_WIDE < kI8Rejected, "levels rise");
+template <int MODE> struct I8Passes;
+template <> struct I8Passes<I8_PLAIN> {
+  static constexpr int PLANES = 3, PASSES = 2, SEG_KB = I8_SEG_KB;
+  __device__ static constexpr int blocks(int pass) { return pass ? 2 : 1; }
+  __device__ static constexpr int digits(int pass) { return pass ? 4 : 8; }
+  __device__ static constexpr int low(int pass) { return pass ? 0 : 4; }
+  __device__ static constexpr int sums(int) { return 4; }
+};
+template <> struct I8Passes<I8_WIDE> {
+  static constexpr int PLANES = 3, PASSES = 3, SEG_KB = I8_SEG_KB;
+  __device__ static constexpr int blocks(int pass) { return pass == 2 ? 8 : 1; }
+  __device__ static constexpr int digits(int pass) { return pass == 0 ? 8 : pass == 1 ? 5 : 1; }
+  __device__ static constexpr int low(int pass) { return pass == 0 ? 5 : pass == 1 ? 1 : 0; }
+  __device__ static constexpr int sums(int pass) { return pass == 2 ? 1 : 4; }
+};
+template <> struct I8Passes<I8_BOUND> {  // the leading bits: one plane, one digit
+  static constexpr int PLANES = 1, PASSES = 1, SEG_KB = I8_BOUND_MAX_KB;
+  __device__ static constexpr int blocks(int) { return 8; }
+  __device__ static constexpr int digits(int) { return 1; }
+  __device__ static constexpr int low(int) { return 0; }
+  __device__ static constexpr int sums(int) { return 1; }
+};
+
+// The digit products of a stage with `blocks` K blocks; as digits arrive in the
+// order 0 7 1 6 2 5 3 4.  Accumulator i holds diagonal low + i; `first`: its
+// sums start here.
+template <int BN, int MODE, int PASS>
+__device__ __forceinline__ void i8_issue(uint32_t st, uint32_t tmem, bool first, int blocks) {
   using S = I8Shape<BN>;
+  using P = I8Passes<MODE>;
+  constexpr int BLOCKS = P::blocks(PASS), ND = P::digits(PASS), LOW = P::low(PASS), SUMS = P::sums(PASS);
   constexpr uint32_t idesc = i8_idesc<BN>();
+  static_assert(BLOCKS * ND <= 8, "stage");
   const uint64_t a0 = i8_desc(st, I8_BM), b0 = i8_desc(st + I8_A_TILE, BN);
-  constexpr int BLOCKS = PASS == 0 ? 1 : 2, ND = PASS == 0 ? 8 : 4;
 #pragma unroll
-  for (int kb = 0; kb < BLOCKS; ++kb)
+  for (int kb = 0; kb < BLOCKS; ++kb) {
+    if (kb >= blocks) break;
 #pragma unroll
     for (int s = 0; s < ND; ++s)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int d = PASS == 0 ? 4 + i : i, t = d - s;
+      for (int i = 0; i < SUMS; ++i) {
+        const int t = LOW + i - s;
         if (t < 0 || t >= ND) continue;
         const uint32_t oa = (uint32_t)((kb * ND + s) * S::SUB) >> 4, ob = (uint32_t)((kb * ND + t) * S::SUB) >> 4;
-        i8_mma(tmem + i * 128, a0 + oa, b0 + ob, idesc, (kb == 0 && s == 0) ? (first ? 0u : 1u) : 1u);
+        const bool start = kb == 0 && (s == 0 || t == ND - 1);  // the diagonal's first product
+        i8_mma(tmem + i * 128, a0 + oa, b0 + ob, idesc, start && first ? 0u : 1u);
       }
+  }
 }
 
-template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kernel(const __grid_constant__ I8Args p) {
+// MODE I8_BOUND: raises *level where an output of two non-zero rows lies below
+// a line.  I8_PLAIN, I8_WIDE: the product, if it has that level.
+template <int BN, int MODE>
+__global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kernel(const __grid_constant__ I8Args p) {
   using S = I8Shape<BN>;
+  using P = I8Passes<MODE>;
+  {  // (one answer for the CTA: another one of the launch may raise it)
+    const int level = *(volatile const int*)p.level;
+    if (__syncthreads_or(MODE == I8_BOUND ? level == kI8Rejected : level != MODE)) return;
+  }
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -144,7 +209,7 @@ template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kerne
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles = p.mtiles * p.ntiles;
   const int ntile = (int)blockIdx.x < tiles ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int nseg = (p.nkb + I8_SEG_KB - 1) / I8_SEG_KB;
+  const int nseg = (p.nkb + P::SEG_KB - 1) / P::SEG_KB;
   const long long lim = g_i8_main_wait_limit;
   if (threadIdx.x == 0) {
     for (int i = 0; i < I8_STAGES; ++i) {
@@ -181,22 +246,24 @@ template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kerne
       const int t = (int)blockIdx.x + i * (int)gridDim.x;
       const long long row0 = isb ? (long long)(t / p.mtiles) * BN : (long long)(t % p.mtiles) * I8_BM;
       for (int seg = 0; seg < nseg && ok; ++seg)
-        for (int pl = 0; pl < 3 && ok; ++pl) {
+        for (int pl = 0; pl < P::PLANES && ok; ++pl) {
           const signed char* plane = isb ? p.B + pl * p.b_plane : p.A + pl * p.a_plane;
-          const int k0 = seg * I8_SEG_KB, k1 = min(p.nkb, k0 + I8_SEG_KB);
-          for (int pass = 0; pass < 2 && ok; ++pass)
-            for (int kb = k0; kb < k1; kb += pass ? 2 : 1, ++it) {
+          const int k0 = seg * P::SEG_KB, k1 = min(p.nkb, k0 + P::SEG_KB);
+          for (int pass = 0; pass < P::PASSES && ok; ++pass)
+            for (int kb = k0; kb < k1; kb += P::blocks(pass), ++it) {
               const int s = it % I8_STAGES;
               if (it >= I8_STAGES && !mbar_wait(empty + 8 * s, (uint32_t)((it / I8_STAGES - 1) & 1), lim)) s_fail = 1;
               if (__any_sync(0xffffffffu, s_fail != 0)) {
                 ok = false;
                 break;
               }
-              const int kk = pass ? kb + (sub >> 2) : kb, dg = pass ? sub & 3 : sub;
-              if (lane == 0) mbar_expect_tx(full + 8 * s, S::STAGE);
+              const int nd = P::digits(pass), blocks = min(P::blocks(pass), k1 - kb);
+              const int kk = kb + sub / nd, dg = sub % nd;
+              const long long block = MODE == I8_BOUND ? kk : (long long)kk * I8_S + dg;
+              if (lane == 0) mbar_expect_tx(full + 8 * s, blocks * nd * S::SUB);
               __syncwarp();
-              bulk_load(base + s * S::STAGE + dst, plane + ((((long long)kk * I8_S + dg) * 2 + kc) * rows + row0) * 16,
-                        bytes, full + 8 * s);
+              if (sub < blocks * nd)
+                bulk_load(base + s * S::STAGE + dst, plane + ((block * 2 + kc) * rows + row0) * 16, bytes, full + 8 * s);
               loaded = it + 1;
             }
         }
@@ -207,20 +274,24 @@ template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kerne
       bool ok = true;
       for (int i = 0; i < ntile && ok; ++i)
         for (int seg = 0; seg < nseg && ok; ++seg)
-          for (int pl = 0; pl < 3 && ok; ++pl) {
-            const int k0 = seg * I8_SEG_KB, k1 = min(p.nkb, k0 + I8_SEG_KB);
-            for (int pass = 0; pass < 2 && ok; ++pass, ++u) {
+          for (int pl = 0; pl < P::PLANES && ok; ++pl) {
+            const int k0 = seg * P::SEG_KB, k1 = min(p.nkb, k0 + P::SEG_KB);
+            for (int pass = 0; pass < P::PASSES && ok; ++pass, ++u) {
               if (u > 0 && !mbar_wait(acc_empty, (uint32_t)((u - 1) & 1), lim)) ok = false;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              for (int kb = k0; ok && kb < k1; kb += pass ? 2 : 1, ++it) {
+              for (int kb = k0; ok && kb < k1; kb += P::blocks(pass), ++it) {
                 const int s = it % I8_STAGES;
                 if (s_fail || !mbar_wait(full + 8 * s, (uint32_t)((it / I8_STAGES) & 1), lim)) {
                   ok = false;
                   break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (pass == 0) i8_issue<BN, 0>(base + s * S::STAGE, tmem, kb == k0);
-                else i8_issue<BN, 1>(base + s * S::STAGE, tmem, kb == k0);
+                const uint32_t stage = base + s * S::STAGE;
+                if (pass == 0) i8_issue<BN, MODE, 0>(stage, tmem, kb == k0, k1 - kb);
+                if constexpr (P::PASSES > 1)
+                  if (pass == 1) i8_issue<BN, MODE, 1>(stage, tmem, kb == k0, k1 - kb);
+                if constexpr (P::PASSES > 2)
+                  if (pass == 2) i8_issue<BN, MODE, 2>(stage, tmem, kb == k0, k1 - kb);
                 tc_commit(empty + 8 * s);
                 issued = it + 1;
               }
@@ -243,11 +314,11 @@ template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kerne
       const int f = r / p.mpad, e = r - f * p.mpad;
       const int n0 = (t / p.mtiles) * BN + c0;
       const bool row_ok = e < p.M;
-      const int ea = p.ea[r];
+      const int ea = MODE == I8_BOUND ? 0 : p.ea[r];
       Cx<double>* C = (f ? p.C[1] : p.C[0]) + (row_ok ? e : 0);
       for (int seg = 0; seg < nseg && ok; ++seg)
-        for (int pl = 0; pl < 3 && ok; ++pl)
-          for (int pass = 0; pass < 2; ++pass, ++u) {
+        for (int pl = 0; pl < P::PLANES && ok; ++pl)
+          for (int pass = 0; pass < P::PASSES; ++pass, ++u) {
             const bool stop = __any_sync(0xffffffffu, s_fail != 0);
             if (!__all_sync(0xffffffffu, !stop && mbar_wait(acc_full, (uint32_t)(u & 1), lim))) {
               ok = false;
@@ -255,9 +326,27 @@ template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kerne
               break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if constexpr (MODE == I8_BOUND) {
+              int level = I8_PLAIN;
+              const bool live = row_ok && p.amax[r] != 0;
+#pragma unroll 1
+              for (int c = 0; c < CH; c += 8) {
+                int v[8];
+                tmem_ld8(tmem + tlane + (uint32_t)(c0 + c), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                  if (v[q] < p.wide_line && live && n0 + c + q < p.N && p.bmax[n0 + c + q] != 0)
+                    level = max(level, v[q] < p.reject_line ? kI8Rejected : (int)I8_WIDE);
+              }
+              if (level > *(volatile int*)p.level) atomicMax(p.level, level);
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+              mbar_arrive(acc_empty);
+              continue;
+            }
             const bool first = seg == 0 && pl == 0 && pass == 0;
-            // x = X 2^(e - 61); the four sums in units of 256^7 (pass 0) or 256^11
-            const int unit = ea - 2 * I8_TOP + (pass ? 88 : 56);
+            // x = X 2^(e - 61); the last sum in units of 256^(14 - diagonal)
+            const int unit = ea - 2 * I8_TOP + 8 * (15 - P::low(pass) - P::sums(pass));
             const double sre = pl == 0 ? p.alpha : pl == 1 ? -p.alpha : 0.0, sim = pl == 2 ? p.alpha : -p.alpha;
 #pragma unroll 1
             for (int c = 0; c < CH; c += 8) {
@@ -274,11 +363,10 @@ template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kerne
 #pragma unroll
               for (int q = 0; q < 8; ++q) {
                 if (!row_ok || n0 + c + q >= p.N) continue;
-                const long long x =
-                    ((((long long)v[0][q] << 8) + v[1][q]) * 65536) + (((long long)v[2][q] << 8) + v[3][q]);
-                const int ex = unit + p.eb[n0 + c + q];
-                double y = scalbn((double)x, ex);
-                if (ex >= I8_BAD / 2) y = NAN;
+                const long long x = P::sums(pass) == 1 ? (long long)v[0][q]
+                                                       : ((((long long)v[0][q] << 8) + v[1][q]) * 65536) +
+                                                             (((long long)v[2][q] << 8) + v[3][q]);
+                const double y = scalbn((double)x, unit + p.eb[n0 + c + q]);
                 if (first) o[q] = p.beta == 0.0 ? cx<double>(0, 0) : p.beta * o[q];
                 o[q].x = fma(sre, y, o[q].x);
                 o[q].y = fma(sim, y, o[q].y);
@@ -292,7 +380,10 @@ template <int BN> __global__ void __launch_bounds__(I8_THREADS, 1) i8_gemm_kerne
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (threadIdx.x == 0 && s_fail) record_status(p.status, QCL_TIMEOUT, (long long)blockIdx.x);
+  if (threadIdx.x == 0 && s_fail) {
+    record_status(p.status, QCL_TIMEOUT, (long long)blockIdx.x);
+    if (MODE == I8_BOUND) atomicMax(p.level, kI8Rejected);
+  }
   if (warp == I8_DRAIN + 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   // after a failure copies may still be in flight into this CTA's shared memory
@@ -350,35 +441,76 @@ __device__ __forceinline__ void byte_transpose(unsigned a, unsigned b, unsigned 
   out[3] = __byte_perm(ab1, cd1, 0x7632);
 }
 
-// One thread per row and 16-wide K half: 16 values, their 3 x 16 integers, and
-// 3 x 8 digit rows of 16 bytes.  A warp reads and writes 512 contiguous bytes.
-__global__ void __launch_bounds__(256) i8_split_kernel(I8Src a, const unsigned long long* __restrict__ rowmax,
-                                                       int* __restrict__ exps, signed char* __restrict__ out,
-                                                       long long plane, int halves) {
+// Exponent of a row maximum (0 for a zero row), and the factors of
+// x 2^(top - ex) in two exact steps (either alone stays in range).
+__device__ __forceinline__ int i8_scale(double mx, int top, double& s1, double& s2) {
+  int ex = 0;
+  if (mx > 0.0 && !isinf(mx)) frexp(mx, &ex);
+  const int sh = top - ex, sh1 = sh / 2;
+  s1 = ldexp(1.0, sh1);
+  s2 = ldexp(1.0, sh - sh1);
+  return ex;
+}
+
+// Element k of a row, weighted.
+__device__ __forceinline__ Cx<double> i8_element(const I8Src& a, const Cx<double>* X, int k) {
+  const Cx<double> v = X[a.ld * k];
+  const double w = a.w ? a.w[k % a.wmod] : 1.0;
+  return cx<double>(v.x * w, v.y * w);
+}
+
+// The leading 7 bits of the larger part of every entry, relative to the power
+// of two above the row maximum and rounded down; layout as the digits.  One
+// thread per row and 16-wide K half.
+__global__ void __launch_bounds__(256) i8_leading_kernel(I8Src a, const unsigned long long* __restrict__ rowmax,
+                                                         signed char* __restrict__ out, int halves, int* level) {
+  if (*(volatile const int*)level == kI8Rejected) return;
   const int r = blockIdx.x * 32 + (threadIdx.x & 31), f = r / a.rpad, e = r - f * a.rpad;
   const int half = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (half >= halves) return;
   const bool live = e < a.rows;
   const double mx = live ? __longlong_as_double((long long)rowmax[r]) : 0.0;
-  int ex = 0;
-  const bool bad = isinf(mx);
-  if (mx > 0.0 && !bad) frexp(mx, &ex);
-  if (half == 0) exps[r] = bad ? I8_BAD : ex;
-  // x 2^(61 - ex) in two exact steps (either factor alone stays in range)
-  const int sh = I8_TOP - ex, sh1 = sh / 2;
-  const double s1 = ldexp(1.0, sh1), s2 = ldexp(1.0, sh - sh1);
-  const bool use = live && !bad;
+  double s1, s2;
+  i8_scale(mx, 7, s1, s2);
+  if (isinf(mx) && half == 0) atomicMax(level, kI8Rejected);
+  const bool use = live && !isinf(mx);
+  const Cx<double>* X = (f ? a.X[1] : a.X[0]) + e;
+  unsigned q[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    q[g] = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = half * 16 + 4 * g + i;
+      if (!use || k >= a.K) continue;
+      const Cx<double> v = i8_element(a, X, k);
+      q[g] |= (unsigned)__double2int_rz(fmax(fabs(v.x), fabs(v.y)) * s1 * s2) << (8 * i);
+    }
+  }
+  *reinterpret_cast<uint4*>(out + ((long long)half * a.total + r) * 16) = make_uint4(q[0], q[1], q[2], q[3]);
+}
+
+// One thread per row and 16-wide K half: 16 values, their 3 x 16 integers, and
+// 3 x 8 digit rows of 16 bytes.  A warp reads and writes 512 contiguous bytes.
+__global__ void __launch_bounds__(256) i8_split_kernel(I8Src a, const unsigned long long* __restrict__ rowmax,
+                                                       int* __restrict__ exps, signed char* __restrict__ out,
+                                                       long long plane, int halves, const int* level) {
+  if (*level == kI8Rejected) return;
+  const int r = blockIdx.x * 32 + (threadIdx.x & 31), f = r / a.rpad, e = r - f * a.rpad;
+  const int half = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (half >= halves) return;
+  const bool live = e < a.rows;
+  const double mx = live ? __longlong_as_double((long long)rowmax[r]) : 0.0;
+  double s1, s2;
+  const int ex = i8_scale(mx, I8_TOP, s1, s2);
+  if (half == 0) exps[r] = ex;
   const Cx<double>* X = (f ? a.X[1] : a.X[0]) + e;
   long long xr[16], xi[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const int k = half * 16 + i;
     Cx<double> v = cx<double>(0, 0);
-    if (use && k < a.K) {
-      v = X[a.ld * k];
-      const double w = a.w ? a.w[k % a.wmod] : 1.0;
-      v = cx<double>(v.x * w, v.y * w);
-    }
+    if (live && k < a.K) v = i8_element(a, X, k);
     xr[i] = __double2ll_rn(v.x * s1 * s2);
     xi[i] = __double2ll_rn(v.y * s1 * s2);
   }
@@ -443,135 +575,183 @@ static int i8_pick_bn(int mtiles, int N, int sms, double* cost = nullptr) {
   return best;
 }
 
-struct I8Dims {
-  int mpad, nkb;
-  size_t a_row, b_row;  // bytes per operand row (digits, row maximum, exponent)
+// Operand rows for m rows of a field of A and for n columns (whole tiles of every width).
+static int i8_mpad(int m) { return ceil_div(m, I8_BM) * I8_BM; }
+static int i8_bpad(int n) { return ceil_div(n, I8_MAXBN) * I8_MAXBN + I8_MAXBN; }
+
+// The work area: the product's level, the row maxima of all rows, the exponents
+// and the digits (or leading bits) of one panel of B and one of A.
+struct I8Layout {
+  int mpan, npan, mpans, npans;  // rows of a field and columns per panel, panels
+  int rows, bpad;                // operand rows of a full panel of A (both fields) and of B
+  int nkb;                       // K blocks (even)
+  size_t level, amax, bmax, ea, eb, B, A, bytes;
 };
-static I8Dims i8_dims(int M, int K) {
-  I8Dims d;
-  d.mpad = ceil_div(M, I8_BM) * I8_BM;
-  d.nkb = ceil_div(K, 2 * I8_KB) * 2;
-  d.a_row = d.b_row = 3 * (size_t)d.nkb * I8_KB * I8_S + 16;
-  return d;
+static I8Layout i8_layout(int M, int fields, int N, int K, int mp, int np) {
+  const auto panel = [](int n, int parts, int unit) { return std::min(n, ceil_div(ceil_div(n, parts), unit) * unit); };
+  I8Layout l;
+  l.mpan = panel(M, mp, I8_BM);
+  l.npan = panel(N, np, I8_MAXBN);
+  l.mpans = ceil_div(M, l.mpan);
+  l.npans = ceil_div(N, l.npan);
+  l.rows = fields * i8_mpad(l.mpan);
+  l.bpad = i8_bpad(l.npan);
+  l.nkb = ceil_div(K, 2 * I8_KB) * 2;
+  size_t at = 0;
+  const auto take = [&](size_t n) {
+    const size_t r = at;
+    at += (n + 255) / 256 * 256;
+    return r;
+  };
+  const size_t row = 3 * (size_t)l.nkb * I8_KB * I8_S;  // digits; the leading bits take less
+  l.level = take(sizeof(int));
+  l.amax = take((size_t)l.mpans * l.rows * 8);
+  l.bmax = take((size_t)l.npans * l.bpad * 8);
+  l.ea = take((size_t)l.rows * 4);
+  l.eb = take((size_t)l.bpad * 4);
+  l.B = take(l.bpad * row);
+  l.A = take(l.rows * row);
+  l.bytes = at;
+  return l;
 }
-// Rows of a padded B panel: whole tiles of every width.
-static int i8_bpad(int N) { return ceil_div(N, I8_MAXBN) * I8_MAXBN + I8_MAXBN; }
 
-size_t i8_work_bytes(int M, int fields, int N, int K) {
-  const I8Dims d = i8_dims(M, K);
-  return (size_t)fields * d.mpad * d.a_row + (size_t)i8_bpad(N) * d.b_row + 4096;
+size_t i8_work_bytes(int M, int fields, int N, int K, int panel_rows) {
+  return i8_layout(M, fields, N, K, panel_rows > 0 ? ceil_div(M, panel_rows) : 1, 1).bytes;
 }
 
-// Whether the product is large enough for the split to pay (FP64 tensor path
-// against this one, both passes and the split included):
-//   rows x K x columns  2048 x 576^2: 192 / 181 us, 1000 x 1152^2: 374 / 279 us,
-//   383 x 2048^2: 667 / 470 us, 1024 x 2048^2: 1301 / 530 us, 1024 x 8192^2:
-//   17.98 / 6.92 ms; below the line 400 x 1152^2: 225 / 276 us, 128 x 2048^2:
-//   392 / 462 us, 64 x 4096^2: 780 / 980 us (few row tiles, split costs remain).
+// Whether the product is large enough for the bound and the split to pay.  One
+// iteration of a solve with one such map, FP64 tensor path / this one / this one
+// rejecting the product (rows x K x columns):
+//   1000 x 1152^2: 767 / 772 / 828 us, 384 x 2048^2: 820 / 782 / 860 us,
+//   1024 x 2048^2: 1734 / 1149 / 1820 us, 2048 x 4096^2: 10.87 / 5.60 / 11.21 ms;
+// beyond the lines 600 x 1152^2 (8e8): 578 us at best either way, 192 x 4096^2:
+// 1299 / 1370 / 1486 us (few rows share the passes over B).
 bool i8_worthwhile(int M, int fields, int N, int K) {
-  return (double)M * fields * N * K >= 1e9 && (long long)M * fields >= 192 && N >= 64 && K >= 64;
+  return (double)M * fields * N * K >= 1e9 && (long long)M * fields >= 384 && N >= 64 && K >= 64;
 }
 
-template <int BN> static int launch_i8_t(const I8Args& a, int sms, cudaStream_t st) {
+template <int BN, int MODE> static int launch_i8_t(const I8Args& a, int sms, cudaStream_t st) {
   static bool configured = false;
   if (!configured) {
-    QCL_CUDA_CHECK(cudaFuncSetAttribute(i8_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<BN>::SMEM));
+    QCL_CUDA_CHECK(
+        cudaFuncSetAttribute(i8_gemm_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<BN>::SMEM));
     configured = true;
   }
   const int tiles = a.mtiles * a.ntiles;
-  i8_gemm_kernel<BN><<<std::min(tiles, sms), I8_THREADS, I8Shape<BN>::SMEM, st>>>(a);
+  i8_gemm_kernel<BN, MODE><<<std::min(tiles, sms), I8_THREADS, I8Shape<BN>::SMEM, st>>>(a);
   QCL_LAUNCH_CHECK("i8_gemm_kernel");
   return QCL_OK;
 }
 
-static int i8_split(const I8Src& a, unsigned long long* rowmax, int* exps, signed char* out, int nkb, cudaStream_t st) {
+template <int BN> static int launch_i8_levels(const I8Args& a, int sms, cudaStream_t st) {
+  const int s = launch_i8_t<BN, I8_PLAIN>(a, sms, st);
+  return s ? s : launch_i8_t<BN, I8_WIDE>(a, sms, st);
+}
+
+static int i8_row_max(const I8Src& a, unsigned long long* rowmax, cudaStream_t st) {
   QCL_CUDA_CHECK(cudaMemsetAsync(rowmax, 0, (size_t)a.total * sizeof(unsigned long long), st));
   const int rb = a.total / 32;
-  int ks = std::max(1, std::min(ceil_div(a.K, 64), 8 * 148 / rb));
+  const int ks = std::max(1, std::min(ceil_div(a.K, 64), 8 * 148 / rb));
   const int kper = ceil_div(a.K, ks);
   i8_row_max_kernel<<<dim3(rb, ceil_div(a.K, kper)), 256, 0, st>>>(a, rowmax, kper);
   QCL_LAUNCH_CHECK("i8_row_max_kernel");
+  return QCL_OK;
+}
+
+// K blocks of leading bits.
+static int i8_bound_blocks(int K) { return std::min(ceil_div(K, I8_KB), I8_BOUND_MAX_KB); }
+static int i8_leading(const I8Src& a, const unsigned long long* rowmax, signed char* out, int* level, cudaStream_t st) {
+  const int halves = 2 * i8_bound_blocks(a.K);
+  i8_leading_kernel<<<dim3(a.total / 32, ceil_div(halves, 8)), 256, 0, st>>>(a, rowmax, out, halves, level);
+  QCL_LAUNCH_CHECK("i8_leading_kernel");
+  return QCL_OK;
+}
+
+static int i8_split(const I8Src& a, const unsigned long long* rowmax, int* exps, signed char* out, int nkb,
+                    const int* level, cudaStream_t st) {
   const long long plane = (long long)nkb * I8_S * 2 * a.total * 16;
-  i8_split_kernel<<<dim3(rb, ceil_div(2 * nkb, 8)), 256, 0, st>>>(a, rowmax, exps, out, plane, 2 * nkb);
+  i8_split_kernel<<<dim3(a.total / 32, ceil_div(2 * nkb, 8)), 256, 0, st>>>(a, rowmax, exps, out, plane, 2 * nkb,
+                                                                            level);
   QCL_LAUNCH_CHECK("i8_split_kernel");
   return QCL_OK;
 }
 
+// The product, unless *(int*)work is kI8Rejected afterwards: then C is as it
+// was, and the caller's launch on the FP64 tensor path takes over
+// (GemmArgs::i8_level).
 int launch_i8_gemm(int M, int fields, int N, int K, const void* const* A, long long lda, const double* w, int wmod,
                    const void* B, long long ldb, void* const* C, long long ldc, double alpha, double beta, void* work,
                    size_t work_bytes, int* status, cudaStream_t st) {
-  const I8Dims d = i8_dims(M, K);
   const int sms = sm_count();
   // panels: rows of A (one field) and columns of B that the work area holds
   int mp = 1, np = 1;
-  auto panel = [](int n, int parts, int unit) { return std::min(n, ceil_div(ceil_div(n, parts), unit) * unit); };
-  auto need = [&]() {
-    const int m = panel(M, mp, I8_BM), n = panel(N, np, I8_MAXBN);
-    return i8_work_bytes(m, fields, n, K);
-  };
-  while (need() > work_bytes) {
-    const size_t ab = (size_t)fields * panel(M, mp, I8_BM) * d.a_row, bb = (size_t)panel(N, np, I8_MAXBN) * d.b_row;
-    if (ab >= bb && panel(M, mp, I8_BM) > I8_BM) ++mp;
-    else if (panel(N, np, I8_MAXBN) > I8_MAXBN) ++np;
-    else if (panel(M, mp, I8_BM) > I8_BM) ++mp;
+  I8Layout l = i8_layout(M, fields, N, K, mp, np);
+  while (l.bytes > work_bytes) {
+    if (l.rows >= l.bpad && l.mpan > I8_BM) ++mp;
+    else if (l.npan > I8_MAXBN) ++np;
+    else if (l.mpan > I8_BM) ++mp;
     else {
       set_last_error("i8 product: work area of %zu bytes is too small", work_bytes);
       return QCL_UNSUPPORTED;
     }
+    l = i8_layout(M, fields, N, K, mp, np);
   }
-  const int mpan = panel(M, mp, I8_BM), npan = panel(N, np, I8_MAXBN);
-  for (int n0 = 0; n0 < N; n0 += npan) {
-    const int n = std::min(npan, N - n0), bpad = i8_bpad(n);
-    char* q = (char*)work;
-    auto take = [&](size_t bytes) {
-      char* r = q;
-      q += (bytes + 255) / 256 * 256;
-      return r;
-    };
-    unsigned long long* bmax = (unsigned long long*)take((size_t)bpad * 8);
-    int* eb = (int*)take((size_t)bpad * 4);
-    signed char* Bd = (signed char*)take(3 * (size_t)d.nkb * I8_KB * I8_S * bpad);
-    int s;
-    I8Src bs{{(const Cx<double>*)B + n0, nullptr}, ldb, nullptr, 1, n, bpad, bpad, K};
-    if ((s = i8_split(bs, bmax, eb, Bd, d.nkb, st))) return s;
-    for (int m0 = 0; m0 < M; m0 += mpan) {
-      const int m = std::min(mpan, M - m0), mpad = ceil_div(m, I8_BM) * I8_BM, rows = fields * mpad;
-      char* keep = q;
-      unsigned long long* amax = (unsigned long long*)take((size_t)rows * 8);
-      int* ea = (int*)take((size_t)rows * 4);
-      signed char* Ad = (signed char*)take(3 * (size_t)d.nkb * I8_KB * I8_S * rows);
-      q = keep;
-      I8Src as{{(const Cx<double>*)A[0] + m0, fields > 1 ? (const Cx<double>*)A[1] + m0 : nullptr}, lda, w, wmod, m, mpad,
-               rows, K};
-      if ((s = i8_split(as, amax, ea, Ad, d.nkb, st))) return s;
-      I8Args g{};
-      g.A = Ad;
-      g.B = Bd;
-      g.a_plane = (long long)d.nkb * I8_S * 2 * rows * 16;
-      g.b_plane = (long long)d.nkb * I8_S * 2 * bpad * 16;
-      g.a_rows = rows;
-      g.b_rows = bpad;
-      g.nkb = d.nkb;
-      g.mtiles = rows / I8_BM;
-      g.M = m;
-      g.mpad = mpad;
-      g.N = n;
-      g.ea = ea;
-      g.eb = eb;
-      for (int f = 0; f < fields; ++f) g.C[f] = (Cx<double>*)C[f] + m0 + ldc * n0;
-      g.ldc = ldc;
-      g.alpha = alpha;
-      g.beta = beta;
-      g.status = status;
-      const int bn = i8_pick_bn(g.mtiles, n, sms);
-      g.ntiles = ceil_div(n, bn);
-      if (bn == 128) s = launch_i8_t<128>(g, sms, st);
-      else if (bn == 112) s = launch_i8_t<112>(g, sms, st);
-      else if (bn == 96) s = launch_i8_t<96>(g, sms, st);
-      else s = launch_i8_t<64>(g, sms, st);
-      if (s) return s;
+  char* const base = (char*)work;
+  int* const level = (int*)(base + l.level);
+  int *const ea = (int*)(base + l.ea), *const eb = (int*)(base + l.eb);
+  signed char *const Bd = (signed char*)(base + l.B), *const Ad = (signed char*)(base + l.A);
+  QCL_CUDA_CHECK(cudaMemsetAsync(level, 0, sizeof(int), st));
+  int s;
+  for (int bound = 1; bound >= 0; --bound)  // the bound of every panel before the first digit of C
+    for (int j = 0; j < l.npans; ++j) {
+      const int n0 = j * l.npan, n = std::min(l.npan, N - n0), bpad = i8_bpad(n);
+      unsigned long long* const bmax = (unsigned long long*)(base + l.bmax) + (size_t)j * l.bpad;
+      const I8Src bs{{(const Cx<double>*)B + n0, nullptr}, ldb, nullptr, 1, n, bpad, bpad, K};
+      if (bound && (s = i8_row_max(bs, bmax, st))) return s;
+      if ((s = bound ? i8_leading(bs, bmax, Bd, level, st) : i8_split(bs, bmax, eb, Bd, l.nkb, level, st))) return s;
+      for (int i = 0; i < l.mpans; ++i) {
+        const int m0 = i * l.mpan, m = std::min(l.mpan, M - m0), mpad = i8_mpad(m), rows = fields * mpad;
+        unsigned long long* const amax = (unsigned long long*)(base + l.amax) + (size_t)i * l.rows;
+        const I8Src as{{(const Cx<double>*)A[0] + m0, fields > 1 ? (const Cx<double>*)A[1] + m0 : nullptr}, lda, w, wmod,
+                       m, mpad, rows, K};
+        if (bound && j == 0 && (s = i8_row_max(as, amax, st))) return s;
+        if (j == 0 || l.mpans > 1)
+          if ((s = bound ? i8_leading(as, amax, Ad, level, st) : i8_split(as, amax, ea, Ad, l.nkb, level, st)))
+            return s;
+        I8Args g{};
+        g.A = Ad;
+        g.B = Bd;
+        g.a_plane = (long long)l.nkb * I8_S * 2 * rows * 16;
+        g.b_plane = (long long)l.nkb * I8_S * 2 * bpad * 16;
+        g.a_rows = rows;
+        g.b_rows = bpad;
+        g.nkb = bound ? i8_bound_blocks(K) : l.nkb;
+        g.mtiles = rows / I8_BM;
+        g.M = m;
+        g.mpad = mpad;
+        g.N = n;
+        g.ea = ea;
+        g.eb = eb;
+        g.amax = amax;
+        g.bmax = bmax;
+        g.level = level;
+        g.wide_line = (int)ceil(16384 * sqrt((double)K) / 100);
+        g.reject_line = (int)ceil(16384 * sqrt((double)K) / 1500);
+        for (int f = 0; f < fields; ++f) g.C[f] = (Cx<double>*)C[f] + m0 + ldc * n0;
+        g.ldc = ldc;
+        g.alpha = alpha;
+        g.beta = beta;
+        g.status = status;
+        const int bn = bound ? 128 : i8_pick_bn(g.mtiles, n, sms);
+        g.ntiles = ceil_div(n, bn);
+        if (bound) s = launch_i8_t<128, I8_BOUND>(g, sms, st);
+        else if (bn == 128) s = launch_i8_levels<128>(g, sms, st);
+        else if (bn == 112) s = launch_i8_levels<112>(g, sms, st);
+        else if (bn == 96) s = launch_i8_levels<96>(g, sms, st);
+        else s = launch_i8_levels<64>(g, sms, st);
+        if (s) return s;
+      }
     }
-  }
   return QCL_OK;
 }
 

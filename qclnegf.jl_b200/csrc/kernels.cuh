@@ -161,8 +161,10 @@ int launch_tc_presplit(int M, int Nout, int Kc, const void* Bop, const float* aw
 int launch_tc_dense_contraction(int NE, int Nc, const void* Bop, const void* G, void* S, double alpha, double beta,
                                 float* awork, int* status, cudaStream_t st);
 // complex128 products on the integer tensor path (i8_gemm.cu): up to two
-// fields of M rows against one operator
-size_t i8_work_bytes(int M, int fields, int N, int K);
+// fields of M rows against one operator, where that is as accurate as FP64 sums
+constexpr int kI8Rejected = 2;  // the product's level (first word of the work area) where it is not
+// (panel_rows > 0: rows of A at a time)
+size_t i8_work_bytes(int M, int fields, int N, int K, int panel_rows = 0);
 bool i8_worthwhile(int M, int fields, int N, int K);
 int launch_i8_gemm(int M, int fields, int N, int K, const void* const* A, long long lda, const double* w, int wmod,
                    const void* B, long long ldb, void* const* C, long long ldc, double alpha, double beta, void* work,
