@@ -487,6 +487,12 @@ static int launch_gemm(const GemmArgs<double>& args, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Contraction dispatch
 // ---------------------------------------------------------------------------
+// Whether a complex128 product goes to the integer path: large enough, and
+// the operator's work area holds its smallest panels.
+static bool takes_i8(const KernelOpDev& op, int M, int fields, int N, int K) {
+  return op.i8_work && i8_worthwhile(M, fields, N, K) && op.i8_bytes >= i8_least_bytes(M, fields, N, K);
+}
+
 // One or two fields G[f] -> S[f].  work holds contraction_work_elems elements;
 // with two fields, work2 as many again.
 template <typename R>
@@ -523,7 +529,7 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
       return QCL_OK;
     }
     GemmArgs<R> g{};
-    if (sizeof(R) == 8 && op.i8_work && i8_worthwhile(NE, fields, Nc, Nc)) {
+    if (sizeof(R) == 8 && takes_i8(op, NE, fields, Nc, Nc)) {
       if (int s = launch_i8_gemm(NE, fields, Nc, Nc, Gv, NEl, wk, Nk, op.matrix, Nc, Sv, NEl, alpha_q, beta, op.i8_work,
                                  op.i8_bytes, op.status, st))
         return s;
@@ -645,7 +651,7 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
       }
       const double bc = c == 0 ? beta : 1.0;
       const Cx<R>* blk = (const Cx<R>*)op.block + (size_t)N2 * N2 * i0;
-      const bool i8 = sizeof(R) == 8 && op.i8_work && i8_worthwhile((int)Mr, 1, N2, jc * N2);
+      const bool i8 = sizeof(R) == 8 && takes_i8(op, (int)Mr, 1, N2, jc * N2);
       if (i8) {
         const void* A[1] = {Z};
         void* C[1] = {Sv[fi]};
@@ -738,16 +744,21 @@ size_t contraction_work_elems(const KernelOpDev& op, int NE, int Nk, int N) {
 
 // The area for the whole operands, or, for a stage-2 product of a separable
 // sum with many more rows than columns, for a panel of rows.
-size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N) {
+size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N, size_t* least) {
   const int N2 = N * N;
+  if (least) *least = 0;
   if (op.kind == QCL_KERNEL_DENSE) {
     const int Nc = Nk * N2;
-    return i8_worthwhile(NE, 2, Nc, Nc) ? i8_work_bytes(NE, 2, Nc, Nc) : 0;
+    if (!i8_worthwhile(NE, 2, Nc, Nc)) return 0;
+    if (least) *least = i8_least_bytes(NE, 2, Nc, Nc);
+    return i8_work_bytes(NE, 2, Nc, Nc);
   }
   if (op.kind == QCL_KERNEL_SEPARABLE_SUM) {
     const long long Mr = (long long)NE * Nk;
     const int K = (op.J < kSepChunk ? op.J : kSepChunk) * N2;
-    return i8_worthwhile((int)Mr, 1, N2, K) ? i8_work_bytes((int)Mr, 1, N2, K, 4736) : 0;
+    if (!i8_worthwhile((int)Mr, 1, N2, K)) return 0;
+    if (least) *least = i8_least_bytes((int)Mr, 1, N2, K);
+    return i8_work_bytes((int)Mr, 1, N2, K, 4736);
   }
   return 0;
 }

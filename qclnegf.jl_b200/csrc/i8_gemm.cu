@@ -618,6 +618,9 @@ static I8Layout i8_layout(int M, int fields, int N, int K, int mp, int np) {
 size_t i8_work_bytes(int M, int fields, int N, int K, int panel_rows) {
   return i8_layout(M, fields, N, K, panel_rows > 0 ? ceil_div(M, panel_rows) : 1, 1).bytes;
 }
+size_t i8_least_bytes(int M, int fields, int N, int K) {
+  return i8_layout(M, fields, N, K, ceil_div(M, I8_BM), ceil_div(N, I8_MAXBN)).bytes;
+}
 
 // Whether the product is large enough for the bound and the split to pay.  One
 // iteration of a solve with one such map, FP64 tensor path / this one / this one

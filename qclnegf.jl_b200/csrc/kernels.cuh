@@ -165,13 +165,15 @@ int launch_tc_dense_contraction(int NE, int Nc, const void* Bop, const void* G, 
 constexpr int kI8Rejected = 2;  // the product's level (first word of the work area) where it is not
 // (panel_rows > 0: rows of A at a time)
 size_t i8_work_bytes(int M, int fields, int N, int K, int panel_rows = 0);
+size_t i8_least_bytes(int M, int fields, int N, int K);  // with the smallest panels
 bool i8_worthwhile(int M, int fields, int N, int K);
 int launch_i8_gemm(int M, int fields, int N, int K, const void* const* A, long long lda, const double* w, int wmod,
                    const void* B, long long ldb, void* const* C, long long ldc, double alpha, double beta, void* work,
                    size_t work_bytes, int* status, cudaStream_t st);
 int i8_set_wait_limit(long long rounds);
-// Work area of the integer path a complex128 contraction would use (0: none).
-size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N);
+// Work area of the integer path a complex128 contraction would use (0: none)
+// and the least it takes; with less the FP64 tensor path runs.
+size_t contraction_i8_bytes(const KernelOpDev& op, int NE, int Nk, int N, size_t* least = nullptr);
 // Two fields through one operator: S[f] = alpha_q K[wk G[f]].
 int launch_contraction_pair(int precision, const KernelOpDev& op, int NE, int Nk, int N, const double* wk,
                             const void* const* G, void* const* S, double alpha_q, void* work, void* work2,

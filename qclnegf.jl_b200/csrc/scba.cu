@@ -459,7 +459,7 @@ int scba_estimate_memory(const qcl_scba_problem* p, const qcl_mechanism* mechs, 
 // The work area of the integer tensor path, from what the budget leaves over:
 // the contractions run without one (on the FP64 tensor path), so a budget
 // that holds the plan stays sufficient.  Smaller areas split the operands in
-// panels.  Without an explicit budget other contexts will want the device's
+// panels, down to what the least demanding map can use.  Without an explicit budget other contexts will want the device's
 // free memory too: at most a quarter of it.
 static void i8_area(ScbaCtx* c) {
   if (c->precision != QCL_C128 || c->i8_work) return;
@@ -467,8 +467,13 @@ static void i8_area(ScbaCtx* c) {
   if (c->budget) room = c->budget > c->base_peak ? c->budget - c->base_peak : 0;
   else if (cudaMemGetInfo(&room, &tot) == cudaSuccess) room /= 4;
   else room = 0;
-  for (auto& m : c->mech) want = std::max(want, contraction_i8_bytes(m.view(), c->NE, c->Nk, c->N));
-  for (int cut = 1; want > 0 && cut <= 8; cut *= 2) {
+  size_t least = SIZE_MAX;
+  for (auto& m : c->mech) {
+    size_t l;
+    want = std::max(want, contraction_i8_bytes(m.view(), c->NE, c->Nk, c->N, &l));
+    if (l > 0) least = std::min(least, l);
+  }
+  for (int cut = 1; cut <= 8 && want / cut >= least; cut *= 2) {
     const size_t n = want / cut;
     if (n > room) continue;
     if (cudaMalloc(&c->i8_work, n) == cudaSuccess) {
