@@ -464,7 +464,8 @@ int scba_estimate_memory(const qcl_scba_problem* p, const qcl_mechanism* mechs, 
 static void i8_area(ScbaCtx* c) {
   if (c->precision != QCL_C128 || c->i8_work) return;
   size_t want = 0, room = 0, tot = 0;
-  if (c->budget) room = c->budget > c->base_peak ? c->budget - c->base_peak : 0;
+  const size_t held = c->base_peak + c->br_bytes;  // (a promoted context has its branches already)
+  if (c->budget) room = c->budget > held ? c->budget - held : 0;
   else if (cudaMemGetInfo(&room, &tot) == cudaSuccess) room /= 4;
   else room = 0;
   size_t least = SIZE_MAX;
