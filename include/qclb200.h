@@ -371,8 +371,8 @@ typedef struct qcl_scba_problem {
  * during creation (resident plus the largest complex128 staging copy of an
  * operator array).  A QCL_C128 context with large dense or separable-sum
  * operators also takes a work area for the integer tensor path from what its
- * memory_budget_bytes leaves over (with no budget given, from a quarter of the
- * free memory at most); it runs without one where there is no room, so the
+ * memory_budget_bytes leaves over (with no budget given, a quarter of the free
+ * memory and 2 GiB at most); it runs without one where there is no room, so the
  * estimate is what a budget has to hold.  The role of _estimate_production_memory
  * (numerics/optimized/production_cache.jl:475-668) for this library's own
  * allocation plan. */

@@ -459,14 +459,17 @@ int scba_estimate_memory(const qcl_scba_problem* p, const qcl_mechanism* mechs, 
 // The work area of the integer tensor path, from what the budget leaves over:
 // the contractions run without one (on the FP64 tensor path), so a budget
 // that holds the plan stays sufficient.  Smaller areas split the operands in
-// panels, down to what the least demanding map can use.  Without an explicit budget other contexts will want the device's
-// free memory too: at most a quarter of it.
+// panels, down to what the least demanding map can use.  Without an explicit
+// budget other contexts will want the device's free memory too: at most a
+// quarter of it and kI8FreeBytes, which holds the digits of a dense operator
+// of 8192 rows whole.
+constexpr size_t kI8FreeBytes = (size_t)2 << 30;
 static void i8_area(ScbaCtx* c) {
   if (c->precision != QCL_C128 || c->i8_work) return;
   size_t want = 0, room = 0, tot = 0;
   const size_t held = c->base_peak + c->br_bytes;  // (a promoted context has its branches already)
   if (c->budget) room = c->budget > held ? c->budget - held : 0;
-  else if (cudaMemGetInfo(&room, &tot) == cudaSuccess) room /= 4;
+  else if (cudaMemGetInfo(&room, &tot) == cudaSuccess) room = std::min(room / 4, kI8FreeBytes);
   else room = 0;
   size_t least = SIZE_MAX;
   for (auto& m : c->mech) {

@@ -32,3 +32,28 @@ def test_any_budget_above_the_estimate_runs(gpu_ops, NE, Nk, Nb):
     for r in rows:
         assert r["status"] == 0
         assert abs(r["J"] - rows[0]["J"]) <= 1e-9 * abs(rows[0]["J"])
+
+
+def test_area_without_a_budget_is_bounded(gpu_ops):
+    """An operator of 10 240 rows, whose digits take 2.6 GB: without a budget the
+    context keeps at most 2 GiB (and the allocator's 2 MB pages) beyond its
+    estimate."""
+    import dataclasses
+
+    import numpy as np
+    import torch
+    from qclb200.scba import ProductionSCBA, estimate_memory
+
+    pr = _problem(192, 2, 16)
+    Nk = 40
+    nc = Nk * 16 * 16
+    pr = dataclasses.replace(
+        pr, Nk=Nk, wk=np.full(Nk, 0.1), h=np.asfortranarray(np.repeat(pr.h[:1], Nk, axis=0)),
+        mechanisms=[dataclasses.replace(pr.mechanisms[0], matrix=np.asfortranarray(np.eye(nc, dtype=complex)))])
+    ProductionSCBA(_problem(33, 2, 4)).close()  # the library's own memory
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    s = ProductionSCBA(pr)
+    used = before - torch.cuda.mem_get_info()[0]
+    s.close()
+    assert used < estimate_memory(pr)["resident"] + (2 << 30) + (128 << 20)
