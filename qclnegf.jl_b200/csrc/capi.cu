@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -218,7 +219,13 @@ static int run_staged_slabs(Pipeline& P, int slabs, size_t slot_bytes, CopyTeam&
 
 template <typename Parts, typename Launch>
 static int run_staged(Pipeline& P, int slabs, size_t slot_bytes, CopyTeam& team, Parts&& parts, Launch&& launch) {
-  const int s = run_staged_slabs(P, slabs, slot_bytes, team, parts, launch);
+  int s;
+  try {
+    s = run_staged_slabs(P, slabs, slot_bytes, team, parts, launch);
+  } catch (const std::bad_alloc&) {  // the lists of a slab's pieces
+    set_last_error("out of host memory while staging");
+    s = QCL_NOMEM;
+  }
   if (s)  // nothing of a failed call may still use the slots
     for (auto st : P.st) cudaStreamSynchronize(st);
   return s;

@@ -1,19 +1,33 @@
 #include "staging.cuh"
 
+#include <sched.h>
+#include <stdio.h>
 #include <string.h>
 
 #include <algorithm>
-#include <system_error>
+#include <exception>
 
 namespace qcl {
 
 constexpr size_t kUnitBytes = (size_t)256 << 10;
+constexpr int kSpins = 2000;  // yields before a wait sleeps: longer than the gaps between slabs
+
+// Cores that this process may use: its affinity and its CPU quota.
+static int usable_cores() {
+  cpu_set_t set;
+  int n = sched_getaffinity(0, sizeof(set), &set) == 0 ? CPU_COUNT(&set) : (int)std::thread::hardware_concurrency();
+  if (FILE* f = fopen("/sys/fs/cgroup/cpu.max", "r")) {
+    double quota, period;
+    if (fscanf(f, "%lf %lf", &quota, &period) == 2 && period > 0) n = std::min(n, std::max(1, (int)(quota / period)));
+    fclose(f);
+  }
+  return n;
+}
 
 int copy_threads(size_t bytes) {
   // Below 8 MB starting threads costs what they save.
   if (bytes < ((size_t)8 << 20)) return 0;
-  const unsigned n = std::thread::hardware_concurrency();
-  return (int)std::min(n > 1 ? n - 1 : 0u, 11u);
+  return std::min(std::max(usable_cores() - 1, 0), 11);
 }
 
 HostKind host_kind(const void* p) {
@@ -30,24 +44,30 @@ CopyTeam::CopyTeam(int threads) {
     threads_.reserve(threads > 0 ? threads : 0);
     for (int i = 0; i < threads; ++i)
       threads_.emplace_back([this] {
-        unsigned seen = 0;
-        for (;;) {
-          unsigned r;
-          while ((r = round_.load(std::memory_order_acquire)) == seen) {
-            if (stop_.load(std::memory_order_relaxed)) return;
-            std::this_thread::yield();
-          }
-          seen = r;
+        for (unsigned seen = 0;;) {
+          for (int q = 0; q < kSpins && round_ == seen && !stop_; ++q) std::this_thread::yield();
+          std::unique_lock<std::mutex> lock(m_);
+          start_.wait(lock, [&] { return stop_ || round_ != seen; });
+          if (stop_) return;
+          seen = round_;
+          if (!open_) continue;
+          ++active_;
+          lock.unlock();
           work();
-          busy_.fetch_sub(1, std::memory_order_release);
+          lock.lock();
+          if (--active_ == 0) done_.notify_one();
         }
       });
-  } catch (const std::system_error&) {  // fewer threads, or none
+  } catch (const std::exception&) {  // fewer threads, or none
   }
 }
 
 CopyTeam::~CopyTeam() {
-  stop_.store(true);
+  {
+    std::lock_guard<std::mutex> lock(m_);
+    stop_ = true;
+  }
+  start_.notify_all();
   for (auto& t : threads_) t.join();
 }
 
@@ -81,10 +101,24 @@ void CopyTeam::copy(const std::vector<CopyPiece>& pieces) {
   }
   pieces_ = &cut;
   next_.store(0, std::memory_order_relaxed);
-  busy_.store((int)threads_.size(), std::memory_order_relaxed);
-  round_.fetch_add(1, std::memory_order_release);
+  if (!threads_.empty()) {
+    {
+      std::lock_guard<std::mutex> lock(m_);
+      open_ = true;
+      ++round_;
+    }
+    start_.notify_all();
+  }
   work();
-  while (busy_.load(std::memory_order_acquire) != 0) std::this_thread::yield();
+  if (threads_.empty()) return;
+  std::unique_lock<std::mutex> lock(m_);
+  open_ = false;
+  for (int q = 0; q < kSpins && active_ != 0; ++q) {
+    lock.unlock();
+    std::this_thread::yield();
+    lock.lock();
+  }
+  done_.wait(lock, [&] { return active_ == 0; });
 }
 
 }  // namespace qcl

@@ -7,6 +7,8 @@
 // each way.  Here the threads of a CopyTeam share that work.
 #pragma once
 #include <atomic>
+#include <condition_variable>
+#include <mutex>
 #include <thread>
 #include <vector>
 
@@ -23,6 +25,8 @@ struct CopyPiece {
 
 // Threads that copy lists of pieces together with the caller.  Lives for one
 // call; without threads (none could be started) the caller copies alone.
+// Between lists a thread sleeps after a short spin (other processes of the host
+// have a use for its core), and one that wakes late is not waited for.
 class CopyTeam {
  public:
   explicit CopyTeam(int threads);
@@ -39,10 +43,14 @@ class CopyTeam {
   std::vector<std::thread> threads_;
   const std::vector<CopyPiece>* pieces_ = nullptr;
   std::vector<Unit> units_;
-  std::atomic<unsigned> round_{0};
-  std::atomic<size_t> next_{0};
-  std::atomic<int> busy_{0};
+  std::mutex m_;
+  std::condition_variable start_, done_;
+  // written under m_; atomic for the spins
+  std::atomic<unsigned> round_{0};  // of the current list
+  std::atomic<int> active_{0};      // threads that take part in it
   std::atomic<bool> stop_{false};
+  bool open_ = false;               // the list may still be joined
+  std::atomic<size_t> next_{0};
 };
 
 // Host threads worth using for `bytes` (0: leave the copy to the driver).
