@@ -22,7 +22,6 @@
 #include <algorithm>
 #include <chrono>
 #include <map>
-#include <mutex>
 #include <vector>
 
 #include "kernels.cuh"
@@ -53,7 +52,7 @@ struct Mech {
   int* status = nullptr;
   void* i8_work = nullptr;  // the context's work area of the integer tensor path
   size_t i8_bytes = 0;
-  // the stream its candidate is built on (-1: the context's own) with its own
+  // the branch its candidate is built on (-1: the main one) with its own
   // contraction scratch and per-column Hilbert sums
   int branch = -1;
   void* work = nullptr;
@@ -122,7 +121,6 @@ struct ScbaCtx {
   size_t nfield, fbytes;  // elements per field, bytes per field at the active precision
   size_t fcap = 0;        // allocated bytes per field (complex128 size in refinement contexts)
   cudaStream_t st = nullptr;
-  int dev = 0;
   // grids and operators
   double *eps = nullptr, *wE = nullptr, *wk = nullptr;
   void *h = nullptr, *Tp = nullptr, *Tm = nullptr;
@@ -157,13 +155,14 @@ struct ScbaCtx {
   cudaGraph_t gtpl[2] = {nullptr, nullptr};  // the captured iterations (child graphs of a batched sweep)
   cudaStream_t st2 = nullptr;  // side stream of an iteration (forked from st, joined back)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  // branches of the candidate construction (mechanisms, embedding), forked
-  // from st and joined back; br_area holds the branches' scratch
+  // branches of the candidate construction: their scratch, and the streams and
+  // events of iterations that are not captured (made when first used)
+  void* br_area = nullptr;
   cudaStream_t br_st[kBranches] = {};
   cudaEvent_t br_done[kBranches] = {}, br_fork = nullptr;
-  void* br_area = nullptr;
   size_t br_bytes = 0;
   bool use_graph = false;
+  bool capturing = false;  // the iteration is being captured
   // phase telemetry: device time between CUDA events at the phase boundaries of an
   // iteration (the :phase_begin / :phase_end events of production_telemetry.jl:81-200)
   bool telemetry = false;
@@ -189,44 +188,32 @@ struct ScbaCtx {
   double green_eta = 0;
 };
 
-// Streams of closed contexts, kept for the next one on the same device (a
-// stream costs more to create than a small iteration takes to run).  At most
-// kIdleStreams are kept; they are idle and carry no capture.
-constexpr int kIdleStreams = 16;
-static std::mutex g_streams_mutex;
-static std::vector<std::pair<int, cudaStream_t>> g_streams;
+// Branches beside the context's stream, forked from one point of it.  In a
+// captured iteration they are sets of graph nodes that the next launch depends
+// on, so a context that runs its graph needs no streams for them (in a fresh
+// process three more streams take 12 ms to create, in a warm one 0.15 ms).
+// Otherwise each branch has a stream of the context.
+class Branches {
+ public:
+  // Forks here (nothing to do without `on`: every branch is the main stream).
+  int fork(ScbaCtx* c, bool on);
+  bool on() const { return on_; }
+  // The stream for the launches of branch b until the next call (b < 0: the main one).
+  int enter(int b, cudaStream_t* st);
+  // The main stream goes on, after branch b.
+  int join(int b);
 
-static cudaError_t take_stream(cudaStream_t* st) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  {
-    std::lock_guard<std::mutex> lock(g_streams_mutex);
-    for (size_t i = 0; i < g_streams.size(); ++i)
-      if (g_streams[i].first == dev) {
-        *st = g_streams[i].second;
-        g_streams.erase(g_streams.begin() + i);
-        return cudaSuccess;
-      }
-  }
-  return cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
-}
-
-// Gives a stream of the context on device `dev` back.
-static void give_stream(int dev, cudaStream_t st) {
-  if (!st) return;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
-      cudaStreamQuery(st) == cudaSuccess) {
-    std::lock_guard<std::mutex> lock(g_streams_mutex);
-    if (g_streams.size() < kIdleStreams) {
-      g_streams.push_back({dev, st});
-      return;
-    }
-  }
-  cudaGetLastError();
-  cudaStreamDestroy(st);
-}
+ private:
+  using Nodes = std::vector<cudaGraphNode_t>;
+  int nodes(Nodes* t);
+  int set_nodes(const Nodes& t);
+  int leave();
+  ScbaCtx* c_ = nullptr;
+  bool on_ = false, captured_ = false;
+  bool used_[kBranches] = {};
+  int at_ = -1;                 // captured: the branch whose nodes the stream has (-1: main)
+  Nodes tail_[kBranches + 1];   // captured: of the branches and the main one
+};
 
 static void* field_of(const std::vector<void*>& v, int f, int c) { return v[3 * f + c]; }
 int scba_step_launch(ScbaCtx* c, cudaGraph_t* child);
@@ -356,11 +343,11 @@ void scba_destroy(ScbaCtx* c) {
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   for (int i = 0; i < kBranches; ++i) {
     if (c->br_done[i]) cudaEventDestroy(c->br_done[i]);
-    give_stream(c->dev, c->br_st[i]);
+    if (c->br_st[i]) cudaStreamDestroy(c->br_st[i]);
   }
   if (c->br_fork) cudaEventDestroy(c->br_fork);
-  give_stream(c->dev, c->st2);
-  give_stream(c->dev, c->st);
+  if (c->st2) cudaStreamDestroy(c->st2);
+  if (c->st) cudaStreamDestroy(c->st);
   delete c;
 }
 
@@ -492,12 +479,12 @@ static void i8_area(ScbaCtx* c) {
   }
 }
 
-// Scratch and streams for building the mechanisms' candidates side by side.
+// Scratch for building the mechanisms' candidates side by side.
 // They are independent given G, and at small sizes each is a chain of kernels
 // that leaves most of the GPU idle; at large ones the branches only fill the
 // ends of each other's launches.  The LO mechanism (whose shifted fields have
 // one buffer), maps on the integer path (one work area) and the largest of the
-// rest stay on the context's stream.  Optional, like i8_area: at most 64 MB
+// rest stay on the main branch.  Optional, like i8_area: at most 64 MB
 // (or half a field) and what the budget leaves over; without it the
 // mechanisms run one after another.
 static void branch_area(ScbaCtx* c) {
@@ -534,16 +521,10 @@ static void branch_area(ScbaCtx* c) {
     c->mech[i].branch = next++ % (kBranches - 1);
     total += need[i];
   }
-  bool ok = total == 0 || cudaMalloc(&c->br_area, total) == cudaSuccess;
-  ok = ok && cudaEventCreateWithFlags(&c->br_fork, cudaEventDisableTiming) == cudaSuccess;
-  for (int i = 0; i < kBranches && ok; ++i)
-    ok = take_stream(&c->br_st[i]) == cudaSuccess &&
-         cudaEventCreateWithFlags(&c->br_done[i], cudaEventDisableTiming) == cudaSuccess;
-  if (!ok) {  // one after another
+  if (total > 0 && cudaMalloc(&c->br_area, total) != cudaSuccess) {  // one after another
     cudaGetLastError();
+    c->br_area = nullptr;
     for (auto& m : c->mech) m.branch = -1;
-    if (c->br_fork) cudaEventDestroy(c->br_fork);
-    c->br_fork = nullptr;
     return;
   }
   c->br_bytes = total;
@@ -672,11 +653,10 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
                             "low-rank operator does not preserve adjoints and positivity"),
              QCL_ARG));
   {
-    cudaError_t e = cudaGetDevice(&c->dev);
-    if (e == cudaSuccess) e = take_stream(&c->st);
+    cudaError_t e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaStreamCreate"));
     // the residual suite's G-only part runs beside the candidate construction
-    e = take_stream(&c->st2);
+    e = cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaStreamCreate"));
@@ -803,32 +783,101 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
 // ---------------------------------------------------------------------------
 // Candidate maps (stream-ordered launches; no host synchronisation)
 // ---------------------------------------------------------------------------
-// Whether candidates are built on several streams (phase telemetry times the
-// phases one after another).
-static bool branching(const ScbaCtx* c) { return c->br_fork && !c->telemetry; }
+int Branches::nodes(Nodes* t) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t n = 0;
+  QCL_CUDA_CHECK(cudaStreamGetCaptureInfo_v2(c_->st, &cs, nullptr, nullptr, &deps, &n));
+  t->assign(deps, deps + n);
+  return QCL_OK;
+}
 
+int Branches::set_nodes(const Nodes& t) {
+  QCL_CUDA_CHECK(cudaStreamUpdateCaptureDependencies(c_->st, const_cast<cudaGraphNode_t*>(t.data()), t.size(),
+                                                     cudaStreamSetCaptureDependencies));
+  return QCL_OK;
+}
+
+int Branches::leave() { return nodes(&tail_[at_ < 0 ? kBranches : at_]); }
+
+int Branches::fork(ScbaCtx* c, bool on) {
+  c_ = c;
+  on_ = on;
+  captured_ = c->capturing;
+  if (!on_) return QCL_OK;
+  if (captured_) {
+    if (int s = leave()) return s;
+    for (int b = 0; b < kBranches; ++b) tail_[b] = tail_[kBranches];
+    return QCL_OK;
+  }
+  if (!c->br_fork) {
+    cudaError_t e = cudaSuccess;
+    for (int b = 0; b < kBranches && e == cudaSuccess; ++b) {
+      if (!c->br_st[b]) e = cudaStreamCreateWithFlags(&c->br_st[b], cudaStreamNonBlocking);
+      if (e == cudaSuccess && !c->br_done[b]) e = cudaEventCreateWithFlags(&c->br_done[b], cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->br_fork, cudaEventDisableTiming);
+    if (e != cudaSuccess) {  // one after another
+      cudaGetLastError();
+      on_ = false;
+      return QCL_OK;
+    }
+  }
+  QCL_CUDA_CHECK(cudaEventRecord(c->br_fork, c->st));
+  return QCL_OK;
+}
+
+int Branches::enter(int b, cudaStream_t* st) {
+  *st = c_->st;
+  if (!on_) return QCL_OK;
+  if (captured_) {
+    if (b >= 0) used_[b] = true;
+    if (b == at_) return QCL_OK;
+    if (int s = leave()) return s;
+    at_ = b;
+    return set_nodes(tail_[b < 0 ? kBranches : b]);
+  }
+  if (b < 0) return QCL_OK;
+  *st = c_->br_st[b];
+  if (!used_[b]) QCL_CUDA_CHECK(cudaStreamWaitEvent(*st, c_->br_fork, 0));
+  used_[b] = true;
+  return QCL_OK;
+}
+
+int Branches::join(int b) {
+  if (!on_) return QCL_OK;
+  cudaStream_t st;
+  if (int s = enter(-1, &st)) return s;
+  if (!used_[b]) return QCL_OK;
+  if (captured_) {
+    if (int s = leave()) return s;
+    Nodes& main = tail_[kBranches];
+    for (cudaGraphNode_t n : tail_[b])
+      if (std::find(main.begin(), main.end(), n) == main.end()) main.push_back(n);
+    return set_nodes(main);
+  }
+  QCL_CUDA_CHECK(cudaEventRecord(c_->br_done[b], c_->br_st[b]));
+  QCL_CUDA_CHECK(cudaStreamWaitEvent(c_->st, c_->br_done[b], 0));
+  return QCL_OK;
+}
+
+// (on the branches of `br`, forked before; joins them)
 static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, const void* GG, std::vector<void*>& dst,
-                                 bool verify) {
+                                 bool verify, Branches& br) {
   int s;
   const int p = c->precision;
   // contractions run at storage precision (mixed: FP32 with FP64 k-sums)
   const int cp = p == QCL_MIXED ? QCL_C64 : p;
   const long long ncols = (long long)c->Nk * c->N * c->N;
-  const bool fork = branching(c);
-  unsigned used = 0;  // branches taken
-  if (fork) QCL_CUDA_CHECK(cudaEventRecord(c->br_fork, c->st));
   for (int i = 0; i < c->M; ++i) {
     const Mech& m = c->mech[i];
     const KernelOpDev op = m.view();
-    const bool side = fork && m.branch >= 0;
-    const cudaStream_t st = side ? c->br_st[m.branch] : c->st;
+    const bool side = br.on() && m.branch >= 0;
+    cudaStream_t st;
+    if ((s = br.enter(side ? m.branch : -1, &st))) return s;
     void* work = side ? m.work : c->cwork;
     HilbertTables hil = c->hil;  // shares the tables; the per-column sums are the branch's own
-    if (side) {
-      hil.partial = m.hpartial;
-      if (!(used >> m.branch & 1u)) QCL_CUDA_CHECK(cudaStreamWaitEvent(st, c->br_fork, 0));
-      used |= 1u << m.branch;
-    }
+    if (side) hil.partial = m.hpartial;
     void* SL = field_of(dst, i, 1);
     void* SG = field_of(dst, i, 2);
     const void* X[2] = {GL, GG};
@@ -841,11 +890,9 @@ static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, con
       // The candidate total's field is free until the candidates exist: it
       // holds the second combined field.
       const double n = c->N_LO;
-      if ((s = launch_shift_pair(cp, c->NE, ncols, c->shift[2].view(), c->shift[3].view(), n + 1, n, GL, c->tmp,
-                                 c->st)))
+      if ((s = launch_shift_pair(cp, c->NE, ncols, c->shift[2].view(), c->shift[3].view(), n + 1, n, GL, c->tmp, st)))
         return s;
-      if ((s = launch_shift_pair(cp, c->NE, ncols, c->shift[3].view(), c->shift[2].view(), n + 1, n, GG, c->candSL,
-                                 c->st)))
+      if ((s = launch_shift_pair(cp, c->NE, ncols, c->shift[3].view(), c->shift[2].view(), n + 1, n, GG, c->candSL, st)))
         return s;
       X[0] = c->tmp;
       X[1] = c->candSL;
@@ -871,11 +918,8 @@ static int scattering_candidates(ScbaCtx* c, const void* GR, const void* GL, con
     if ((s = launch_scattering_model(cp, c->NE, c->Nk, c->N, c->wk, c->wk_sum, c->diagonal, c->averaged, fam, st)))
       return s;
   }
-  for (int q = 0; q < kBranches; ++q)
-    if (used >> q & 1u) {
-      QCL_CUDA_CHECK(cudaEventRecord(c->br_done[q], c->br_st[q]));
-      QCL_CUDA_CHECK(cudaStreamWaitEvent(c->st, c->br_done[q], 0));
-    }
+  for (int b = 0; b < kBranches - 1; ++b)
+    if ((s = br.join(b))) return s;
   return QCL_OK;
 }
 
@@ -953,19 +997,21 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
     return launch_observables(sp, c->NE, c->Nk, c->N, c->wE, c->wk, field_of(state, c->M, 2), field_of(state, c->M, 1),
                               c->GL, c->GG, c->gs, c->target, c->obspartial, c->scal + SC_OBS, st);
   };
-  const bool fork = branching(c);  // the embedding has a branch of its own, observables follow the residuals
+  // The embedding has a branch of its own, and observables follow the residuals
+  // (phase telemetry times the phases one after another).  The first iteration
+  // of a context that will run its graph does without.
+  Branches br;
+  if ((s = br.fork(c, !c->telemetry && (c->capturing || !c->use_graph)))) return s;
   const int eb = kBranches - 1;
-  if (fork) {
+  if (br.on()) {
     if ((s = observables(c->st2))) return s;
-    QCL_CUDA_CHECK(cudaStreamWaitEvent(c->br_st[eb], c->ev_fork, 0));
-    if ((s = embedding_candidates(c, cand, c->br_st[eb]))) return s;
-    QCL_CUDA_CHECK(cudaEventRecord(c->br_done[eb], c->br_st[eb]));
+    cudaStream_t st;
+    if ((s = br.enter(eb, &st)) || (s = embedding_candidates(c, cand, st))) return s;
   }
   QCL_CUDA_CHECK(cudaEventRecord(c->ev_join, c->st2));
-  if ((s = scattering_candidates(c, c->GR, c->GL, c->GG, cand, c->verify != 0))) return s;
+  if ((s = scattering_candidates(c, c->GR, c->GL, c->GG, cand, c->verify != 0, br))) return s;
   if ((s = phase_mark(c, 2))) return s;
-  if (fork) QCL_CUDA_CHECK(cudaStreamWaitEvent(c->st, c->br_done[eb], 0));
-  else if ((s = embedding_candidates(c, cand, c->st))) return s;
+  if ((s = br.on() ? br.join(eb) : embedding_candidates(c, cand, c->st))) return s;
   if ((s = phase_mark(c, 3))) return s;
   const int F = c->M + 2;
   const void* olds[kMaxMixFields];
@@ -992,7 +1038,7 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
     if ((s = phase_mark(c, 4))) return s;
     if ((s = residuals())) return s;
     if ((s = phase_mark(c, 5))) return s;
-    if (!fork && (s = observables(c->st))) return s;
+    if (!br.on() && (s = observables(c->st))) return s;
     if ((s = phase_mark(c, 6))) return s;
   } else {
     const void* src[1][8];
@@ -1007,7 +1053,7 @@ static int iteration_body(ScbaCtx* c, std::vector<void*>& state, std::vector<voi
                                     c->scal + SC_EMB + 2 * k, c->st)))
         return s;
     if ((s = phase_mark(c, 5))) return s;
-    if (!fork && (s = observables(c->st))) return s;
+    if (!br.on() && (s = observables(c->st))) return s;
     if ((s = phase_mark(c, 6))) return s;
     // Anderson mixing with the causality guard (production_mixing.jl:224-317)
     const int nf = 3 * F;
@@ -1104,7 +1150,9 @@ int scba_seed(ScbaCtx* c, double* mu_out) {
   QCL_CUDA_CHECK(cudaMemcpyAsync(f_d, f.data(), c->NE * sizeof(double), cudaMemcpyHostToDevice, c->st));
   if ((s = launch_seed_green(sp, c->NE, c->Nk, c->N, c->GR, f_d, c->GL, c->GG, c->st))) return s;
   // initial candidates (no roundoff verification), straight into the state
-  if ((s = scattering_candidates(c, c->GR, c->GL, c->GG, c->state, false))) return s;
+  Branches br;
+  if ((s = br.fork(c, false))) return s;
+  if ((s = scattering_candidates(c, c->GR, c->GL, c->GG, c->state, false, br))) return s;
   if ((s = embedding_candidates(c, c->state, c->st))) return s;
   QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));
   QCL_CUDA_CHECK(cudaMemcpy(hst, c->status, sizeof(hst), cudaMemcpyDeviceToHost));
@@ -1160,7 +1208,9 @@ static int run_body(ScbaCtx* c, cudaGraph_t* child) {
   if (!c->graph[c->parity]) {
     cudaGraph_t g;
     QCL_CUDA_CHECK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+    c->capturing = true;
     int s = iteration_body(c, st, cd);
+    c->capturing = false;
     cudaError_t e = cudaStreamEndCapture(c->st, &g);
     if (s) {
       if (e == cudaSuccess) cudaGraphDestroy(g);
@@ -1892,7 +1942,9 @@ int scba_tangent_step(ScbaCtx* c, double* out) {
                               c->gs, c->target, c->obspartial, jout + 2 + N, c->st)))
     return s;
   // Phi_Sigma v: the linear candidate maps of the tangent Green's functions
-  if ((s = scattering_candidates(c, X, dL, dG, c->tw, false))) return s;
+  Branches br;
+  if ((s = br.fork(c, !c->telemetry))) return s;
+  if ((s = scattering_candidates(c, X, dL, dG, c->tw, false, br))) return s;
   if ((s = embedding_candidates(c, c->tw, c->st, X, dL, dG))) return s;
   // w <- Phi_Sigma v + s, then the damped update into w with the residual norms
   const void* olds[kMaxMixFields];
