@@ -1070,9 +1070,9 @@ template <typename RS, int NP, int BPC> static int launch_residual_t(const Resid
 // r_K alone has no tests and is bound by its loads, where longer runs of
 // energies help: N_b = 32, 1024 x 32 blocks, mixed, 2 per CTA instead of 1: 1.52
 // -> 0.98 ms; N_b = 12 and 16, 4 instead of 2: 6400 blocks, c128, 37 -> 30 us,
-// 3064 blocks, mixed, 30 -> 24 us, but 22 us more at 32768 blocks, which fill
-// the SMs with the smaller CTAs.
-constexpr long long kFewRkBlocks = 8192;
+// 3064 blocks, mixed, 30 -> 24 us, and whole iterations at 3064 ... 32768 blocks
+// take the same or less at every count (N_b = 16, c128: 484.9 -> 482.4 us at
+// 3064, 1056 -> 1043 at 8192, 1987 -> 1960 at 16384, 3786 -> 3732 at 32768).
 template <typename RS, int NP, int BPC> static int launch_residual_rk_t(const ResidualArgs<RS>& a, cudaStream_t st) {
   constexpr size_t smem = BPC * (3 * tile_stride<double, NP, BPC>() * sizeof(Cx<double>) + 4 * sizeof(double));
   static bool configured = false;
@@ -1098,8 +1098,7 @@ template <typename RS, int NP, int BPC> static int launch_residual_rows_t(const 
   }
   if (a.part == RES_PART_RK) {
     if (NP == 32) return launch_residual_rk_t<RS, NP, 2>(a, st);
-    if (NP == 16 && (long long)a.NE * a.Nk <= kFewRkBlocks) return launch_residual_rk_t<RS, NP, 4>(a, st);
-    return launch_residual_rk_t<RS, NP, BPC>(a, st);
+    return launch_residual_rk_t<RS, NP, NP == 16 ? 4 : BPC>(a, st);
   }
   const dim3 grid((a.NE + BPC - 1) / BPC, a.Nk);
   residual_rows_kernel<RS, NP, BPC><<<grid, BPC * TT, smem, st>>>(a);
