@@ -7,7 +7,7 @@
 // numerics/optimized/residuals.jl:493-503).
 #include <math.h>
 
-#include "kernels.cuh"
+#include "residual.cuh"
 
 namespace qcl {
 
@@ -767,6 +767,79 @@ int launch_axpby(int precision, size_t n, double a, const void* x, double b, con
     axpby_kernel<float><<<grid_for(n, 256), 256, 0, st>>>(n, a, (const Cx<float>*)x, b, (const Cx<float>*)y,
                                                           (Cx<float>*)out);
   QCL_LAUNCH_CHECK("axpby");
+  return QCL_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Residual suite: the blocks' outputs.
+// ---------------------------------------------------------------------------
+// Fixed-order reduction of the per-block outputs:
+// out = (r_D, r_A, r_K, r_PSD, r_caus).
+__global__ void residual_reduce_kernel(long long blocks, const double* __restrict__ bo, double* partial) {
+  double mx[3] = {0, 0, 0}, sm[4] = {0, 0, 0, 0};
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < blocks;
+       i += (long long)gridDim.x * blockDim.x) {
+    const double* o = bo + kResidualBlockDoubles * i;
+    mx[0] = fmax(mx[0], o[0]) + (isnan(o[0]) ? INFINITY : 0.0);
+    sm[0] += o[1];
+    sm[1] += o[2];
+    sm[2] += o[3];
+    sm[3] += o[4];
+    mx[1] = fmax(mx[1], o[5]) + (isnan(o[5]) ? INFINITY : 0.0);
+    mx[2] = fmax(mx[2], o[6]) + (isnan(o[6]) ? INFINITY : 0.0);
+  }
+  __shared__ double red[7][8];
+  double v[7] = {mx[0], sm[0], sm[1], sm[2], sm[3], mx[1], mx[2]};
+#pragma unroll
+  for (int k = 0; k < 7; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double q = __shfl_xor_sync(0xffffffffu, v[k], o);
+      v[k] = (k == 0 || k >= 5) ? fmax(v[k], q) : v[k] + q;
+    }
+  if ((threadIdx.x & 31) == 0)
+    for (int k = 0; k < 7; ++k) red[k][threadIdx.x >> 5] = v[k];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 7; ++k) {
+      double s = red[k][0];
+      for (int w = 1; w < 8; ++w) s = (k == 0 || k >= 5) ? fmax(s, red[k][w]) : s + red[k][w];
+      partial[7 * blockIdx.x + k] = s;
+    }
+  }
+}
+
+// One warp per quantity, fixed-order lane sums then a fixed shuffle tree.
+__global__ void residual_final_kernel(int ncta, const double* partial, double* out) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ double v[7];
+  const bool is_max = k == 0 || k >= 5;
+  double a = 0;
+  for (int c = lane; c < ncta; c += 32) {
+    const double q = partial[7 * c + k];
+    a = is_max ? fmax(a, q) + (isnan(q) ? INFINITY : 0.0) : a + q;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double q = __shfl_xor_sync(0xffffffffu, a, o);
+    a = is_max ? fmax(a, q) : a + q;
+  }
+  if (lane == 0) v[k] = a;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  out[0] = v[0];
+  out[1] = (isfinite(v[1]) && isfinite(v[2])) ? sqrt(v[1]) / (sqrt(v[2]) + 1e-14) : INFINITY;
+  out[2] = (isfinite(v[3]) && isfinite(v[4])) ? sqrt(v[3]) / (sqrt(v[4]) + 1e-14) : INFINITY;
+  out[3] = v[5];
+  out[4] = v[6];
+}
+
+// Fixed-order reduction of the per-block outputs in `work` into out5.
+int launch_residual_reduce(int NE, int Nk, double* work, double* out5, cudaStream_t st) {
+  double* partial = work + kResidualBlockDoubles * (size_t)NE * Nk;
+  residual_reduce_kernel<<<RES_CTAS, 256, 0, st>>>((long long)NE * Nk, work, partial);
+  residual_final_kernel<<<1, 7 * 32, 0, st>>>(RES_CTAS, partial, out5);
+  QCL_LAUNCH_CHECK("residual_reduce");
   return QCL_OK;
 }
 

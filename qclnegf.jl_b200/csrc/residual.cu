@@ -24,340 +24,9 @@
 // reduced in a fixed order.
 #include <mutex>
 
-#include "blockmat.cuh"
+#include "residual.cuh"
 
 namespace qcl {
-
-// Per-block outputs: r_D, r_A num/den, r_K num/den, r_PSD, r_caus, and the
-// block's positivity-witness ratio and matrix kind.
-constexpr int kResidualBlockDoubles = 9;
-
-template <typename RS> struct ResidualArgs {
-  int NE, Nk, N;
-  const double* eps;
-  const Cx<double>* h;
-  const Cx<RS>* GR;
-  const Cx<RS>* GL;
-  const Cx<RS>* GG;
-  const Cx<RS>* SR;   // totals
-  const Cx<RS>* SL;
-  const Cx<RS>* SG;
-  const Cx<RS>* SLc;  // candidate total lesser
-  double* block_out;  // kResidualBlockDoubles per block
-  int part;           // RES_PART_ALL, RES_PART_MAIN (all but r_K) or RES_PART_RK (r_K only)
-};
-
-struct JacobiRot {
-  double c, s, pr, pi;  // rotation cosine/sine and the phase e^{i phi}
-  int p, q;
-};
-
-template <int NP> struct ResScratch {
-  JacobiRot rot[NP / 2];
-  double red[8];
-  double vals[NP];
-  double d[NP], e2[NP];  // tridiagonal form
-  Cx<double> u[NP], w[NP];
-};
-
-// Visits the (i, j), i, j < N, of an NP x NP tile: team thread tt takes the
-// padded indices tt, tt + TT, ... (compile-time trip count and index split,
-// no runtime division).
-template <int NP, int TT, typename F> __device__ __forceinline__ void tile_for(int N, int tt, F&& f) {
-#pragma unroll 1
-  for (int q = 0; q < (NP * NP + TT - 1) / TT; ++q) {
-    const int idx = tt + q * TT;
-    if (idx < NP * NP) {
-      const int i = idx % NP, j = idx / NP;
-      if (i < N && j < N) f(i, j);
-    }
-  }
-}
-
-// Team sum of two doubles (fixed order).
-template <int TT>
-__device__ __forceinline__ void team_sum2(double& a, double& b, int tt, double* scratch, int team) {
-  a = team_sum<TT>(a, tt, scratch, team);
-  b = team_sum<TT>(b, tt, scratch + 2, team);
-}
-
-// Eigenvalues of the Hermitian NxN matrix H (swizzled NP x NP shared tile);
-// H is destroyed, S.vals[0..N-1] receives the eigenvalues (unsorted).
-// Round-robin parallel Jacobi: in each of the n2-1 rounds of a sweep the
-// rotations of n2/2 disjoint index pairs are computed from the same matrix
-// and applied together (all column updates, then all row updates).  The
-// rotated pair is set to exactly zero and its diagonal to exactly real, so
-// rounding cannot leave a non-Hermitian remainder; a pair whose coupling is
-// negligible against its diagonal (1e-18 relative) is skipped, and a sweep
-// that rotates nothing ends the iteration.
-template <int NP, int TT>
-__device__ void team_eigvals(Cx<double>* H, int N, int tt, ResScratch<NP>& S, int team) {
-  const int n2 = N + (N & 1);
-  for (int sweep = 0; sweep < 40; ++sweep) {
-    double rotated = 0;
-    for (int r = 0; r < n2 - 1; ++r) {
-      if (tt < n2 / 2) {
-        const int i = tt;
-        const int a = (r + i) % (n2 - 1);
-        const int b = (i == 0) ? n2 - 1 : (r - i + n2 - 1) % (n2 - 1);
-        JacobiRot rt;
-        rt.p = a < b ? a : b;
-        rt.q = a < b ? b : a;
-        rt.c = 1;
-        rt.s = 0;
-        rt.pr = 1;
-        rt.pi = 0;
-        if (rt.q < N) {
-          const Cx<double> apq = H[sw<NP>(rt.p, rt.q)];
-          const double mag = hypot(apq.x, apq.y);
-          const double app = H[sw<NP>(rt.p, rt.p)].x, aqq = H[sw<NP>(rt.q, rt.q)].x;
-          if (mag > 1e-18 * (fabs(app) + fabs(aqq)) && isfinite(mag)) {
-            const double theta = (aqq - app) / (2 * mag);
-            double t;
-            if (fabs(theta) > 1e150) t = 0.5 / theta;
-            else t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-            rt.c = 1.0 / sqrt(t * t + 1.0);
-            rt.s = t * rt.c;
-            rt.pr = apq.x / mag;
-            rt.pi = apq.y / mag;
-            rotated = 1;
-          }
-        } else {
-          rt.q = rt.p;  // phantom partner: identity
-        }
-        S.rot[i] = rt;
-      }
-      team_sync<TT>(team);
-      // columns: H <- H J
-      for (int idx = tt; idx < N * (n2 / 2); idx += TT) {
-        const int k = idx % N;
-        const JacobiRot rt = S.rot[idx / N];
-        if (rt.p == rt.q || rt.s == 0) continue;
-        const Cx<double> hp = H[sw<NP>(k, rt.p)], hq = H[sw<NP>(k, rt.q)];
-        const Cx<double> eq = cx<double>(rt.pr, -rt.pi) * hq;  // e^{-i phi} H[k][q]
-        H[sw<NP>(k, rt.p)] = cx<double>(rt.c * hp.x - rt.s * eq.x, rt.c * hp.y - rt.s * eq.y);
-        H[sw<NP>(k, rt.q)] = cx<double>(rt.s * hp.x + rt.c * eq.x, rt.s * hp.y + rt.c * eq.y);
-      }
-      team_sync<TT>(team);
-      // rows: H <- J^H H; the rotated pair becomes exactly diagonal
-      for (int idx = tt; idx < N * (n2 / 2); idx += TT) {
-        const int k = idx % N;
-        const JacobiRot rt = S.rot[idx / N];
-        if (rt.p == rt.q || rt.s == 0) continue;
-        const Cx<double> xp = H[sw<NP>(rt.p, k)], xq = H[sw<NP>(rt.q, k)];
-        const Cx<double> eq = cx<double>(rt.pr, rt.pi) * xq;  // e^{i phi} H[q][k]
-        Cx<double> np_ = cx<double>(rt.c * xp.x - rt.s * eq.x, rt.c * xp.y - rt.s * eq.y);
-        Cx<double> nq_ = cx<double>(rt.s * xp.x + rt.c * eq.x, rt.s * xp.y + rt.c * eq.y);
-        if (k == rt.p) {
-          np_.y = 0;             // H[p][p] real
-          nq_ = cx<double>(0, 0);  // H[q][p] = 0
-        } else if (k == rt.q) {
-          np_ = cx<double>(0, 0);  // H[p][q] = 0
-          nq_.y = 0;             // H[q][q] real
-        }
-        H[sw<NP>(rt.p, k)] = np_;
-        H[sw<NP>(rt.q, k)] = nq_;
-      }
-      team_sync<TT>(team);
-    }
-    rotated = team_max<TT>(rotated, tt, S.red, team);
-    if (rotated == 0) break;
-  }
-  for (int i = tt; i < N; i += TT) S.vals[i] = H[sw<NP>(i, i)].x;
-  team_sync<TT>(team);
-}
-
-// Writes the Hermitian part of f*X into H; returns false if X has non-finite
-// entries (team-uniform).
-template <int NP, int TT>
-__device__ bool hermitian_part(const Cx<double>* X, Cx<double> f, Cx<double>* H, int N, int tt, ResScratch<NP>& S,
-                               int team) {
-  double bad = 0;
-  tile_for<NP, TT>(N, tt, [&](int i, int j) {
-    const Cx<double> v = f * X[sw<NP>(i, j)], w = f * X[sw<NP>(j, i)];
-    if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(w.x) || !isfinite(w.y)) bad = 1;
-    H[sw<NP>(i, j)] = cx<double>(0.5 * (v.x + w.x), 0.5 * (v.y - w.y));
-  });
-  bad = team_max<TT>(bad, tt, S.red, team);
-  team_sync<TT>(team);  // H complete for every thread of the team
-  return bad == 0;
-}
-
-// ---- extreme eigenvalues through a tridiagonal form ---------------------------
-// Householder reduction of the Hermitian N x N tile H (destroyed) to a real
-// symmetric tridiagonal matrix with the same eigenvalues: S.d[0..N) its
-// diagonal, S.e2[0..N-1) its squared off-diagonal.  Step k applies the
-// Hermitian unitary reflector P = I - c u u^H that maps column k below the
-// diagonal onto its first entry, as the rank-2 update of the trailing block
-//   A <- P A P = A - u w^H - w u^H,  p = c A u,  w = p - (c/2)(u^H p) u
-// (Golub & Van Loan, Matrix Computations, sec. 8.3.1).  One team thread per
-// row of the trailing block; backward stable like LAPACK's zhetrd.
-template <int NP, int TT>
-__device__ void team_tridiagonalize(Cx<double>* H, int N, int tt, ResScratch<NP>& S, int team) {
-  for (int k = 0; k + 2 < N; ++k) {
-    const int m = N - k - 1;  // entries below the diagonal in column k
-    const Cx<double> xi = tt < m ? H[sw<NP>(k + 1 + tt, k)] : cx<double>(0, 0);
-    const double a2 = team_sum<TT>(xi.x * xi.x + xi.y * xi.y, tt, S.red, team);
-    const Cx<double> x0 = H[sw<NP>(k + 1, k)];
-    if (tt == 0) {
-      S.d[k] = H[sw<NP>(k, k)].x;
-      S.e2[k] = a2;
-    }
-    if (!(a2 > 0)) {  // team-uniform: column already reduced
-      team_sync<TT>(team);
-      continue;
-    }
-    const double alpha = sqrt(a2), ax0 = hypot(x0.x, x0.y);
-    const Cx<double> ph = ax0 > 0 ? cx<double>(x0.x / ax0, x0.y / ax0) : cx<double>(1, 0);
-    const double c = 1.0 / (alpha * (alpha + ax0));
-    const Cx<double> ui = tt == 0 ? cx<double>(x0.x + alpha * ph.x, x0.y + alpha * ph.y) : xi;
-    if (tt < m) S.u[tt] = ui;
-    team_sync<TT>(team);
-    Cx<double> pv = cx<double>(0, 0);
-    if (tt < m) {
-      for (int j = 0; j < m; ++j) cfma(pv, H[sw<NP>(k + 1 + tt, k + 1 + j)], S.u[j]);
-      pv = c * pv;
-    }
-    const double kk = 0.5 * c * team_sum<TT>(tt < m ? ui.x * pv.x + ui.y * pv.y : 0.0, tt, S.red, team);
-    if (tt < m) S.w[tt] = cx<double>(pv.x - kk * ui.x, pv.y - kk * ui.y);
-    team_sync<TT>(team);
-    for (int idx = tt; idx < m * m; idx += TT) {
-      const int i = idx % m, j = idx / m;
-      Cx<double>& a = H[sw<NP>(k + 1 + i, k + 1 + j)];
-      const Cx<double> t = S.u[i] * conj(S.w[j]) + S.w[i] * conj(S.u[j]);
-      a = cx<double>(a.x - t.x, a.y - t.y);
-    }
-    team_sync<TT>(team);
-  }
-  if (tt == 0) {
-    if (N >= 2) {
-      const Cx<double> t = H[sw<NP>(N - 1, N - 2)];
-      S.d[N - 2] = H[sw<NP>(N - 2, N - 2)].x;
-      S.e2[N - 2] = t.x * t.x + t.y * t.y;
-    }
-    S.d[N - 1] = H[sw<NP>(N - 1, N - 1)].x;
-  }
-  team_sync<TT>(team);
-}
-
-// Number of eigenvalues of the tridiagonal (d, e2) below sigma (Sturm
-// sequence / LDL^T inertia, pivots clamped away from zero as in LAPACK dstebz).
-__device__ __forceinline__ int sturm_count(const double* d, const double* e2, int N, double sigma, double pivmin) {
-  double q = d[0] - sigma;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int c = q < 0;
-  for (int i = 1; i < N; ++i) {
-    q = (d[i] - sigma) - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    c += q < 0;
-  }
-  return c;
-}
-
-__device__ __forceinline__ double tri_pivmin(const double* e2, int N) {
-  double emax = 0;
-  for (int i = 0; i + 1 < N; ++i) emax = fmax(emax, e2[i]);
-  return 2.2250738585072014e-308 * fmax(1.0, emax);
-}
-
-// kth smallest eigenvalue (kth = 1..N) of the tridiagonal by multisection of
-// the Gershgorin interval: each warp evaluates the same 32 shifts per round
-// (every lane of the team ends with the same interval, no exchange needed),
-// until the interval is a few ulps wide.
-__device__ double tri_eig(const double* d, const double* e2, int N, int kth) {
-  constexpr double eps = 2.220446049250313e-16;
-  double lo = INFINITY, hi = -INFINITY;
-  for (int i = 0; i < N; ++i) {
-    const double r = (i > 0 ? sqrt(e2[i - 1]) : 0.0) + (i + 1 < N ? sqrt(e2[i]) : 0.0);
-    lo = fmin(lo, d[i] - r);
-    hi = fmax(hi, d[i] + r);
-  }
-  const double pivmin = tri_pivmin(e2, N);
-  const double tnorm = fmax(fabs(lo), fabs(hi));
-  lo -= 2 * eps * tnorm * N + 2 * pivmin;
-  hi += 2 * eps * tnorm * N + 2 * pivmin;
-  const int lane = threadIdx.x & 31;
-  for (int round = 0; round < 64; ++round) {
-    if (hi - lo <= 2 * eps * fmax(fabs(lo), fabs(hi)) + pivmin) break;
-    const double width = hi - lo;
-    const double sig = lo + width * (double)(lane + 1) / 33.0;
-    const unsigned mask = __ballot_sync(0xffffffffu, sturm_count(d, e2, N, sig, pivmin) >= kth);
-    const int f = mask ? __ffs(mask) - 1 : 32;  // first shift with kth eigenvalues below it
-    const double nlo = f > 0 ? lo + width * (double)f / 33.0 : lo;
-    const double nhi = f < 32 ? lo + width * (double)(f + 1) / 33.0 : hi;
-    lo = nlo;
-    hi = nhi;
-  }
-  return 0.5 * (lo + hi);
-}
-
-// True if H + shift I is numerically positive definite: LDL^T without pivoting
-// (trailing lower triangle updated in place) meets only positive pivots.  H is
-// destroyed.  A success certifies lmin(H) > -shift up to the factorization's
-// backward error O(n eps ||H||) -- the same order as the error of the
-// eigenvalues themselves.
-template <int NP, int TT>
-__device__ bool team_posdef(Cx<double>* H, int N, double shift, int tt, int team) {
-  // TT / NP threads per row (rows past the tile's thread count idle): thread
-  // (i, h) updates entries j = k + 1 + h, k + 1 + h + R, ... <= i of row i
-  constexpr int R = TT / NP >= 1 ? TT / NP : 1;
-  const int i = tt % NP, h = tt / NP;
-  for (int k = 0; k < N; ++k) {
-    const double dk = H[sw<NP>(k, k)].x + shift;
-    if (!(dk > 0)) return false;  // team-uniform: every thread read the same pivot
-    const double inv = 1.0 / dk;
-    if (h < R && i > k && i < N) {
-      const Cx<double> a = H[sw<NP>(i, k)];
-      for (int j = k + 1 + h; j <= i; j += R) {
-        const Cx<double> b = H[sw<NP>(j, k)];
-        Cx<double>& hij = H[sw<NP>(i, j)];
-        const Cx<double> t = a * conj(b);
-        hij = cx<double>(hij.x - inv * t.x, hij.y - inv * t.y);
-      }
-    }
-    team_sync<TT>(team);
-  }
-  return true;
-}
-
-// Positivity ratio of the Hermitian part of f X (written to H, destroyed):
-//   max(0, -lmin - 64 n eps max(|l|max, 1)) / |l|max,
-// INFINITY if f X has non-finite entries.  The diagonal bounds |l|max from
-// below, so when H + 64 n eps max(max|H_ii|, 1) I is positive definite (one
-// LDL^T, the common case) the ratio is 0; otherwise H is rebuilt, reduced to
-// tridiagonal form and lmin, lmax are found by multisection.
-template <int NP, int TT>
-__device__ double psd_of(const Cx<double>* X, Cx<double> f, Cx<double>* H, int N, int tt, ResScratch<NP>& S,
-                         int team) {
-  constexpr double eps = 2.220446049250313e-16;
-  if (!hermitian_part<NP, TT>(X, f, H, N, tt, S, team)) return INFINITY;
-  double dmax = 0;
-  for (int i = 0; i < N; ++i) dmax = fmax(dmax, fabs(H[sw<NP>(i, i)].x));
-  team_sync<TT>(team);
-  if (team_posdef<NP, TT>(H, N, 64.0 * N * eps * fmax(dmax, 1.0), tt, team)) return 0.0;
-  team_sync<TT>(team);
-  hermitian_part<NP, TT>(X, f, H, N, tt, S, team);
-  team_tridiagonalize<NP, TT>(H, N, tt, S, team);
-  for (int i = 0; i < N; ++i)
-    if (!isfinite(S.d[i]) || (i + 1 < N && !isfinite(S.e2[i]))) return INFINITY;
-  const double pivmin = tri_pivmin(S.e2, N);
-  if (sturm_count(S.d, S.e2, N, -64.0 * N * eps * fmax(dmax, 1.0), pivmin) == 0) return 0.0;
-  const double lmin = tri_eig(S.d, S.e2, N, 1), lmax = tri_eig(S.d, S.e2, N, N);
-  const double bn = fmax(fabs(lmin), fabs(lmax));
-  const double budget = 64.0 * N * eps * fmax(bn, 1.0);
-  return fmax(0.0, fmax(0.0, -lmin) - budget) / fmax(bn, 2.2250738585072014e-308);
-}
-
-// Largest eigenvalue of the Hermitian H (destroyed); if `only_if_positive`,
-// returns 0 without the multisection when no eigenvalue is >= 0.
-template <int NP, int TT>
-__device__ double team_lmax(Cx<double>* H, int N, int tt, ResScratch<NP>& S, int team, bool only_if_positive) {
-  team_tridiagonalize<NP, TT>(H, N, tt, S, team);
-  for (int i = 0; i < N; ++i)
-    if (!isfinite(S.d[i]) || (i + 1 < N && !isfinite(S.e2[i]))) return INFINITY;
-  if (only_if_positive && sturm_count(S.d, S.e2, N, 0.0, tri_pivmin(S.e2, N)) == N) return 0.0;
-  return tri_eig(S.d, S.e2, N, N);
-}
 
 template <typename RS, int NP, int BPC>
 __device__ __forceinline__ void load_tile(const Cx<RS>* X, Cx<double>* bufs, int e0, int m, int NE, int Nk, int N) {
@@ -580,477 +249,6 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT) residual_kernel(ResidualArg
   }
 }
 
-// ---------------------------------------------------------------------------
-// The suite for N_b <= 32.  Its seven positivity tests were most of the time
-// of residual_kernel (which remains for N_b > 32): an LDL^T whose trailing block lives in
-// shared memory, one matrix after another, half the lanes idle.  Here each
-// LDL^T keeps one row per lane in registers, so a warp takes 32 / NP matrices
-// at once (four at N_b <= 8, two at N_b <= 16; the two warps of an N_b <= 32
-// team one each), reads their entries straight from the tiles of the fields
-// they are made of, and exchanges one column per step.  Products whose result
-// only enters a norm stay in registers, and G Gamma G^H of r_A is the
-// difference of the two raw Keldysh products, which are formed anyway.
-// Tests that fail are settled afterwards, with every tile free, by the
-// tridiagonal reduction (psd_of, team_lmax).
-// Bound by FP64 issue at 12 warps per SM.  mixed, 32 768 blocks: N_b = 16 2.16 -> 1.21
-// ms, N_b = 32 20.0 -> 8.6 ms; complex128: 2.18 -> 1.31, 20.1 -> 11.5 ms.
-// ---------------------------------------------------------------------------
-enum { HK_A = 0, HK_GL = 1, HK_GG = 2, HK_GAM = 3, HK_RAWL = 4, HK_RAWG = 5, HK_CAUS = 6, HK_COUNT = 7 };
-
-template <int NP> struct RowScratch {
-  Cx<double> col[2][Tile<NP>::TT];  // column being eliminated, per matrix of a round
-  unsigned fail[Tile<NP>::TT / 32], bad[Tile<NP>::TT / 32];
-};
-
-// Entry (i, j) of the Hermitian matrix of a test, from the tiles: G = G^R,
-// X = Sigma^R (HK_CAUS), Sigma< (HK_GAM) or the raw lesser product (HK_RAWL),
-// W = G< (HK_GL), Sigma> (HK_GAM) or the raw greater product, H = G> (HK_GG).
-template <int NP>
-__device__ __forceinline__ Cx<double> herm_entry(int kind, const Cx<double>* G, const Cx<double>* X, const Cx<double>* W,
-                                                 const Cx<double>* H, int i, int j, bool& finite) {
-  const int ij = sw<NP>(i, j), ji = sw<NP>(j, i);
-  if (kind == HK_GAM) {  // i (S> - S<)
-    const Cx<double> g = W[ij], l = X[ij], gt = W[ji], lt = X[ji];
-    const double x = g.x - l.x, y = g.y - l.y, xt = gt.x - lt.x, yt = gt.y - lt.y;
-    finite = finite && isfinite(x) && isfinite(y) && isfinite(xt) && isfinite(yt);
-    return cx<double>(0.5 * (-y - yt), 0.5 * (x - xt));
-  }
-  const Cx<double>* T = kind == HK_A ? G : kind == HK_GL || kind == HK_RAWG ? W : kind == HK_GG ? H : X;
-  const Cx<double> a = T[ij], b = T[ji];
-  finite = finite && isfinite(a.x) && isfinite(a.y) && isfinite(b.x) && isfinite(b.y);
-  if (kind == HK_A) return cx<double>(-(a.y + b.y), a.x - b.x);                        // i (G - G^H)
-  if (kind == HK_CAUS) return cx<double>(-0.5 * (a.y + b.y), 0.5 * (a.x - b.x));       // -Im_H Sigma^R
-  if (kind == HK_GL || kind == HK_RAWL) return cx<double>(0.5 * (a.y + b.y), -0.5 * (a.x - b.x));  // -i X
-  return cx<double>(-0.5 * (a.y + b.y), 0.5 * (a.x - b.x));                            // i X
-}
-
-// LDL^T tests of the matrices `kinds` (4 bits each, `count` of them): bit k of
-// fail / bad is set when matrix kind k has no certificate / is not finite.
-// Every thread of the team returns the same masks.
-template <int NP, int TT>
-__device__ void posdef_rounds(unsigned kinds, int count, const Cx<double>* G, const Cx<double>* X, const Cx<double>* W,
-                              const Cx<double>* H, int N, int tt, RowScratch<NP>& R, int team, unsigned& fail,
-                              unsigned& bad) {
-  constexpr int PER = TT / NP;  // matrices per round
-  constexpr double eps = 2.220446049250313e-16;
-  unsigned f = 0, b = 0;
-#pragma unroll 1
-  for (int base = 0; base < count; base += PER) {
-    const int g = tt / NP, r = tt - g * NP, q = base + g;
-    const bool mine = g < PER && q < count;
-    const int kind = mine ? (int)((kinds >> (4 * q)) & 15u) : HK_A;
-    Cx<double> row[NP];
-    bool finite = true;
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-      row[j] = cx<double>(j == r ? 1.0 : 0.0, 0.0);
-      if (mine && j <= r && r < N) row[j] = herm_entry<NP>(kind, G, X, W, H, r, j, finite);
-    }
-    double d = 0.0;  // largest diagonal entry of the matrix
-#pragma unroll
-    for (int j = 0; j < NP; ++j)
-      if (j == r && r < N) d = fabs(row[j].x);
-    Cx<double>* col = R.col[0] + g * NP;
-    // (lanes past the last matrix use the tail of the buffers)
-    if (PER * NP == TT || g < PER) col[r] = cx<double>(d, finite ? 0.0 : 1.0);
-    __syncwarp();
-    double nonfin = 0.0;
-    d = 0.0;
-    if (g < PER)
-      for (int j = 0; j < N; ++j) {
-        const Cx<double> c = col[j];
-        d = fmax(d, c.x);
-        nonfin += c.y;
-      }
-    const double shift = kind == HK_CAUS ? 0.0 : 64.0 * N * eps * fmax(d, 1.0);
-    bool ok = true;
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      if (k >= N) break;
-      Cx<double>* c = R.col[k & 1] + g * NP;
-      if (g < PER) c[r] = row[k];
-      __syncwarp();
-      if (g < PER) {
-        const double dk = c[k].x + shift;
-        ok = ok && dk > 0;
-        const double inv = 1.0 / dk;
-        const Cx<double> l = cx<double>(row[k].x * inv, row[k].y * inv);
-#pragma unroll
-        for (int j = k + 1; j < NP; ++j) {
-          const Cx<double> a = c[j];  // row[j] -= l conj(a)
-          row[j].x = fma(-l.x, a.x, row[j].x);
-          row[j].x = fma(-l.y, a.y, row[j].x);
-          row[j].y = fma(l.x, a.y, row[j].y);
-          row[j].y = fma(-l.y, a.x, row[j].y);
-        }
-      }
-    }
-    __syncwarp();
-    if (mine && r == 0) {
-      if (nonfin != 0.0) b |= 1u << kind;
-      else if (!ok) f |= 1u << kind;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    f |= __shfl_xor_sync(0xffffffffu, f, o);
-    b |= __shfl_xor_sync(0xffffffffu, b, o);
-  }
-  if (TT > 32) {
-    team_sync<TT>(team);
-    if ((tt & 31) == 0) {
-      R.fail[tt >> 5] = f;
-      R.bad[tt >> 5] = b;
-    }
-    team_sync<TT>(team);
-    f = b = 0;
-#pragma unroll
-    for (int w = 0; w < TT / 32; ++w) {
-      f |= R.fail[w];
-      b |= R.bad[w];
-    }
-  }
-  fail |= f;
-  bad |= b;
-}
-
-// Loads the tiles of `count` fields with all their accesses in flight.
-template <typename RS, int NP, int BPC, size_t STRIDE, int COUNT>
-__device__ __forceinline__ void load_tiles(const Cx<RS>* const (&src)[COUNT], Cx<double>* const (&dst)[COUNT], int e0,
-                                           int m, int NE, int Nk, int N) {
-  constexpr int IT = NP * NP / Tile<NP>::TT;
-  static_assert(IT * Tile<NP>::TT == NP * NP, "tile size");
-  const size_t base = (size_t)e0 + (size_t)NE * m, cstride = (size_t)NE * Nk;
-  const int eloc = threadIdx.x % BPC;
-  const bool ein = e0 + eloc < NE;
-  constexpr int G = IT % 4 == 0 ? 4 : IT % 3 == 0 ? 3 : IT;  // elements per field in flight
-#pragma unroll 1
-  for (int q0 = 0; q0 < IT; q0 += G) {
-    Cx<RS> v[COUNT][G];
-#pragma unroll
-    for (int f = 0; f < COUNT; ++f)
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-        const int el = (threadIdx.x + (q0 + q) * BPC * Tile<NP>::TT) / BPC, a = el % NP, b = el / NP;
-        v[f][q] = cx<RS>(0, 0);
-        if (ein && a < N && b < N) v[f][q] = src[f][base + eloc + cstride * ((size_t)a + (size_t)N * b)];
-      }
-#pragma unroll
-    for (int f = 0; f < COUNT; ++f)
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-        const int el = (threadIdx.x + (q0 + q) * BPC * Tile<NP>::TT) / BPC;
-        dst[f][eloc * STRIDE + sw<NP>(el % NP, el / NP)] = cvt<double>(v[f][q]);
-      }
-  }
-}
-
-// Visits the accumulators of a team product: f(row, column, value), within N.
-template <int NP, int TT, typename F>
-__device__ __forceinline__ void acc_for(const DmmaTile<NP, TT>& acc, int N, int tt, F&& f) {
-  constexpr int NT = DmmaTile<NP, TT>::NT, NW = DmmaTile<NP, TT>::NW, RPW = DmmaTile<NP, TT>::RPW;
-  const int warp = tt >> 5, lane = tt & 31, lr = lane >> 2, lc = lane & 3;
-#pragma unroll
-  for (int r = 0; r < RPW; ++r)
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int a = (warp + r * NW) * 8 + lr, b = j * 8 + 2 * lc + i;
-        if (a < N && b < N) f(a, b, cx<double>(acc.re[r][j][i], acc.im[r][j][i]));
-      }
-}
-
-// sum |K - G S G^H|^2 and sum |K|^2 with S in tile T (overwritten by G S).
-template <int NP, int TT>
-__device__ void keldysh_defect(const Cx<double>* G, Cx<double>* T, const Cx<double>* K, int N, int tt, double* scratch,
-                               int team, double& num, double& den) {
-  DmmaTile<NP, TT> acc;
-  team_matmul_dmma<NP, TT>(G, T, acc, N, tt, false);
-  team_sync<TT>(team);
-  team_store_dmma<NP, TT>(T, acc, tt);
-  team_sync<TT>(team);
-  team_matmul_dmma<NP, TT>(T, G, acc, N, tt, true);
-  num = den = 0;
-  acc_for<NP, TT>(acc, N, tt, [&](int i, int j, Cx<double> q) {
-    const Cx<double> a = K[sw<NP>(i, j)];
-    num += (a.x - q.x) * (a.x - q.x) + (a.y - q.y) * (a.y - q.y);
-    den += a.x * a.x + a.y * a.y;
-  });
-  team_sum2<TT>(num, den, tt, scratch, team);
-}
-
-// r_K alone (RES_PART_RK).
-template <typename RS, int NP, int BPC>
-__global__ void __launch_bounds__(BPC* Tile<NP>::TT) residual_rk_kernel(ResidualArgs<RS> p) {
-  constexpr int TT = Tile<NP>::TT;
-  constexpr size_t MSZ = tile_stride<double, NP, BPC>();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<double>* bG = reinterpret_cast<Cx<double>*>(smem_raw);
-  Cx<double>* bX = bG + BPC * MSZ;
-  Cx<double>* bW = bX + BPC * MSZ;
-  double* red = reinterpret_cast<double*>(bW + BPC * MSZ);
-  const int N = p.N, NE = p.NE, Nk = p.Nk, m = blockIdx.y, e0 = blockIdx.x * BPC;
-  const int team = threadIdx.x / TT, tt = threadIdx.x % TT, e = e0 + team;
-  load_tiles<RS, NP, BPC, MSZ, 3>({p.GR, p.GL, p.SLc}, {bG, bX, bW}, e0, m, NE, Nk, N);
-  __syncthreads();
-  double kNum, kDen;
-  keldysh_defect<NP, TT>(bG + team * MSZ, bW + team * MSZ, bX + team * MSZ, N, tt, red + 4 * team, team, kNum, kDen);
-  if (tt == 0 && e < NE) {
-    double* o = p.block_out + kResidualBlockDoubles * ((size_t)e + (size_t)NE * m);
-    o[3] = isfinite(kNum) ? kNum : INFINITY;
-    o[4] = isfinite(kDen) ? kDen : INFINITY;
-  }
-}
-
-// Up to N_b = 16 registers bound the CTAs per SM, so a fourth tile is free and
-// saves a load and a round of tests (N_b = 12: 0.95 against 1.05 ms); above,
-// three tiles give the fourth CTA (N_b = 32, mixed: 17.4 against 8.6 ms).
-template <int NP> constexpr bool rows_four_tiles() { return NP <= 16; }
-// Register budget: the CTAs per SM that the tiles' shared memory allows (168
-// registers at N_b <= 16; 128 there spill: 1.24 -> 1.47 ms).
-template <int NP> constexpr int rows_min_ctas() { return NP == 8 ? 2 : NP == 16 ? 6 : NP == 32 ? 4 : 3; }
-
-template <typename RS, int NP, int BPC>
-__global__ void __launch_bounds__(BPC* Tile<NP>::TT, (rows_min_ctas<NP>())) residual_rows_kernel(ResidualArgs<RS> p) {
-  constexpr bool FOUR = rows_four_tiles<NP>();
-  constexpr int TT = Tile<NP>::TT;
-  constexpr size_t MSZ = (size_t)NP * NP;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<double>* bG = reinterpret_cast<Cx<double>*>(smem_raw);
-  Cx<double>* bX = bG + BPC * MSZ;
-  Cx<double>* bW = bX + BPC * MSZ;
-  Cx<double>* bH = FOUR ? bW + BPC * MSZ : bX;
-  RowScratch<NP>* rows = reinterpret_cast<RowScratch<NP>*>((FOUR ? bH : bW) + BPC * MSZ);
-  ResScratch<NP>* scr = reinterpret_cast<ResScratch<NP>*>(rows + BPC);
-  const int N = p.N, NE = p.NE, Nk = p.Nk, m = blockIdx.y, e0 = blockIdx.x * BPC;
-  const int team = threadIdx.x / TT, tt = threadIdx.x % TT, e = e0 + team;
-  const bool live = e < NE;
-  Cx<double>* G = bG + team * MSZ;
-  Cx<double>* X = bX + team * MSZ;
-  Cx<double>* W = bW + team * MSZ;
-  const Cx<double>* H = bH + team * MSZ;
-  RowScratch<NP>& R = rows[team];
-  ResScratch<NP>& S = scr[team];
-  unsigned fail = 0, bad = 0;
-  auto kinds = [](int a, int b = 0, int c = 0, int d = 0) { return (unsigned)(a | b << 4 | c << 8 | d << 12); };
-
-  // ---- causality, A ---------------------------------------------------------
-  if constexpr (FOUR) load_tiles<RS, NP, BPC, MSZ, 4>({p.GR, p.SR, p.GL, p.GG}, {bG, bX, bW, bH}, e0, m, NE, Nk, N);
-  else load_tiles<RS, NP, BPC, MSZ, 3>({p.GR, p.SR, p.GL}, {bG, bX, bW}, e0, m, NE, Nk, N);
-  __syncthreads();
-  posdef_rounds<NP, TT>(kinds(HK_CAUS, HK_A, HK_GL, HK_GG), FOUR ? 4 : 2, G, X, W, H, N, tt, R, team, fail, bad);
-  team_sync<TT>(team);
-
-  DmmaTile<NP, TT> acc;
-  // ---- r_D: D over Sigma^R, ||D G - I|| from the accumulators ---------------
-  const double eps_e = live ? p.eps[e] : 0.0;
-  double nD = 0, nG = 0;
-  tile_for<NP, TT>(N, tt, [&](int i, int j) {
-    const Cx<double> hv = p.h[(size_t)m + (size_t)Nk * ((size_t)i + (size_t)N * j)];
-    Cx<double> d = X[sw<NP>(i, j)];
-    d = cx<double>(-hv.x - d.x, -hv.y - d.y);
-    if (i == j) d.x += eps_e;
-    X[sw<NP>(i, j)] = d;
-    nD += d.x * d.x + d.y * d.y;
-    const Cx<double> g = G[sw<NP>(i, j)];
-    nG += g.x * g.x + g.y * g.y;
-  });
-  team_sum2<TT>(nD, nG, tt, S.red, team);
-  team_sync<TT>(team);
-  team_matmul_dmma<NP, TT>(X, G, acc, N, tt, false);
-  double nR = 0;
-  acc_for<NP, TT>(acc, N, tt, [&](int i, int j, Cx<double> v) {
-    if (i == j) v.x -= 1;
-    nR += v.x * v.x + v.y * v.y;
-  });
-  nR = team_sum<TT>(nR, tt, S.red, team);
-  double rD = sqrt(nR) / (sqrt(nD) * sqrt(nG) + sqrt((double)N));
-  if (!isfinite(rD)) rD = INFINITY;
-
-  // ---- r_K ------------------------------------------------------------------
-  const bool with_rk = p.part == RES_PART_ALL;  // launch-uniform
-  double kNum = 0, kDen = 0;
-  if (with_rk) {
-    __syncthreads();
-    load_tiles<RS, NP, BPC, MSZ, 1>({p.SLc}, {bX}, e0, m, NE, Nk, N);
-    __syncthreads();
-    keldysh_defect<NP, TT>(G, X, W, N, tt, S.red, team, kNum, kDen);
-  }
-
-  // ---- G<, G>, Gamma, then the raw products ---------------------------------
-  __syncthreads();
-  if constexpr (!FOUR) {
-    load_tiles<RS, NP, BPC, MSZ, 1>({p.GG}, {bX}, e0, m, NE, Nk, N);
-    __syncthreads();
-    posdef_rounds<NP, TT>(kinds(HK_GL, HK_GG), 2, G, X, W, H, N, tt, R, team, fail, bad);
-    __syncthreads();
-  }
-  load_tiles<RS, NP, BPC, MSZ, 2>({p.SL, p.SG}, {bX, bW}, e0, m, NE, Nk, N);
-  __syncthreads();
-  posdef_rounds<NP, TT>(kinds(HK_GAM), 1, G, X, W, H, N, tt, R, team, fail, bad);
-  team_sync<TT>(team);
-  auto sandwich = [&](Cx<double>* T) {  // T <- G T G^H
-    team_matmul_dmma<NP, TT>(G, T, acc, N, tt, false);
-    team_sync<TT>(team);
-    team_store_dmma<NP, TT>(T, acc, tt);
-    team_sync<TT>(team);
-    team_matmul_dmma<NP, TT>(T, G, acc, N, tt, true);
-    team_sync<TT>(team);
-    team_store_dmma<NP, TT>(T, acc, tt);
-    team_sync<TT>(team);
-  };
-  sandwich(X);
-  sandwich(W);
-  posdef_rounds<NP, TT>(kinds(HK_RAWL, HK_RAWG), 2, G, X, W, H, N, tt, R, team, fail, bad);
-  // ---- r_A: A - G Gamma G^H = A - i (raw> - raw<) ---------------------------
-  double aNum = 0, aDen = 0;
-  tile_for<NP, TT>(N, tt, [&](int i, int j) {
-    const Cx<double> g = G[sw<NP>(i, j)], gt = G[sw<NP>(j, i)], rl = X[sw<NP>(i, j)], rg = W[sw<NP>(i, j)];
-    const double ax = -(g.y + gt.y), ay = g.x - gt.x;
-    const double dx = ax + (rg.y - rl.y), dy = ay - (rg.x - rl.x);
-    aNum += dx * dx + dy * dy;
-    aDen += ax * ax + ay * ay;
-  });
-  team_sum2<TT>(aNum, aDen, tt, S.red, team);
-
-  // ---- tests without a certificate ------------------------------------------
-  double psd = 0, wr = -1.0, wk = -1.0;  // as in residual_kernel
-  double caus = bad >> HK_CAUS & 1u ? INFINITY : 0.0;
-  const Cx<double> one = cx<double>(1, 0), mi = cx<double>(0, -1), pi = cx<double>(0, 1);
-#pragma unroll 1
-  for (int kind = 0; kind < 6; ++kind) {
-    double r = bad >> kind & 1u ? INFINITY : 0.0;
-    // a CTA's blocks reload together: the loads are CTA-wide
-    const bool need = (fail >> kind & 1u) && live;
-    if (__syncthreads_or(need)) {
-      const Cx<RS>* src = kind == HK_A ? p.GR : kind == HK_GL ? p.GL : kind == HK_GG ? p.GG : kind == HK_RAWG ? p.SG : p.SL;
-      load_tiles<RS, NP, BPC, MSZ, 1>({src}, {bX}, e0, m, NE, Nk, N);
-      if (kind == HK_GAM) load_tiles<RS, NP, BPC, MSZ, 1>({p.SG}, {bW}, e0, m, NE, Nk, N);
-      __syncthreads();
-      if (need) {
-        if (kind == HK_RAWL || kind == HK_RAWG) sandwich(X);
-        if (kind == HK_A || kind == HK_GAM) {
-          tile_for<NP, TT>(N, tt, [&](int i, int j) {
-            const Cx<double> g = kind == HK_A ? G[sw<NP>(i, j)] : W[sw<NP>(i, j)];
-            const Cx<double> l = kind == HK_A ? conj(G[sw<NP>(j, i)]) : X[sw<NP>(i, j)];
-            X[sw<NP>(i, j)] = pi * cx<double>(g.x - l.x, g.y - l.y);
-          });
-          team_sync<TT>(team);
-        }
-        r = psd_of<NP, TT>(X, kind == HK_GL || kind == HK_RAWL ? mi : kind == HK_GG || kind == HK_RAWG ? pi : one, W, N,
-                           tt, S, team);
-        team_sync<TT>(team);
-      }
-    }
-    psd = fmax(psd, r);
-    if (kind >= 4 && !isfinite(r)) continue;
-    if (r > wr) {  // kinds in ascending order: the lowest kind keeps a tie
-      wr = r;
-      wk = kind;
-    }
-  }
-  const bool need = (fail >> HK_CAUS & 1u) && live;
-  if (__syncthreads_or(need)) {
-    load_tiles<RS, NP, BPC, MSZ, 1>({p.SR}, {bX}, e0, m, NE, Nk, N);
-    __syncthreads();
-    if (need) {
-      tile_for<NP, TT>(N, tt, [&](int i, int j) {
-        const Cx<double> a = X[sw<NP>(i, j)], b = X[sw<NP>(j, i)];
-        W[sw<NP>(i, j)] = cx<double>(0.5 * (a.y + b.y), -0.5 * (a.x - b.x));  // (a - conj(b)) / (2i)
-      });
-      team_sync<TT>(team);
-      const double num = fmax(0.0, team_lmax<NP, TT>(W, N, tt, S, team, true));
-      team_sync<TT>(team);
-      if (num > 0 && isfinite(num)) {  // ||Sigma^R||_2^2 = lmax(Sigma^R Sigma^R^H)
-        team_matmul<double, double, NP>(X, X, W, N, tt, true);
-        team_sync<TT>(team);
-        const double lmax = team_lmax<NP, TT>(W, N, tt, S, team, false);
-        caus = num / (sqrt(fmax(lmax, 0.0)) + 1e-14);
-      } else if (!isfinite(num)) {
-        caus = INFINITY;
-      }
-    }
-  }
-
-  if (tt == 0 && live) {
-    double* o = p.block_out + kResidualBlockDoubles * ((size_t)e + (size_t)NE * m);
-    o[0] = rD;
-    o[1] = isfinite(aNum) ? aNum : INFINITY;
-    o[2] = isfinite(aDen) ? aDen : INFINITY;
-    if (with_rk) {
-      o[3] = isfinite(kNum) ? kNum : INFINITY;
-      o[4] = isfinite(kDen) ? kDen : INFINITY;
-    }
-    o[5] = psd;
-    o[6] = caus;
-    o[7] = wr;
-    o[8] = wk;
-  }
-}
-
-// Fixed-order reduction of the per-block outputs:
-// out = (r_D, r_A, r_K, r_PSD, r_caus).
-__global__ void residual_reduce_kernel(long long blocks, const double* __restrict__ bo, double* partial) {
-  double mx[3] = {0, 0, 0}, sm[4] = {0, 0, 0, 0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < blocks;
-       i += (long long)gridDim.x * blockDim.x) {
-    const double* o = bo + kResidualBlockDoubles * i;
-    mx[0] = fmax(mx[0], o[0]) + (isnan(o[0]) ? INFINITY : 0.0);
-    sm[0] += o[1];
-    sm[1] += o[2];
-    sm[2] += o[3];
-    sm[3] += o[4];
-    mx[1] = fmax(mx[1], o[5]) + (isnan(o[5]) ? INFINITY : 0.0);
-    mx[2] = fmax(mx[2], o[6]) + (isnan(o[6]) ? INFINITY : 0.0);
-  }
-  __shared__ double red[7][8];
-  double v[7] = {mx[0], sm[0], sm[1], sm[2], sm[3], mx[1], mx[2]};
-#pragma unroll
-  for (int k = 0; k < 7; ++k)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double q = __shfl_xor_sync(0xffffffffu, v[k], o);
-      v[k] = (k == 0 || k >= 5) ? fmax(v[k], q) : v[k] + q;
-    }
-  if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 7; ++k) red[k][threadIdx.x >> 5] = v[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 7; ++k) {
-      double s = red[k][0];
-      for (int w = 1; w < 8; ++w) s = (k == 0 || k >= 5) ? fmax(s, red[k][w]) : s + red[k][w];
-      partial[7 * blockIdx.x + k] = s;
-    }
-  }
-}
-
-// One warp per quantity, fixed-order lane sums then a fixed shuffle tree.
-__global__ void residual_final_kernel(int ncta, const double* partial, double* out) {
-  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __shared__ double v[7];
-  const bool is_max = k == 0 || k >= 5;
-  double a = 0;
-  for (int c = lane; c < ncta; c += 32) {
-    const double q = partial[7 * c + k];
-    a = is_max ? fmax(a, q) + (isnan(q) ? INFINITY : 0.0) : a + q;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double q = __shfl_xor_sync(0xffffffffu, a, o);
-    a = is_max ? fmax(a, q) : a + q;
-  }
-  if (lane == 0) v[k] = a;
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  out[0] = v[0];
-  out[1] = (isfinite(v[1]) && isfinite(v[2])) ? sqrt(v[1]) / (sqrt(v[2]) + 1e-14) : INFINITY;
-  out[2] = (isfinite(v[3]) && isfinite(v[4])) ? sqrt(v[3]) / (sqrt(v[4]) + 1e-14) : INFINITY;
-  out[3] = v[5];
-  out[4] = v[6];
-}
-
 template <typename RS, int NP, int BPC> static int launch_residual_t(const ResidualArgs<RS>& a, cudaStream_t st) {
   constexpr int TT = Tile<NP>::TT;
   // four tiles per team (G, X, W, H) and the scratch
@@ -1067,51 +265,12 @@ template <typename RS, int NP, int BPC> static int launch_residual_t(const Resid
   return QCL_OK;
 }
 
-// r_K alone has no tests and is bound by its loads, where longer runs of
-// energies help: N_b = 32, 1024 x 32 blocks, mixed, 2 per CTA instead of 1: 1.52
-// -> 0.98 ms; N_b = 12 and 16, 4 instead of 2: 6400 blocks, c128, 37 -> 30 us,
-// 3064 blocks, mixed, 30 -> 24 us, and whole iterations at 3064 ... 32768 blocks
-// take the same or less at every count (N_b = 16, c128: 484.9 -> 482.4 us at
-// 3064, 1056 -> 1043 at 8192, 1987 -> 1960 at 16384, 3786 -> 3732 at 32768).
-template <typename RS, int NP, int BPC> static int launch_residual_rk_t(const ResidualArgs<RS>& a, cudaStream_t st) {
-  constexpr size_t smem = BPC * (3 * tile_stride<double, NP, BPC>() * sizeof(Cx<double>) + 4 * sizeof(double));
-  static bool configured = false;
-  if (!configured) {
-    QCL_CUDA_CHECK(cudaFuncSetAttribute(residual_rk_kernel<RS, NP, BPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-    configured = true;
-  }
-  residual_rk_kernel<RS, NP, BPC><<<dim3((a.NE + BPC - 1) / BPC, a.Nk), BPC * Tile<NP>::TT, smem, st>>>(a);
-  QCL_LAUNCH_CHECK("residual_rk_kernel");
-  return QCL_OK;
-}
-
-template <typename RS, int NP, int BPC> static int launch_residual_rows_t(const ResidualArgs<RS>& a, cudaStream_t st) {
-  constexpr int TT = Tile<NP>::TT;
-  constexpr size_t tile = (size_t)BPC * NP * NP * sizeof(Cx<double>);
-  constexpr size_t smem = (rows_four_tiles<NP>() ? 4 : 3) * tile + BPC * (sizeof(RowScratch<NP>) + sizeof(ResScratch<NP>));
-  static bool configured = false;
-  if (!configured) {
-    QCL_CUDA_CHECK(cudaFuncSetAttribute(residual_rows_kernel<RS, NP, BPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-    configured = true;
-  }
-  if (a.part == RES_PART_RK) {
-    if (NP == 32) return launch_residual_rk_t<RS, NP, 2>(a, st);
-    return launch_residual_rk_t<RS, NP, NP == 16 ? 4 : BPC>(a, st);
-  }
-  const dim3 grid((a.NE + BPC - 1) / BPC, a.Nk);
-  residual_rows_kernel<RS, NP, BPC><<<grid, BPC * TT, smem, st>>>(a);
-  QCL_LAUNCH_CHECK("residual_rows_kernel");
-  return QCL_OK;
-}
-
 template <typename RS> static int launch_residual_p(const ResidualArgs<RS>& a, cudaStream_t st) {
   switch (padded_size(a.N)) {
-    case 8: return launch_residual_rows_t<RS, 8, 8>(a, st);
-    case 16: return launch_residual_rows_t<RS, 16, 2>(a, st);
-    case 24: return launch_residual_rows_t<RS, 24, 2>(a, st);
-    case 32: return launch_residual_rows_t<RS, 32, 1>(a, st);
+    case 8:
+    case 16: return launch_residual_rows_small(a, st);
+    case 24:
+    case 32: return launch_residual_rows_large(a, st);
     case 48: return launch_residual_t<RS, 48, 1>(a, st);
     default:
       set_last_error("basis size N_b=%d exceeds the supported maximum 48", a.N);
@@ -1792,7 +951,6 @@ int launch_anderson_guard(int precision, int NE, int Nk, int N, void* const* fie
   return launch_guard_p<float>(a, st);
 }
 
-constexpr int RES_CTAS = 148;
 
 size_t residual_work_doubles(int NE, int Nk) { return kResidualBlockDoubles * (size_t)NE * Nk + 7 * RES_CTAS; }
 
@@ -1856,15 +1014,6 @@ int launch_residual_blocks(int precision, int part, int NE, int Nk, int N, const
                         (const Cx<float>*)GG, (const Cx<float>*)SR, (const Cx<float>*)SL, (const Cx<float>*)SG,
                         (const Cx<float>*)SLc, work, part};
   return launch_residual_p<float>(a, st);
-}
-
-// Fixed-order reduction of the per-block outputs in `work` into out5.
-int launch_residual_reduce(int NE, int Nk, double* work, double* out5, cudaStream_t st) {
-  double* partial = work + kResidualBlockDoubles * (size_t)NE * Nk;
-  residual_reduce_kernel<<<RES_CTAS, 256, 0, st>>>((long long)NE * Nk, work, partial);
-  residual_final_kernel<<<1, 7 * 32, 0, st>>>(RES_CTAS, partial, out5);
-  QCL_LAUNCH_CHECK("residual_reduce");
-  return QCL_OK;
 }
 
 int launch_residual_suite(int precision, int NE, int Nk, int N, const double* eps, const void* h, const void* GR,
