@@ -21,26 +21,9 @@
 #include <mutex>
 
 #include "blockmat.cuh"
+#include "dyson.cuh"
 
 namespace qcl {
-
-template <typename RS> struct DysonArgs {
-  int NE, Nk, N, m0;  // blocks of momenta m0 .. m0 + gridDim.y - 1
-  const double* eps;
-  double eta;
-  const Cx<double>* h;  // (Nk, N, N), FP64 always
-  const Cx<RS>* sigR;
-  const Cx<RS>* sigL;
-  const Cx<RS>* sigG;   // may be null
-  Cx<RS>* GR;           // may be null
-  Cx<RS>* GL;           // may be null
-  Cx<RS>* GG;           // may be null
-  double* scale;        // (NE, Nk), may be null
-  Cx<double>* traceL;   // (NE, Nk) raw tr G<, may be null
-  Cx<double>* traceG;   // (NE, Nk) raw tr G>, may be null
-  int* status;
-  int mcount;
-};
 
 // Argmax key of a pivot candidate: the high 32 bits of its magnitude (IEEE
 // order = unsigned order for non-negative values) with the low 6 bits replaced
@@ -55,13 +38,6 @@ __device__ __forceinline__ unsigned pivot_key(float mag, int row) {
   return (__float_as_uint(mag) & ~63u) | (unsigned)(63 - row);
 }
 __device__ __forceinline__ bool pivot_key_zero(unsigned key) { return (key >> 6) == 0u; }
-// The magnitude's bits as one integer, for exact comparisons, and the same
-// test for zero.
-__device__ __forceinline__ unsigned long long mag_bits(double mag) { return (unsigned long long)__double_as_longlong(mag); }
-__device__ __forceinline__ unsigned mag_bits(float mag) { return __float_as_uint(mag); }
-__device__ __forceinline__ bool mag_zero(unsigned long long bits) { return (bits >> 38) == 0u; }
-__device__ __forceinline__ bool mag_zero(unsigned bits) { return (bits >> 6) == 0u; }
-
 // Shared-memory store under a predicate, without a branch.
 __device__ __forceinline__ void st_shared_if(Cx<double>* ptr, Cx<double> v, bool pred) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(ptr);
@@ -520,185 +496,6 @@ __global__ void __launch_bounds__(BPC* Tile<NP>::TT, (dyson_min_ctas<RS, RL, NP,
   }
 }
 
-// ---------------------------------------------------------------------------
-// Small bases (N_b <= 6): one thread per (E, k) block, the block in registers.  The lanes of a warp are 32 consecutive
-// energies, so every element of a field is one contiguous access of the warp
-// and nothing goes through shared memory; a warp-per-block team pads N_b = 5
-// to 8 x 8 and works with 20 of 32 lanes.  In-place Gauss-Jordan with row
-// interchanges (predicated swaps keep every register index static), then the
-// products row by row with Sigma re-read from L1 (a second N x N register
-// block would spill).  Bound by FP64 issue and load latency at 8 warps per SM.
-// N_E x N_k = 2401 x 61, complex128, G^R, G^<, G^>: N_b = 5 696 -> 131 us (54 us
-// of HBM traffic), N_b = 3 569 -> 35 us, N_b = 6 733 -> 238 us.
-// ---------------------------------------------------------------------------
-constexpr int kSmallThreads = 64;
-// One thread's chain of a block is longer than a team's: with few blocks the
-// team kernel answers sooner (123 blocks: N_b = 5 12.6 / 16.7 us, N_b = 6 12.7 /
-// 25.5 us; 6400 blocks: 33.1 / 17.6 and 35.2 / 29.1 us; N_b <= 4 is faster at
-// every count).
-static bool dyson_small(int N, long long blocks) {
-  return N <= 4 || (N == 5 && blocks >= 2048) || (N == 6 && blocks >= 4096);
-}
-// The kernel reads a block's Sigma^< and Sigma^> row by row between its
-// stores; the team kernel has them in shared memory before it stores, so a
-// call that writes a Green function over one of them takes that kernel.
-template <typename RS> static bool dyson_in_place(const DysonArgs<RS>& a) {
-  const size_t bytes = (size_t)a.NE * a.Nk * a.N * a.N * sizeof(Cx<RS>);
-  const auto overlap = [&](const void* x, const void* y) {
-    return x && y && (const char*)x < (const char*)y + bytes && (const char*)y < (const char*)x + bytes;
-  };
-  const Cx<RS>* const outs[3] = {a.GR, a.GL, a.GG};
-  for (const Cx<RS>* out : outs)
-    if (overlap(a.sigL, out) || overlap(a.sigG, out)) return true;
-  return false;
-}
-
-template <typename RS, typename RL, typename RM, int N>
-__global__ void __launch_bounds__(kSmallThreads) dyson_small_kernel(DysonArgs<RS> p) {
-  const int e = blockIdx.x * kSmallThreads + threadIdx.x, NE = p.NE, Nk = p.Nk, m = p.m0 + blockIdx.y;
-  if (e >= NE) return;
-  const size_t at = (size_t)e + (size_t)NE * m, cs = (size_t)NE * Nk;
-  Cx<RL> w[N][N];
-  const double eps_e = p.eps[e];
-  double s = 0.0;
-#pragma unroll
-  for (int a = 0; a < N; ++a) {
-    double rsum = 0.0;
-#pragma unroll
-    for (int b = 0; b < N; ++b) {
-      const Cx<double> hv = p.h[(size_t)m + (size_t)Nk * (a + N * b)];
-      const Cx<RS> sv = p.sigR[at + cs * (a + N * b)];
-      double re = -hv.x - (double)sv.x, im = -hv.y - (double)sv.y;
-      if (a == b) {
-        re += eps_e;
-        im += p.eta;
-      }
-      w[a][b] = cx<RL>((RL)re, (RL)im);
-      rsum += sqrt(re * re + im * im);
-    }
-    s = fmax(s, rsum);
-  }
-  const RL inv_s = (RL)(1.0 / s);
-  const bool scale_ok = s > 0.0 && isfinite(s);
-#pragma unroll
-  for (int a = 0; a < N; ++a)
-#pragma unroll
-    for (int b = 0; b < N; ++b) w[a][b] = inv_s * w[a][b];
-  int piv[N], zstep = -1;
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    // by the bits of the magnitudes, as pivot_key: a NaN ranks above any number
-    int best = k;
-    auto mag = mag_bits(cabs1(w[k][k]));
-#pragma unroll
-    for (int r = k + 1; r < N; ++r) {
-      const auto q = mag_bits(cabs1(w[r][k]));
-      if (q > mag) {
-        mag = q;
-        best = r;
-      }
-    }
-    piv[k] = best;
-    const bool zero = mag_zero(mag);
-    if (zero && zstep < 0) zstep = k;
-#pragma unroll
-    for (int r = k + 1; r < N; ++r)
-#pragma unroll
-      for (int b = 0; b < N; ++b) {
-        const Cx<RL> x = w[k][b], y = w[r][b];
-        w[k][b] = best == r ? y : x;
-        w[r][b] = best == r ? x : y;
-      }
-    const Cx<RL> rp = zero ? cx<RL>(0, 0) : crecip_pivot(w[k][k]);
-    w[k][k] = cx<RL>(1, 0);
-#pragma unroll
-    for (int b = 0; b < N; ++b) w[k][b] = rp * w[k][b];
-#pragma unroll
-    for (int r = 0; r < N; ++r) {
-      if (r == k) continue;
-      const Cx<RL> f = w[r][k];
-      w[r][k] = cx<RL>(0, 0);
-#pragma unroll
-      for (int b = 0; b < N; ++b) cfms(w[r][b], f, w[k][b]);
-    }
-  }
-#pragma unroll
-  for (int k = N - 1; k >= 0; --k)  // undo the interchanges on the columns
-#pragma unroll
-    for (int c = k + 1; c < N; ++c)
-#pragma unroll
-      for (int a = 0; a < N; ++a) {
-        const Cx<RL> x = w[a][k], y = w[a][c];
-        w[a][k] = piv[k] == c ? y : x;
-        w[a][c] = piv[k] == c ? x : y;
-      }
-  if (!scale_ok || zstep >= 0)
-    record_status(p.status, QCL_SINGULAR, (long long)at * kSingularPivotSpan + (scale_ok ? zstep + 1 : 0));
-  if (p.scale) p.scale[at] = s;
-  Cx<RS> g[N][N];
-#pragma unroll
-  for (int a = 0; a < N; ++a)
-#pragma unroll
-    for (int b = 0; b < N; ++b) {
-      g[a][b] = cvt<RS>(inv_s * w[a][b]);
-      if (p.GR) p.GR[at + cs * (a + N * b)] = g[a][b];
-    }
-#pragma unroll 1
-  for (int which = 0; which < 2; ++which) {
-    const Cx<RS>* __restrict__ sig = which == 0 ? p.sigL : p.sigG;
-    Cx<RS>* __restrict__ out = which == 0 ? p.GL : p.GG;
-    Cx<double>* tr = which == 0 ? p.traceL : p.traceG;
-    if (sig == nullptr || out == nullptr) continue;
-    double tre = 0, tim = 0;
-#pragma unroll
-    for (int a = 0; a < N; ++a) {
-      Cx<RM> t[N];
-#pragma unroll
-      for (int b = 0; b < N; ++b) t[b] = cx<RM>(0, 0);
-#pragma unroll
-      for (int l = 0; l < N; ++l)
-#pragma unroll
-        for (int b = 0; b < N; ++b) cfma(t[b], cvt<RM>(g[a][l]), cvt<RM>(sig[at + cs * (l + N * b)]));
-#pragma unroll
-      for (int b = 0; b < N; ++b) {
-        const Cx<RS> tb = cvt<RS>(t[b]);  // the product is stored between the two stages, as in the team kernel
-        t[b] = cvt<RM>(tb);
-      }
-#pragma unroll
-      for (int b = 0; b < N; ++b) {
-        Cx<RM> o = cx<RM>(0, 0);
-#pragma unroll
-        for (int l = 0; l < N; ++l) cfma_conj(o, t[l], cvt<RM>(g[b][l]));
-        const Cx<RS> v = cvt<RS>(o);
-        out[at + cs * (a + N * b)] = v;
-        if (a == b) {
-          tre += (double)v.x;
-          tim += (double)v.y;
-        }
-      }
-    }
-    if (tr) tr[at] = cx<double>(tre, tim);
-  }
-}
-
-template <typename RS, typename RL, typename RM>
-static int launch_dyson_small(const DysonArgs<RS>& a, cudaStream_t st) {
-  const dim3 grid((a.NE + kSmallThreads - 1) / kSmallThreads, a.mcount);
-#define SMALL(NV) \
-  case NV: dyson_small_kernel<RS, RL, RM, NV><<<grid, kSmallThreads, 0, st>>>(a); break
-  switch (a.N) {
-    SMALL(1);
-    SMALL(2);
-    SMALL(3);
-    SMALL(4);
-    SMALL(5);
-    SMALL(6);
-  }
-#undef SMALL
-  QCL_LAUNCH_CHECK("dyson_small_kernel");
-  return QCL_OK;
-}
-
 template <typename RS, typename RL, typename RM, int NP, int BPC>
 static int launch_dyson_t(const DysonArgs<RS>& a, cudaStream_t st) {
   constexpr int TT = Tile<NP>::TT;
@@ -799,6 +596,27 @@ static int launch_dyson_np(const DysonArgs<RS>& a, int bpc, cudaStream_t st) {
     if (bpc == 2) return launch_dyson_t<RS, RL, RM, 48, 2>(a, st);
     return launch_dyson_t<RS, RL, RM, 48, 1>(a, st);
   }
+}
+
+// Which kernel.  One thread's chain of a block is longer than a team's: with few blocks the
+// team kernel answers sooner (123 blocks: N_b = 5 12.6 / 16.7 us, N_b = 6 12.7 /
+// 25.5 us; 6400 blocks: 33.1 / 17.6 and 35.2 / 29.1 us; N_b <= 4 is faster at
+// every count).
+static bool dyson_small(int N, long long blocks) {
+  return N <= 4 || (N == 5 && blocks >= 2048) || (N == 6 && blocks >= 4096);
+}
+// The small kernel reads a block's Sigma^< and Sigma^> row by row between its
+// stores; the team kernel has them in shared memory before it stores, so a
+// call that writes a Green function over one of them takes that kernel.
+template <typename RS> static bool dyson_in_place(const DysonArgs<RS>& a) {
+  const size_t bytes = (size_t)a.NE * a.Nk * a.N * a.N * sizeof(Cx<RS>);
+  const auto overlap = [&](const void* x, const void* y) {
+    return x && y && (const char*)x < (const char*)y + bytes && (const char*)y < (const char*)x + bytes;
+  };
+  const Cx<RS>* const outs[3] = {a.GR, a.GL, a.GG};
+  for (const Cx<RS>* out : outs)
+    if (overlap(a.sigL, out) || overlap(a.sigG, out)) return true;
+  return false;
 }
 
 template <typename RS, typename RL, typename RM>
