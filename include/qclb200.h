@@ -561,7 +561,8 @@ void qcl_sweep_destroy(qcl_sweep* sweep);
  * (E, k) blocks per CTA, which sets threads, shared memory and registers per
  * CTA -- for one basis class (N_b padded to 8, 16, 24, 32 or 48) and
  * precision on a synthetic NE x Nk batch; every later Dyson launch of that
- * class in the process uses the fastest.  qcl_autotune_reset restores the
+ * class in the process uses the fastest (N_b <= 6 mostly runs one thread per
+ * block, which has no such shape).  qcl_autotune_reset restores the
  * built-in choices; qcl_tuned_dyson_bpc reports the one in use. */
 typedef struct qcl_tune_result {
   int dyson_bpc;   /* chosen blocks per CTA */

@@ -407,7 +407,8 @@ struct I8Src {
 
 // Largest part of each row as FP64 bits (non-negative values order as
 // integers; a non-finite value gives +inf), which the caller zeroes first.
-__global__ void i8_row_max_kernel(I8Src a, unsigned long long* __restrict__ rowmax, int kper) {
+__global__ void i8_row_max_kernel(I8Src a, unsigned long long* __restrict__ rowmax, int kper, const int* level) {
+  if (*level == kI8Rejected) return;  // by an earlier panel (launch-uniform)
   __shared__ double red[8][32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int r = blockIdx.x * 32 + tx, f = r / a.rpad, e = r - f * a.rpad;
@@ -651,12 +652,12 @@ template <int BN> static int launch_i8_levels(const I8Args& a, int sms, cudaStre
   return s ? s : launch_i8_t<BN, I8_WIDE>(a, sms, st);
 }
 
-static int i8_row_max(const I8Src& a, unsigned long long* rowmax, cudaStream_t st) {
+static int i8_row_max(const I8Src& a, unsigned long long* rowmax, const int* level, cudaStream_t st) {
   QCL_CUDA_CHECK(cudaMemsetAsync(rowmax, 0, (size_t)a.total * sizeof(unsigned long long), st));
   const int rb = a.total / 32;
   const int ks = std::max(1, std::min(ceil_div(a.K, 64), 8 * 148 / rb));
   const int kper = ceil_div(a.K, ks);
-  i8_row_max_kernel<<<dim3(rb, ceil_div(a.K, kper)), 256, 0, st>>>(a, rowmax, kper);
+  i8_row_max_kernel<<<dim3(rb, ceil_div(a.K, kper)), 256, 0, st>>>(a, rowmax, kper, level);
   QCL_LAUNCH_CHECK("i8_row_max_kernel");
   return QCL_OK;
 }
@@ -710,14 +711,14 @@ int launch_i8_gemm(int M, int fields, int N, int K, const void* const* A, long l
       const int n0 = j * l.npan, n = std::min(l.npan, N - n0), bpad = i8_bpad(n);
       unsigned long long* const bmax = (unsigned long long*)(base + l.bmax) + (size_t)j * l.bpad;
       const I8Src bs{{(const Cx<double>*)B + n0, nullptr}, ldb, nullptr, 1, n, bpad, bpad, K};
-      if (bound && (s = i8_row_max(bs, bmax, st))) return s;
+      if (bound && (s = i8_row_max(bs, bmax, level, st))) return s;
       if ((s = bound ? i8_leading(bs, bmax, Bd, level, st) : i8_split(bs, bmax, eb, Bd, l.nkb, level, st))) return s;
       for (int i = 0; i < l.mpans; ++i) {
         const int m0 = i * l.mpan, m = std::min(l.mpan, M - m0), mpad = i8_mpad(m), rows = fields * mpad;
         unsigned long long* const amax = (unsigned long long*)(base + l.amax) + (size_t)i * l.rows;
         const I8Src as{{(const Cx<double>*)A[0] + m0, fields > 1 ? (const Cx<double>*)A[1] + m0 : nullptr}, lda, w, wmod,
                        m, mpad, rows, K};
-        if (bound && j == 0 && (s = i8_row_max(as, amax, st))) return s;
+        if (bound && j == 0 && (s = i8_row_max(as, amax, level, st))) return s;
         if (j == 0 || l.mpans > 1)
           if ((s = bound ? i8_leading(as, amax, Ad, level, st) : i8_split(as, amax, ea, Ad, l.nkb, level, st)))
             return s;
