@@ -133,7 +133,9 @@ struct ScbaCtx {
   void *tot[3] = {nullptr, nullptr, nullptr};
   void* candSL = nullptr;
   void* tmp = nullptr;
-  void* slab = nullptr;  // small fields share one allocation
+  // small contexts: one allocation for what lives as long as the context
+  char* slab = nullptr;
+  size_t slab_bytes = 0, slab_used = 0;
   void* cwork = nullptr;
   size_t cwork_bytes = 0;
   void* i8_work = nullptr;  // complex128: work area of the integer tensor path, where the budget has room
@@ -224,28 +226,46 @@ static int dalloc(void** p, size_t bytes) {
   if (e != cudaSuccess) return cuda_status(e, "cudaMalloc (SCBA context)");
   return QCL_OK;
 }
+// Memory that lives as long as the context, from its slab where that has room
+// (an allocation costs a small context more than its use of the memory).
+static int dalloc(ScbaCtx* c, void** p, size_t bytes) {
+  const size_t n = (bytes + 511) / 512 * 512;
+  if (c->slab && c->slab_used + n <= c->slab_bytes) {
+    *p = c->slab + c->slab_used;
+    c->slab_used += n;
+    return QCL_OK;
+  }
+  return dalloc(p, bytes);
+}
+static void dfree(ScbaCtx* c, void* p) {
+  if (!c->slab || (char*)p < c->slab || (char*)p >= c->slab + c->slab_bytes) cudaFree(p);
+}
 // Uploads go on the context's stream: the context's kernels run on a
 // non-blocking stream, which a plain cudaMemcpy (legacy stream; from pageable
 // memory it may return before the DMA has landed) would not order them after.
 // The source may be host or device memory (unified addressing picks the
 // direction), so operators assembled on the device need no host round trip.
-template <typename T> static int dupload(T** p, const void* host, size_t bytes, cudaStream_t st) {
-  int s = dalloc((void**)p, bytes);
-  if (s) return s;
-  QCL_CUDA_CHECK(cudaMemcpyAsync(*p, host, bytes, cudaMemcpyDefault, st));
-  QCL_CUDA_CHECK(cudaStreamSynchronize(st));  // the host buffer may be a temporary
+static int upload(ScbaCtx* c, void* dst, const void* src, size_t bytes) {
+  QCL_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, c->st));
+  QCL_CUDA_CHECK(cudaStreamSynchronize(c->st));  // the source may be a temporary
   return QCL_OK;
+}
+template <typename T> static int dupload(ScbaCtx* c, T** p, const void* src, size_t bytes) {
+  const int s = dalloc(c, (void**)p, bytes);
+  return s ? s : upload(c, *p, src, bytes);
 }
 
 // Uploads an operator array in the context's precision; a refinement context
 // of reduced precision also keeps the complex128 array (*keep64) for promote.
 static int upload_op(ScbaCtx* c, void** dst, const void* host_c128, size_t n, void** keep64 = nullptr) {
+  if (c->precision == QCL_C128) return dupload(c, dst, host_c128, n * 16);
+  // (not from the slab: the copies are freed here and by promote)
   void* tmp = nullptr;
-  int s = dupload(&tmp, host_c128, n * 16, c->st);
+  int s = dalloc(&tmp, n * 16);
   if (s) return s;
-  if (c->precision == QCL_C128) {
-    *dst = tmp;
-    return QCL_OK;
+  if ((s = upload(c, tmp, host_c128, n * 16))) {
+    cudaFree(tmp);
+    return s;
   }
   if ((s = dalloc(dst, n * 8))) {
     cudaFree(tmp);
@@ -269,7 +289,7 @@ static int fill_plan(ScbaCtx* c, DevShift& d, double delta) {
   int s = build_shift_plan_host(c->NE, c->eps_h.data(), delta, l, r, th, v);
   if (s) return s;
   if (!d.theta) {
-    if ((s = dalloc((void**)&d.theta, host.size()))) return s;
+    if ((s = dalloc(c, (void**)&d.theta, host.size()))) return s;
     d.left = (int*)(d.theta + NE);
     d.right = d.left + NE;
     d.valid = (unsigned char*)(d.right + NE);
@@ -286,30 +306,18 @@ void scba_destroy(ScbaCtx* c) {
     if (c->graph[g]) cudaGraphExecDestroy(c->graph[g]);
   for (int g = 0; g < 2; ++g)
     if (c->gtpl[g]) cudaGraphDestroy(c->gtpl[g]);
-  cudaFree(c->eps);
-  cudaFree(c->wE);
-  cudaFree(c->wk);
-  cudaFree(c->h);
-  cudaFree(c->Tp);
-  cudaFree(c->Tm);
-  for (auto& d : c->shift) cudaFree(d.theta);  // the plan's one allocation
+  for (void* p : {(void*)c->eps, (void*)c->wE, (void*)c->wk, c->h, c->Tp, c->Tm}) dfree(c, p);
+  for (auto& d : c->shift) dfree(c, d.theta);  // the plan's one allocation
   for (auto& m : c->mech) {
-    cudaFree(m.block);
-    cudaFree(m.matrix);
-    cudaFree(m.left);
-    cudaFree(m.right);
-    cudaFree(m.radial);
+    for (void* p : {m.block, m.matrix, m.left, m.right, m.radial}) dfree(c, p);
     cudaFree(m.tc_bop);
     for (void* q : m.tc_chunks) cudaFree(q);
     for (void* q : m.tc_stage1) cudaFree(q);
     for (void* q : {m.block64, m.matrix64, m.left64, m.right64, m.radial64}) cudaFree(q);
   }
-  if (!c->slab) {
-    for (void* p : c->state) cudaFree(p);
-    for (void* p : c->cand) cudaFree(p);
-    for (void* p : {c->GR, c->GL, c->GG, c->tot[0], c->tot[1], c->tot[2], c->candSL, c->tmp}) cudaFree(p);
-  }
-  cudaFree(c->slab);
+  for (void* p : c->state) dfree(c, p);
+  for (void* p : c->cand) dfree(c, p);
+  for (void* p : {c->GR, c->GL, c->GG, c->tot[0], c->tot[1], c->tot[2], c->candSL, c->tmp}) dfree(c, p);
   for (auto* v : {&c->tv, &c->tw, &c->tsrc})
     for (void* p : *v) cudaFree(p);
   for (int k = 0; k < 3; ++k) {
@@ -320,21 +328,13 @@ void scba_destroy(ScbaCtx* c) {
   cudaFree(c->ttrG);
   cudaFree(c->tscal);
   if (c->tscal_h) cudaFreeHost(c->tscal_h);
-  cudaFree(c->cwork);
   cudaFree(c->i8_work);
   cudaFree(c->br_area);
-  cudaFree(c->trL);
-  cudaFree(c->trG);
-  cudaFree(c->rpartial);
-  cudaFree(c->mpartial);
-  cudaFree(c->reswork);
-  cudaFree(c->obspartial);
-  cudaFree(c->scal);
+  for (void* p : {c->cwork, (void*)c->trL, (void*)c->trG, (void*)c->rpartial, (void*)c->mpartial, (void*)c->reswork,
+                  (void*)c->obspartial, (void*)c->scal, c->Xh, c->Rh, (void*)c->ameta, (void*)c->apartial})
+    dfree(c, p);
+  cudaFree(c->slab);
   cudaFreeHost(c->scal_h);
-  cudaFree(c->Xh);
-  cudaFree(c->Rh);
-  cudaFree(c->ameta);
-  cudaFree(c->apartial);
   if (c->ameta_h) cudaFreeHost(c->ameta_h);
   free_hilbert_tables(c->hil);
   for (auto& e : c->pev)
@@ -538,6 +538,10 @@ static void branch_area(ScbaCtx* c) {
   }
 }
 
+// Contexts up to this size take one allocation (41 x 3 x 4: create 1.14 -> 1.04 ms,
+// close 1.13 -> 1.05 ms).
+constexpr size_t kSlabLimit = (size_t)64 << 20;
+
 int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx** out) {
   *out = nullptr;
   if (!p || p->NE < 2 || p->Nk < 1 || p->Nb < 1) {
@@ -564,7 +568,7 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
     set_last_error("refinement applies to a reduced-precision context (QCL_C64 or QCL_MIXED)");
     return QCL_ARG;
   }
-  size_t budget = p->memory_budget_bytes, base_peak = 0;
+  size_t budget = p->memory_budget_bytes, base_peak = 0, slab = 0;
   {
     // preflight: refuse before the first allocation (build_production_cache,
     // production_cache.jl:764-770)
@@ -572,6 +576,7 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
     int s0 = plan_memory(p, mechs, &mp);
     if (s0) return s0;
     base_peak = mp.peak();
+    slab = mp.fields + mp.workspace + mp.anderson + (p->precision == QCL_C128 ? mp.operators : 0);
     if (budget == 0) {
       size_t fr = 0, tot = 0;
       cudaError_t e = cudaMemGetInfo(&fr, &tot);
@@ -661,12 +666,18 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaStreamCreate"));
   }
-  TRY(dupload(&c->eps, p->eps, c->NE * sizeof(double), c->st));
-  TRY(dupload(&c->wE, p->wE, c->NE * sizeof(double), c->st));
-  TRY(dupload(&c->wk, p->wk, c->Nk * sizeof(double), c->st));
-  TRY(dupload(&c->h, p->h, (size_t)c->Nk * c->N * c->N * 16, c->st));
-  TRY(dupload(&c->Tp, p->Tplus, (size_t)c->N * c->N * 16, c->st));
-  TRY(dupload(&c->Tm, p->Tminus, (size_t)c->N * c->N * 16, c->st));
+  if (slab <= kSlabLimit) {
+    // the plan, the grids and what every one of some 100 arrays takes to the next 512 bytes
+    slab += (size_t)c->NE * 88 + (size_t)(c->Nk + 2) * (16 * c->N * c->N + 8) + 100 * 512;
+    if (cudaMalloc(&c->slab, slab) == cudaSuccess) c->slab_bytes = slab;
+    else cudaGetLastError();  // an allocation each
+  }
+  TRY(dupload(c, &c->eps, p->eps, c->NE * sizeof(double)));
+  TRY(dupload(c, &c->wE, p->wE, c->NE * sizeof(double)));
+  TRY(dupload(c, &c->wk, p->wk, c->Nk * sizeof(double)));
+  TRY(dupload(c, &c->h, p->h, (size_t)c->Nk * c->N * c->N * 16));
+  TRY(dupload(c, &c->Tp, p->Tplus, (size_t)c->N * c->N * 16));
+  TRY(dupload(c, &c->Tm, p->Tminus, (size_t)c->N * c->N * 16));
   TRY(fill_plan(c, c->shift[0], +c->Ep));
   TRY(fill_plan(c, c->shift[1], -c->Ep));
   TRY(fill_plan(c, c->shift[2], +c->hw_LO));
@@ -720,8 +731,6 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
   c->state.assign(3 * F, nullptr);
   c->cand.assign(3 * F, nullptr);
   {
-    // the fields: one allocation each, or, where each would be small (an
-    // allocation costs more than the field's use of it), one for all
     std::vector<void**> fields;
     for (int i = 0; i < 3 * F; ++i) {
       fields.push_back(&c->state[i]);
@@ -729,25 +738,19 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
     }
     for (void** f : {&c->GR, &c->GL, &c->GG, &c->tot[0], &c->tot[1], &c->tot[2], &c->candSL, &c->tmp})
       fields.push_back(f);
-    const size_t step = (c->fcap + 511) / 512 * 512;
-    if (step <= ((size_t)1 << 20)) {
-      TRY(dalloc(&c->slab, step * fields.size()));
-      for (size_t i = 0; i < fields.size(); ++i) *fields[i] = (char*)c->slab + i * step;
-    } else {
-      for (void** f : fields) TRY(dalloc(f, c->fcap));
-    }
+    for (void** f : fields) TRY(dalloc(c, f, c->fcap));
   }
-  TRY(dalloc(&c->cwork, cwork));
+  TRY(dalloc(c, &c->cwork, cwork));
   c->cwork_bytes = cwork;
-  TRY(dalloc((void**)&c->trL, (size_t)c->NE * c->Nk * 16));
-  TRY(dalloc((void**)&c->trG, (size_t)c->NE * c->Nk * 16));
-  TRY(dalloc((void**)&c->rpartial, kReduceCtas * 4 * sizeof(double)));
-  TRY(dalloc((void**)&c->mpartial, std::max(residual_mix_multi_partial_doubles(3 * (c->M + 2)),
+  TRY(dalloc(c, (void**)&c->trL, (size_t)c->NE * c->Nk * 16));
+  TRY(dalloc(c, (void**)&c->trG, (size_t)c->NE * c->Nk * 16));
+  TRY(dalloc(c, (void**)&c->rpartial, kReduceCtas * 4 * sizeof(double)));
+  TRY(dalloc(c, (void**)&c->mpartial, std::max(residual_mix_multi_partial_doubles(3 * (c->M + 2)),
                                             mix_families_partial_doubles()) * sizeof(double)));
-  TRY(dalloc((void**)&c->reswork, residual_work_doubles(c->NE, c->Nk) * sizeof(double)));
-  TRY(dalloc((void**)&c->obspartial, observables_partial_doubles(c->N) * sizeof(double)));
+  TRY(dalloc(c, (void**)&c->reswork, residual_work_doubles(c->NE, c->Nk) * sizeof(double)));
+  TRY(dalloc(c, (void**)&c->obspartial, observables_partial_doubles(c->N) * sizeof(double)));
   QCL_CUDA_CHECK(cudaMemsetAsync(c->obspartial, 0, observables_partial_doubles(c->N) * sizeof(double), c->st));
-  TRY(dalloc((void**)&c->scal, SC_ALLOC * sizeof(double)));
+  TRY(dalloc(c, (void**)&c->scal, SC_ALLOC * sizeof(double)));
   {
     cudaError_t e = cudaMallocHost((void**)&c->scal_h, SC_TOTAL * sizeof(double));
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaMallocHost"));
@@ -758,10 +761,10 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
   for (auto& m : c->mech) m.status = c->status;
   if (c->mixing) {
     const size_t nf = 3 * (size_t)(c->M + 2);
-    TRY(dalloc(&c->Xh, (size_t)c->and_depth * nf * c->fcap));
-    TRY(dalloc(&c->Rh, (size_t)c->and_depth * nf * c->fcap));
-    TRY(dalloc((void**)&c->ameta, sizeof(AndersonMeta)));
-    TRY(dalloc((void**)&c->apartial, anderson_partial_doubles((int)nf) * sizeof(double)));
+    TRY(dalloc(c, &c->Xh, (size_t)c->and_depth * nf * c->fcap));
+    TRY(dalloc(c, &c->Rh, (size_t)c->and_depth * nf * c->fcap));
+    TRY(dalloc(c, (void**)&c->ameta, sizeof(AndersonMeta)));
+    TRY(dalloc(c, (void**)&c->apartial, anderson_partial_doubles((int)nf) * sizeof(double)));
     cudaError_t e = cudaMallocHost((void**)&c->ameta_h, sizeof(AndersonMeta));
     if (e != cudaSuccess) TRY(cuda_status(e, "cudaMallocHost"));
     memset(c->ameta_h, 0, sizeof(AndersonMeta));
