@@ -33,9 +33,10 @@
 // that: before it, the leading 7 bits of all entries (rounded down, so that
 // their sum is a lower bound of S) go through one int8 product, 1/108 of the
 // work.  One output below the line adds the diagonal s + t = 8 to the product;
-// what is left then is the rounding of the operands, 2^-62.8 rms of the maxima
-// per entry, whose line is sqrt(K) / 1500.  One output below that rejects the
-// product, which then takes the FP64 tensor path.  Outputs of a zero row are
+// what is left then is the rounding of the operands, 2^-62 of the maxima per
+// entry (2^-62.8 rms): S = 0.006 by the bounds, sqrt(K) / 1500 by the rms.  One
+// output below that line rejects the product, which then takes the FP64 tensor
+// path.  Outputs of a zero row are
 // exact and exempt; a non-finite entry rejects.  Errors in units of sum |a| |b|,
 // here / FP64 path:
 //   normal entries, K = 1024 ... 8192: 3.4 ... 1.3e-18 / 6e-17
@@ -62,7 +63,8 @@
 // Bound: the int8 rate and the power limit (980 of 1000 W drawn).  2048 x 8192
 // x 8192 (both Keldysh components of an operator with 32 momenta and 16
 // states): 9.9 ms = 3.0 POP/s of the 4.2 POP/s that resident operands reach,
-// plus 1.2 ms for the split; the FP64 tensor path takes 36 ms.
+// plus 1.2 ms for the split and 0.35 ms for the bound; the FP64 tensor path takes
+// 36 ms.  With the extra diagonal about 12.5 ms.
 #include <algorithm>
 #include <cmath>
 
