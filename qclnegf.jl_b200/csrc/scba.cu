@@ -358,6 +358,7 @@ void scba_destroy(ScbaCtx* c) {
 // ---------------------------------------------------------------------------
 struct MemPlan {
   size_t fields = 0, operators = 0, workspace = 0, anderson = 0, transient = 0;
+  size_t hilbert = 0;  // part of the workspace
   size_t resident() const { return fields + operators + workspace + anderson; }
   size_t peak() const { return resident() + transient; }
 };
@@ -420,10 +421,11 @@ static int plan_memory(const qcl_scba_problem* p, const qcl_mechanism* mechs, Me
     if (p->refinement && !c128) cwork = std::max(cwork, op_work_elems(q, QCL_C128, NE, Nk, N) * 16);
   }
   const int L = next_pow2(2 * NE - 1);
+  mp->hilbert = (size_t)16 * 16 * L /* FFT tables */ + (size_t)Nk * N * N * 2 * 8 /* per-column partials */;
   mp->workspace = cwork + 2 * (size_t)NE * Nk * 16 + (size_t)kReduceCtas * 4 * 8 +
-                  std::max(residual_mix_multi_partial_doubles(3 * (M + 2)), mix_families_partial_doubles()) * 8 + residual_work_doubles(NE, Nk) * 8 +
-                  observables_partial_doubles(N) * 8 + 4096 /* scalars, status */ +
-                  (size_t)16 * 16 * L /* FFT tables */ + (size_t)Nk * N * N * 2 * 8 /* per-column partials */;
+                  std::max(residual_mix_multi_partial_doubles(3 * (M + 2)), mix_families_partial_doubles()) * 8 +
+                  residual_work_doubles(NE, Nk) * 8 + observables_partial_doubles(N) * 8 + 4096 /* scalars, status */ +
+                  mp->hilbert;
   if (p->mixing)
     mp->anderson = 2 * (size_t)p->anderson_history_depth * 3 * (M + 2) * fcap +
                    anderson_partial_doubles(3 * (M + 2)) * 8 + sizeof(AndersonMeta);
@@ -576,7 +578,7 @@ int scba_create(const qcl_scba_problem* p, const qcl_mechanism* mechs, ScbaCtx**
     int s0 = plan_memory(p, mechs, &mp);
     if (s0) return s0;
     base_peak = mp.peak();
-    slab = mp.fields + mp.workspace + mp.anderson + (p->precision == QCL_C128 ? mp.operators : 0);
+    slab = mp.fields + mp.workspace - mp.hilbert + mp.anderson + (p->precision == QCL_C128 ? mp.operators : 0);
     if (budget == 0) {
       size_t fr = 0, tot = 0;
       cudaError_t e = cudaMemGetInfo(&fr, &tot);
