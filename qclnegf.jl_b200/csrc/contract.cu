@@ -487,6 +487,8 @@ static int launch_gemm(const GemmArgs<double>& args, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Contraction dispatch
 // ---------------------------------------------------------------------------
+constexpr size_t kOperandAlign = 256;  // of tensor-core operands behind the intermediate (a tensor map needs 16)
+
 // Whether a complex128 product goes to the integer path: large enough, and
 // the operator's work area holds its smallest panels.
 static bool takes_i8(const KernelOpDev& op, int M, int fields, int N, int K) {
@@ -625,7 +627,7 @@ static int contraction_t(const KernelOpDev& op, int NE, int Nk, int N, const dou
     const size_t zfield = (size_t)Mr * N2;        // one intermediate field
     Cx<R>* Z = (Cx<R>*)work;
     const int jmax = J < kSepChunk ? J : kSepChunk;  // terms per chunk
-    float* awork = (float*)((char*)work + (size_t)jmax * zfield * sizeof(Cx<R>));
+    float* awork = (float*)((char*)work + (jmax * zfield * sizeof(Cx<R>) + kOperandAlign - 1) / kOperandAlign * kOperandAlign);
     // complex64 with tensor-core stage-1 operands: G split once for all chunks,
     // rows (e, (c,d)), K = m', behind the stage-2 work area
     float* gwork = awork + tc_a_work_floats2((int)Mr, jmax * N2);
@@ -735,8 +737,8 @@ size_t contraction_work_elems(const KernelOpDev& op, int NE, int Nk, int N) {
     const int jmax = op.J < kSepChunk ? op.J : kSepChunk;
     const size_t zf = (size_t)jmax * NE * Nk * N * N;
     if (op.tc_chunks)
-      return zf + (tc_a_work_floats2(NE * Nk, jmax * N * N) + (op.tc_stage1 ? tc_a_work_floats2(NE * N * N, Nk) : 0) +
-                   1) / 2;
+      return zf + kOperandAlign / sizeof(Cx<float>) +
+             (tc_a_work_floats2(NE * Nk, jmax * N * N) + (op.tc_stage1 ? tc_a_work_floats2(NE * N * N, Nk) : 0) + 1) / 2;
     return zf;
   }
   return 0;
